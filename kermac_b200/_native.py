@@ -174,6 +174,37 @@ def lib() -> C.CDLL:
         return handle
 
 
+# The extension that takes ordinary calls from torch tensors straight to the C-ABI (csrc/km_torch_call.cpp).
+# Not loaded yet: None; not usable with this torch: False (every call then marshals through ctypes).
+_call = None
+
+
+def torch_call():
+    """The bound `_torch_call` extension, or False where it cannot be loaded."""
+    global _call
+    if _call is None:
+        handle = lib()
+        with _lock:
+            if _call is None:
+                try:
+                    from . import _torch_call
+                except ImportError as exc:
+                    import warnings
+                    warnings.warn(f"kermac_b200._torch_call is not usable ({exc}): calls go through ctypes and cost "
+                                  "about 20 us more; rebuild with `make -C kermac_b200/csrc`", RuntimeWarning)
+                    _call = False
+                    return _call
+                from .build_a_kernel import InnerOperator, KernelType, PowerType
+                address = lambda fn: C.cast(fn, C.c_void_p).value       # noqa: E731
+                _torch_call.bind((address(handle.kermac_b200_build_kernel), address(handle.kermac_b200_cdist_grad),
+                                  address(handle.kermac_b200_cdist_grad_scratch_bytes),
+                                  address(handle.kermac_b200_kernel_matvec),
+                                  address(handle.kermac_b200_kernel_matvec_scratch_bytes)),
+                                 (InnerOperator, PowerType, KernelType))
+                _call = _torch_call
+    return _call
+
+
 def last_error() -> str:
     msg = lib().kermac_b200_last_error()
     return msg.decode("utf-8", "replace") if msg else ""

@@ -132,6 +132,20 @@ def _is_cuda(t: torch.Tensor) -> bool:
     return t.is_cuda
 
 
+def _torch_call_for(t):
+    """The `_torch_call` extension for a call on `t`; loads it with the first CUDA tensor."""
+    if not isinstance(t, torch.Tensor) or not t.is_cuda:
+        return False
+    return _native.torch_call()
+
+
+def _call_result(result, what):
+    """What a `_torch_call` function returned: the output tensor, or a C-ABI error code to raise for."""
+    if type(result) is int:
+        _native.check(result, what)
+    return result
+
+
 def _current_stream_for(tensor_device):
     """(stream pointer) of torch's current stream, which must live on `tensor_device`."""
     pt_stream = torch.cuda.current_stream()
@@ -309,6 +323,16 @@ def run_kernel(
     affected tiles are not written and a device flag is raised.  Nothing here reads it: poll
     `kermac_b200._native.device_error_flag()` at your own synchronisation points (0 = clean).
     """
+    # An ordinary call goes straight to the C-ABI (csrc/km_torch_call.cpp); what that declines (None) is
+    # validated and marshalled below.
+    call = _native._call
+    if call is None:
+        call = _torch_call_for(a)
+    if call and not debug:
+        result = call.run_kernel(kernel_descriptor, a, b, out, p, inner_p, outer_p, bandwidth, epsilon, regularization,
+                                 regularization_offset_x, regularization_offset_y)
+        if result is not None:
+            return _call_result(result, "kermac_b200_build_kernel")
     args, out, keep_alive = _marshal_build(
         kernel_descriptor, a, b, out, p, inner_p, outer_p, bandwidth, epsilon, regularization,
         regularization_offset_x, regularization_offset_y)

@@ -9,7 +9,9 @@ from __future__ import annotations
 
 import torch
 
-from .build_a_kernel import InnerOperator, KernelDescriptor, KernelType, PowerType, run_kernel
+from . import _native
+from .build_a_kernel import (InnerOperator, KernelDescriptor, KernelType, PowerType, _call_result, _torch_call_for,
+                             run_kernel)
 
 __all__ = ["cdist"]
 
@@ -41,6 +43,13 @@ def cdist(
         TypeError: inputs are not float32 torch tensors.
         ValueError: shapes, strides, batch sizes or devices are invalid.
     """
+    call = _native._call
+    if call is None:
+        call = _torch_call_for(a)
+    if call and not debug:
+        result = call.cdist(a, b, out, p, skip_epilogue)
+        if result is not None:
+            return _call_result(result, "kermac_b200_build_kernel")
     descriptor, powers = descriptor_for(p, skip_epilogue)
     return run_kernel(descriptor, a, b, out=out, try_to_align=try_to_align, debug=debug, **powers)
 

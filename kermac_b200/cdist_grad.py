@@ -13,7 +13,7 @@ from typing import Union
 import torch
 
 from . import _native
-from .build_a_kernel import _current_stream_for, _is_cuda
+from .build_a_kernel import _call_result, _current_stream_for, _is_cuda, _torch_call_for
 from .common import merge_batch_size, tensor_stats
 
 __all__ = ["cdist_grad"]
@@ -150,6 +150,13 @@ def cdist_grad(
         TypeError: inputs are not float32 torch tensors.
         ValueError: shapes, strides, dimensions or CUDA devices are invalid.
     """
+    call = _native._call
+    if call is None:
+        call = _torch_call_for(a)
+    if call and not debug:
+        result = call.cdist_grad(a, b, c, d, out, p, _CONTRACTIONS.get(contraction))
+        if result is not None:
+            return _call_result(result, "kermac_b200_cdist_grad")
     args, out = _marshal_grad(a, b, c, d, out, p, contraction)
     stream_ptr = _current_stream_for(a.device)
     library = _native.lib()

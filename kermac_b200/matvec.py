@@ -14,8 +14,8 @@ from typing import Optional, Union
 import torch
 
 from . import _native
-from .build_a_kernel import (KernelDescriptor, _check_descriptor_arguments, _check_hyper_tensor,
-                             _current_stream_for, _is_cuda, _resolve_powers)
+from .build_a_kernel import (KernelDescriptor, _call_result, _check_descriptor_arguments, _check_hyper_tensor,
+                             _current_stream_for, _is_cuda, _resolve_powers, _torch_call_for)
 from .common import merge_batch_size, tensor_stats
 
 __all__ = ["kernel_matvec"]
@@ -145,6 +145,14 @@ def kernel_matvec(
     runs out leaves the affected rows unwritten and raises a device flag that nothing here reads:
     poll `kermac_b200._native.device_error_flag()` at your own synchronisation points.
     """
+    call = _native._call
+    if call is None:
+        call = _torch_call_for(a)
+    if call and not debug:
+        result = call.kernel_matvec(kernel_descriptor, a, b, c, out, p, inner_p, outer_p, bandwidth, epsilon, regularization,
+                                    regularization_offset_x, regularization_offset_y, split_m, contraction)
+        if result is not None:
+            return _call_result(result, "kermac_b200_kernel_matvec")
     args, out, keep_alive = _marshal_matvec(kernel_descriptor, a, b, c, out, p, inner_p, outer_p, bandwidth, epsilon,
                                             regularization, regularization_offset_x, regularization_offset_y)
     stream_ptr = _current_stream_for(a.device)

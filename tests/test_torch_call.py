@@ -1,0 +1,71 @@
+"""The extension that takes ordinary calls straight to the C-ABI: same results as the ctypes marshalling
+(which `debug=True` still uses), and anything out of the ordinary is declined, so that the Python layer's own
+checks and exceptions apply."""
+import pytest
+import torch
+
+import kermac_b200 as kermac
+from kermac_b200 import _native
+
+
+def test_declines_what_is_not_an_ordinary_call():
+    call = _native.torch_call()
+    assert call, "the extension is built together with the library"
+    a, b = torch.zeros(4, 3), torch.zeros(5, 3)
+    assert call.cdist(a, b, None, 2.0, False) is None                       # not on a CUDA device
+    assert call.cdist(a.numpy(), b, None, 2.0, False) is None
+    assert call.cdist(a, b, None, "2", False) is None
+    assert call.run_kernel(object(), a, b, *[None] * 7, 0, 0) is None
+    assert call.cdist_grad(a, b, b, a, None, 2.0, None) is None
+
+
+def _col(t):
+    return t.transpose(-1, -2).contiguous().transpose(-1, -2)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("L", [1, 3])
+@pytest.mark.parametrize("layout", ["row", "col"])
+def test_same_bits_as_the_ctypes_marshalling(L, layout, capsys):
+    g = torch.Generator().manual_seed(5)
+    def gen(*shape):
+        return torch.randn(*((L,) + shape if L > 1 else shape), generator=g).cuda()
+    M, N, K, O = 70, 33, 12, 3
+    a, b = gen(M, K), gen(N, K)[:1] if L > 1 else gen(N, K)                  # b broadcasts over the batch
+    if layout == "col":
+        a, b = _col(a), _col(b)
+    c, ga, gb, gc, gd = gen(O, M), gen(K, M).abs(), gen(N, K), gen(O, K), gen(N, M)
+    bw = torch.full((L,), 3.0, device="cuda")
+    gauss = kermac.KernelDescriptor(kermac.InnerOperator.DIFF, kermac.PowerType.SQUARE, kermac.PowerType.NOOP,
+                                    kermac.KernelType.GAUSSIAN)
+    out = torch.empty(L, M, N, device="cuda")
+    calls = [
+        lambda **k: kermac.cdist(a, b, **k), lambda **k: kermac.cdist(a, b, p=1, **k),
+        lambda **k: kermac.cdist(a, b, p=1.3, out=_col(out), **k), lambda **k: kermac.cdist(a, b, p=2.0, skip_epilogue=True, **k),
+        lambda **k: kermac.run_kernel(kermac.kernel_descriptor_laplace_l1, a, b, bandwidth=bw, **k),
+        lambda **k: kermac.run_kernel(gauss, a, b, bandwidth=2.0, epsilon=1e-3, regularization=0.5, regularization_offset_x=4, **k),
+        lambda **k: kermac.run_kernel(kermac.kernel_descriptor_p_norm, a, b, inner_p=1.5, outer_p=0.5, **k),
+        lambda **k: kermac.run_kernel(kermac.kernel_descriptor_mma, a, b, **k),
+        lambda **k: kermac.cdist_grad(ga, gb, gc, gd, p=1.5, **k), lambda **k: kermac.cdist_grad(ga, gb, gc, gd, p=1.0, **k),
+        lambda **k: kermac.kernel_matvec(kermac.kernel_descriptor_laplace_l2, a, b, c, bandwidth=bw, **k),
+    ]
+    for call in calls:
+        fast, slow = call(), call(debug=True)
+        assert "Kermac Debug" in capsys.readouterr().out
+        assert fast.shape == slow.shape and torch.equal(fast, slow)
+    assert kermac.cdist(a, b, out=out) is out
+
+
+@pytest.mark.gpu
+def test_exceptions_of_the_python_layer_still_apply():
+    a, b = torch.zeros(4, 3, device="cuda"), torch.zeros(5, 3, device="cuda")
+    with pytest.raises(ValueError, match="K dimensions must match"):
+        kermac.cdist(a, b[:, :2].contiguous())
+    with pytest.raises(TypeError, match="float32"):
+        kermac.cdist(a.double(), b)
+    with pytest.raises(ValueError, match="non-standard memory layout"):
+        kermac.cdist(torch.zeros(4, 6, device="cuda")[:, ::2], b)
+    with pytest.raises(ValueError, match="must be on a CUDA device"):
+        kermac.cdist(a, b.cpu())
+    with pytest.raises(ValueError, match="contraction"):
+        kermac.cdist_grad(torch.zeros(3, 4, device="cuda"), b, b[:2], torch.zeros(5, 4, device="cuda"), contraction="no")
