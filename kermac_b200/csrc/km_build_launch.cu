@@ -4,6 +4,7 @@
 #include <cstring>
 
 #include "km_build_cpasync_table.cuh"
+#include "km_build_small.h"
 #include "km_build_tma.cuh"
 #include "km_host.h"
 
@@ -27,10 +28,41 @@ bool layout_ok(long long rows, long long cols, long long s_row, long long s_col)
 
 struct BuildPlan {
     BuildParams p;
-    bool avec, bvec;
+    bool avec, bvec;       // can be copied 16 bytes at a time along the points
+    bool awide, bwide;     // ... or along k
     bool swapped;
     int  variant;
+    bool small;      // 64 x 64 tiles
 };
+
+// When the 64 x 64 kernel is the faster one (K >= 1, an inner step it has).  Measured on B200, 128 x 128
+// kernels against the 64 x 64 one, us:
+//   torch rows, 16-byte aligned: always, because the 64 x 64 kernel loads those 16 bytes at a time too
+//       square  2 x 1000^2 x 64: 22.9 / 18.8   8000^2 x 96: 580 / 431   16384^2 x 256: 5330 / 4695
+//       |.|     2 x 1000^2 x 64: 28.9 / 17.6   8000^2 x 96: 637 / 429   16384^2 x 256: 5947 / 4671
+//       |.|^1.3 2 x 1000^2 x 64: 74.0 / 65.9   8000^2 x 96: 2413 / 2230 16384^2 x 256: 26139 / 24770
+//   an operand that both can only copy word by word: few tiles; for |.| and |.|^p also a short k loop
+//       square  1000^2 x 27: 33.7 / 11.2   4000^2 x 27: 66.0 / 64.8   4000^2 x 129: 206 / 245
+//       |.|     1000^2 x 27: 32.6 / 9.3    4001 x 4003 x 64: 140 / 118   8001 x 8003 x 300: 1727 / 1911
+//       |.|^1.3 1000^2 x 27: 44.8 / 21.7   4001 x 4003 x 64: 440 / 425   8001 x 8003 x 300: 7543 / 7636
+//   both operands contiguous along the points: a short k loop, or few tiles:
+//       square  2048^2 x 64: 28.9 / 22.8   2048^2 x 512: 156 / 140   4000^2 x 512: 521 / 509
+//               4000^2 x 1024: 1029 / 1045   16384^2 x 128: 2148 / 2127   16384^2 x 256: 4111 / 4159
+//       |.|     2048^2 x 64: 33.0 / 24.8   2048^2 x 512: 171 / 158   4000^2 x 512: 581 / 569
+//               4000^2 x 1024: 1124 / 1142   16384^2 x 64: 1383 / 1279   16384^2 x 128: 2375 / 2400
+//       |.|^1.3 2048^2 x 64: 125 / 107   2048^2 x 512: 923 / 814   4000^2 x 1024: 6278 / 6081
+//               16384^2 x 128: 12559 / 12527   16384^2 x 256: 24802 / 24864
+// The line is drawn by the whole problem, not by the launch's tile range: the two kernels spread the two
+// forms of the fractional power differently over a tile, and ranges must add up to the full launch's bits.
+bool small_preferred(const BuildParams& p, bool avec, bool bvec, bool awide, bool bwide) {
+    const long long tiles =
+        (p.symmetric ? (long long)p.tiles_n * (p.tiles_n + 1) / 2 : (long long)p.tiles_m * p.tiles_n) * p.L;
+    if (!awide || !bwide)
+        return tiles <= 512 || ((p.inner_id == IN_DIFF_ABS || p.inner_id == IN_DIFF_POW) && p.K <= 128);
+    if (!avec || !bvec) return true;
+    if (p.K <= (p.inner_id == IN_DIFF_ABS ? 96 : 128)) return true;
+    return tiles <= 512 || (tiles <= 1024 && (p.K <= 512 || p.inner_id == IN_DIFF_POW));
+}
 
 int make_plan(const KmBuildArgs* a, BuildPlan* plan) {
     if (!a) return fail(KM_ERR_NULL_POINTER, "args is NULL");
@@ -137,6 +169,10 @@ int make_plan(const KmBuildArgs* a, BuildPlan* plan) {
         return fail(KM_ERR_BAD_STRIDE, "the TMA variant needs m-contiguous, 16-byte aligned a and b with 16-byte pitches");
     if (variant == KM_VARIANT_AUTO) variant = (tma_ok && tma_preferred(p)) ? KM_VARIANT_TMA : KM_VARIANT_CPASYNC;
     plan->variant = variant;
+    plan->awide   = small_wide_loads(p.A, p.a_sm, p.a_sk, p.a_sl, p.K, p.L);
+    plan->bwide   = small_wide_loads(p.B, p.b_sn, p.b_sk, p.b_sl, p.K, p.L);
+    plan->small   = a->variant == KM_VARIANT_AUTO && small_supported(p) &&
+                    small_preferred(p, plan->avec, plan->bvec, plan->awide, plan->bwide);
     return 0;
 }
 
@@ -155,6 +191,7 @@ extern "C" int kermac_b200_build_kernel(const KmBuildArgs* args, void* stream) {
     if (int rc = require_sm100()) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
 
+    if (plan.small) return launch_build_small(p, plan.variant == KM_VARIANT_TMA, st);
     if (plan.variant == KM_VARIANT_TMA) return launch_build_tma(p, st);
 
     BuildKernelFn fn = cpasync_kernel(p.inner_id, plan.avec, plan.bvec, p.symmetric != 0);
@@ -198,9 +235,9 @@ extern "C" int kermac_b200_describe_variant(const KmBuildArgs* args, char* buf, 
     const BuildParams& p = plan.p;
     snprintf(buf, (size_t)buf_len,
              "build_kernel variant=%s inner=%s outer_power=%d kernel_type=%d exchanged=%d a_vec16=%d b_vec16=%d "
-             "out_vec16=%d tiles=%dx%d batches=%d symmetric=%d tile_range=%d+%d",
+             "out_vec16=%d tiles=%dx%d batches=%d symmetric=%d tile_range=%d+%d kernel_tile=%d",
              plan.variant == KM_VARIANT_TMA ? "tma" : "cpasync", kInnerNames[p.inner_id], p.outer_power, p.kernel_type,
              plan.swapped ? 1 : 0, plan.avec ? 1 : 0, plan.bvec ? 1 : 0, p.c_vec4, p.tiles_m, p.tiles_n, p.L, p.symmetric,
-             p.tile_first, p.tile_count);
+             p.tile_first, p.tile_count, plan.small ? 64 : BUILD_TILE);
     return 0;
 }

@@ -23,6 +23,7 @@
 #include <mutex>
 
 #include "km_build_cpasync.cuh"
+#include "km_build_small.h"
 #include "km_build_tma.cuh"
 #include "km_mbar.cuh"
 #include "km_host.h"
@@ -347,6 +348,7 @@ extern "C" int kermac_b200_device_error_flag(void) {
     if (v) cudaMemcpyToSymbol(km::g_tma_wait_expired, &zero, sizeof(int));
     const int mv = km::matvec_take_wait_flag();
     const int gv = km::grad_tensor_take_wait_flag();
-    if (mv < 0 || gv < 0) return KM_ERR_INTERNAL;
-    return (v || mv || gv) ? 1 : 0;
+    const int sv = km::small_take_wait_flag();
+    if (mv < 0 || gv < 0 || sv < 0) return KM_ERR_INTERNAL;
+    return (v || mv || gv || sv) ? 1 : 0;
 }

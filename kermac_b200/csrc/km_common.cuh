@@ -295,29 +295,30 @@ __host__ __device__ inline int inner_id(int op, int power) {
     return -1;
 }
 
-// Which of the 8 x 4 element pairs of a register block take their exponential on the FP32
-// pipe (ex2_poly2) rather than on MUFU: KM_POW_POLY_EIGHTHS of every 8 pairs.
+// Which of the 8 x MP element pairs of a register block (MP = 4, or 2 in the 64 x 64 kernel) take their
+// exponential on the FP32 pipe (ex2_poly2) rather than on MUFU: KM_POW_POLY_EIGHTHS of every 8 pairs.
 #ifndef KM_POW_POLY_EIGHTHS
 #define KM_POW_POLY_EIGHTHS 6
 #endif
+template <int MP>
 __device__ __forceinline__ constexpr bool pow_pair_uses_fp32_exp(int n, int mp) {
-    return ((n & 1) * 4 + mp) < KM_POW_POLY_EIGHTHS;
+    return ((n % (8 / MP)) * MP + mp) < KM_POW_POLY_EIGHTHS;
 }
 
-// One k step of an 8 (rows of the pair-packed operand) x 8 register block.
-//   ap[4]  : the 8 values of the m-side operand as 4 packed pairs (m, m+1)
+// One k step of an 8 (rows of the pair-packed operand) x 2 MP register block.
+//   ap[MP] : the 2 MP values of the m-side operand as packed pairs (m, m+1)
 //   bv[8]  : the 8 values of the n-side operand
 //   acc    : acc[n][mp] packed pair of accumulators for (m = 2 mp, 2 mp + 1)
 // `sgn` is +1 normally and -1 when the launcher exchanged the two operands (so
 // that signed inner steps still see b - a).
-template <int INNER>
-__device__ __forceinline__ void inner_block(u64 (&acc)[8][4], const u64 (&ap)[4], const float (&bv)[8], float p_inner,
+template <int INNER, int MP>
+__device__ __forceinline__ void inner_block(u64 (&acc)[8][MP], const u64 (&ap)[MP], const float (&bv)[8], float p_inner,
                                             float sgn) {
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
         const u64 bd = pack2(bv[n], bv[n]);
 #pragma unroll
-        for (int mp = 0; mp < 4; ++mp) {
+        for (int mp = 0; mp < MP; ++mp) {
             if constexpr (INNER == IN_DIFF_SQUARE) {
                 const u64 d = sub2(bd, ap[mp]);
                 acc[n][mp]  = fma2(d, d, acc[n][mp]);
@@ -332,7 +333,7 @@ __device__ __forceinline__ void inner_block(u64 (&acc)[8][4], const u64 (&ap)[4]
                     a0 += fabsf(d0);
                     a1 += fabsf(d1);
                 } else if constexpr (INNER == IN_DIFF_POW || INNER == IN_DOT_POW) {
-                    if (pow_pair_uses_fp32_exp(n, mp)) {
+                    if (pow_pair_uses_fp32_exp<MP>(n, mp)) {
                         // most pairs: lg2 on MUFU, the exponential on the FP32 pipe.  A pair costs
                         // ~30 issue slots this way against ~10 (and 32 MUFU cycles instead of 16)
                         // the all-MUFU way; the share is set where the kernel measured fastest.
@@ -366,16 +367,20 @@ __device__ __forceinline__ void inner_block(u64 (&acc)[8][4], const u64 (&ap)[4]
 }
 
 // Consumes one staged k slab ([BK][PITCH] floats per operand, tile dimension
-// contiguous) for a thread whose 8 x 8 block reads the m-side at sa + {0, 32} and
-// the n-side at sb + {0, 16}.  Only the first `kvalid` k rows are used, so a partial
+// contiguous) for a thread whose 8 x 2 MP block reads the m-side at sa + {0, 32} (MP = 4) or
+// sa (MP = 2) and the n-side at sb + {0, 16}.  Only the first `kvalid` k rows are used, so a partial
 // last slab contributes exactly the rows that exist.
-template <int INNER, int BK, int PITCH>
-__device__ __forceinline__ void consume_slab(u64 (&acc)[8][4], const float* sa, const float* sb, int kvalid,
+template <int INNER, int BK, int PITCH, int MP>
+__device__ __forceinline__ void consume_slab(u64 (&acc)[8][MP], const float* sa, const float* sb, int kvalid,
                                              float p_inner, float sgn) {
     auto step = [&](int kk) {
-        const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(sa + kk * PITCH);
-        const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(sa + kk * PITCH + 32);
-        const u64   ap[4] = {a0.x, a0.y, a1.x, a1.y};
+        u64 ap[MP];
+#pragma unroll
+        for (int i = 0; i < MP / 2; ++i) {
+            const ulonglong2 a2 = *reinterpret_cast<const ulonglong2*>(sa + kk * PITCH + i * 32);
+            ap[2 * i]     = a2.x;
+            ap[2 * i + 1] = a2.y;
+        }
         float bv[8];
         if constexpr (INNER == IN_DIFF_ABS || INNER == IN_DOT_ABS) {
             // The |.| step reads the n-side values one by one (warp-wide broadcasts): each lands in the
