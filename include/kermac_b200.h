@@ -133,6 +133,14 @@ typedef struct KmBuildArgs {
 
 int kermac_b200_build_kernel(const KmBuildArgs* args, void* stream);
 
+/* The same call with device scratch, which pays where a or b is held as rows (k contiguous): large problems
+ * rewrite such operands k-major first.  kermac_b200_build_scratch_bytes says how much the call would use (0:
+ * none, or the arguments are rejected); without it (NULL, too small, not 16-byte aligned) the call is
+ * kermac_b200_build_kernel.  The scratch may be reused once the stream has passed the call.  No reference
+ * counterpart. */
+int64_t kermac_b200_build_scratch_bytes(const KmBuildArgs* args);
+int kermac_b200_build_kernel_scratch(const KmBuildArgs* args, void* scratch, int64_t scratch_bytes, void* stream);
+
 /* Number of 128 x 128 output tiles of one batch entry of this problem: the extent of the
  * linear tile order that tile_first / tile_count index.  Negative KM_ERR_* code when the
  * arguments are rejected.  Counterpart of the grid computation at

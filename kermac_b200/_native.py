@@ -22,6 +22,8 @@ VARIANT_AUTO, VARIANT_CPASYNC, VARIANT_TMA = 0, 1, 2
 
 EXPORTED_SYMBOLS = (
     "kermac_b200_build_kernel",
+    "kermac_b200_build_kernel_scratch",
+    "kermac_b200_build_scratch_bytes",
     "kermac_b200_build_tile_count",
     "kermac_b200_cdist_grad",
     "kermac_b200_cdist_grad_scratch_bytes",
@@ -115,6 +117,10 @@ def library_path() -> str:
 def _declare(lib: C.CDLL) -> None:
     lib.kermac_b200_build_kernel.argtypes = [C.POINTER(KmBuildArgs), C.c_void_p]
     lib.kermac_b200_build_kernel.restype = C.c_int
+    lib.kermac_b200_build_kernel_scratch.argtypes = [C.POINTER(KmBuildArgs), C.c_void_p, C.c_int64, C.c_void_p]
+    lib.kermac_b200_build_kernel_scratch.restype = C.c_int
+    lib.kermac_b200_build_scratch_bytes.argtypes = [C.POINTER(KmBuildArgs)]
+    lib.kermac_b200_build_scratch_bytes.restype = C.c_int64
     lib.kermac_b200_build_tile_count.argtypes = [C.POINTER(KmBuildArgs)]
     lib.kermac_b200_build_tile_count.restype = C.c_int64
     lib.kermac_b200_selftest_wait_expiry.argtypes = [C.c_int32, C.c_void_p]
@@ -196,7 +202,8 @@ def torch_call():
                     return _call
                 from .build_a_kernel import InnerOperator, KernelType, PowerType
                 address = lambda fn: C.cast(fn, C.c_void_p).value       # noqa: E731
-                _torch_call.bind((address(handle.kermac_b200_build_kernel), address(handle.kermac_b200_cdist_grad),
+                _torch_call.bind((address(handle.kermac_b200_build_kernel_scratch),
+                                  address(handle.kermac_b200_build_scratch_bytes), address(handle.kermac_b200_cdist_grad),
                                   address(handle.kermac_b200_cdist_grad_scratch_bytes),
                                   address(handle.kermac_b200_kernel_matvec),
                                   address(handle.kermac_b200_kernel_matvec_scratch_bytes)),

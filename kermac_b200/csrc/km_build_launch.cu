@@ -1,12 +1,14 @@
 // kermac_b200_build_kernel: validation, operand exchange for n-contiguous outputs,
 // variant choice and launch.  Host-side counterpart of the second half of the
 // reference's run_kernel (src/kermac/build_a_kernel.py:237-392).
+#include <algorithm>
 #include <cstring>
 
 #include "km_build_cpasync_table.cuh"
 #include "km_build_small.h"
 #include "km_build_tma.cuh"
 #include "km_host.h"
+#include "km_pack.h"
 
 namespace km {
 
@@ -33,6 +35,7 @@ struct BuildPlan {
     bool swapped;
     int  variant;
     bool small;      // 64 x 64 tiles
+    bool automatic;  // the caller left the variant to this file
 };
 
 // When the 64 x 64 kernel is the faster one (K >= 1, an inner step it has).  Measured on B200, 128 x 128
@@ -171,9 +174,51 @@ int make_plan(const KmBuildArgs* a, BuildPlan* plan) {
     plan->variant = variant;
     plan->awide   = small_wide_loads(p.A, p.a_sm, p.a_sk, p.a_sl, p.K, p.L);
     plan->bwide   = small_wide_loads(p.B, p.b_sn, p.b_sk, p.b_sl, p.K, p.L);
-    plan->small   = a->variant == KM_VARIANT_AUTO && small_supported(p) &&
-                    small_preferred(p, plan->avec, plan->bvec, plan->awide, plan->bwide);
+    plan->automatic = a->variant == KM_VARIANT_AUTO;
+    plan->small     = plan->automatic && small_supported(p) &&
+                      small_preferred(p, plan->avec, plan->bvec, plan->awide, plan->bwide);
     return 0;
+}
+
+// Which operands of a planned call are worth rewriting k-major first.
+struct PackPlan {
+    PackJob job[2];
+    int     n;            // operands to pack; 0: none
+    bool    a, b;         // (kernel-side A / B)
+    bool    shared;       // B is the same matrix as A
+    long long floats[2];
+};
+
+// Measured on B200, the 64 x 64 kernel on torch rows against the kernel that packed operands take, us:
+//   square  4000^2 x 64: 82 / 70   8000^2 x 96: 431 / 382   4000^2 x 512: 568 / 509   16384^2 x 512: 9050 / 8030
+//   |.|     8000^2 x 96: 429 / 427   4000^2 x 512: 568 / 569   16384^2 x 512: 9090 / 8800
+//   |.|^1.3 level everywhere
+// so a pair and feature costs 7.4e-15 s less for the square and product steps, and 2e-15 s for |.| where packed
+// operands go to the 128 x 128 kernel.  An operand that could only be copied word by word costs 1e-14 s more
+// (square 8001 x 8003 x 300: 1561 us, packed 1150; |.| 1727 / 1250; |.|^1.3 7543 / 6940).  Packing must save half as much again as it costs.
+void plan_pack_operands(const BuildPlan& plan, PackPlan* pack) {
+    std::memset(pack, 0, sizeof(*pack));
+    const BuildParams& p = plan.p;
+    if ((plan.avec && plan.bvec) || p.M == 0 || p.N == 0 || !plan.automatic || !small_supported(p)) return;
+    double gain = 7.4e-15;
+    if (p.inner_id == IN_DIFF_ABS) gain = small_preferred(p, true, true, true, true) ? 0.0 : 2e-15;
+    if (p.inner_id == IN_DIFF_POW) gain = 0.0;
+    gain += ((plan.awide ? 0 : 1) + (plan.bwide ? 0 : 1)) * 1e-14;
+    if (gain == 0.0) return;
+    const double tiles = p.symmetric ? 0.5 * p.tiles_n * (p.tiles_n + 1.0) : (double)p.tile_count;
+    const double pairs = tiles * p.L * std::min((double)BUILD_TILE, (double)p.M) * std::min((double)BUILD_TILE, (double)p.N);
+    pack->a      = !plan.avec;
+    pack->b      = !plan.bvec;
+    pack->shared = p.A == p.B && p.M == p.N && p.a_sm == p.b_sn && p.a_sk == p.b_sk && p.a_sl == p.b_sl;
+    if (pack->a) {
+        pack->floats[pack->n] = plan_pack(&pack->job[pack->n], p.A, p.M, p.K, p.L, p.a_sm, p.a_sk, p.a_sl);
+        ++pack->n;
+    }
+    if (pack->b && !pack->shared) {
+        pack->floats[pack->n] = plan_pack(&pack->job[pack->n], p.B, p.N, p.K, p.L, p.b_sn, p.b_sk, p.b_sl);
+        ++pack->n;
+    }
+    if (pairs * p.K * gain < 1.5 * pack_seconds(pack->floats[0] + pack->floats[1])) pack->n = 0;
 }
 
 const char* const kInnerNames[IN_COUNT] = {"diff_abs", "diff_square", "diff_pow", "diff_noop", "diff_sqrt",
@@ -182,15 +227,11 @@ const char* const kInnerNames[IN_COUNT] = {"diff_abs", "diff_square", "diff_pow"
 }  // namespace
 }  // namespace km
 
-extern "C" int kermac_b200_build_kernel(const KmBuildArgs* args, void* stream) {
-    using namespace km;
-    BuildPlan plan;
-    if (int rc = make_plan(args, &plan)) return rc;
-    BuildParams& p = plan.p;
-    if (p.M == 0 || p.N == 0 || p.tile_count == 0) return 0;
-    if (int rc = require_sm100()) return rc;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
+namespace km {
+namespace {
 
+int launch_plan(const BuildPlan& plan, cudaStream_t st) {
+    const BuildParams& p = plan.p;
     if (plan.small) return launch_build_small(p, plan.variant == KM_VARIANT_TMA, st);
     if (plan.variant == KM_VARIANT_TMA) return launch_build_tma(p, st);
 
@@ -215,6 +256,57 @@ extern "C" int kermac_b200_build_kernel(const KmBuildArgs* args, void* stream) {
         if (int rc = cuda_status(cudaGetLastError(), "launch of build_cpasync_kernel")) return rc;
     }
     return 0;
+}
+
+}  // namespace
+}  // namespace km
+
+extern "C" int kermac_b200_build_kernel(const KmBuildArgs* args, void* stream) {
+    using namespace km;
+    BuildPlan plan;
+    if (int rc = make_plan(args, &plan)) return rc;
+    if (plan.p.M == 0 || plan.p.N == 0 || plan.p.tile_count == 0) return 0;
+    if (int rc = require_sm100()) return rc;
+    return launch_plan(plan, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int64_t kermac_b200_build_scratch_bytes(const KmBuildArgs* args) {
+    using namespace km;
+    BuildPlan plan;
+    if (make_plan(args, &plan)) return 0;
+    PackPlan pack;
+    plan_pack_operands(plan, &pack);
+    return pack.n ? (int64_t)(pack.floats[0] + pack.floats[1]) * 4 : 0;
+}
+
+extern "C" int kermac_b200_build_kernel_scratch(const KmBuildArgs* args, void* scratch, int64_t scratch_bytes, void* stream) {
+    using namespace km;
+    BuildPlan plan;
+    if (int rc = make_plan(args, &plan)) return rc;
+    if (plan.p.M == 0 || plan.p.N == 0 || plan.p.tile_count == 0) return 0;
+    if (int rc = require_sm100()) return rc;
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    PackPlan pack;
+    plan_pack_operands(plan, &pack);
+    const int64_t need = (int64_t)(pack.floats[0] + pack.floats[1]) * 4;
+    if (!pack.n || !scratch || !aligned16(scratch) || scratch_bytes < need) return launch_plan(plan, st);
+
+    pack.job[0].dst = static_cast<float*>(scratch);
+    pack.job[1].dst = pack.job[0].dst + pack.floats[0];
+    if (int rc = launch_pack(pack.job, pack.n, plan.p.K, st)) return rc;
+    // the same call on the packed operands (plan.swapped: the kernel's A is the caller's b)
+    KmBuildArgs packed = *args;
+    const PackJob* next = pack.job;
+    auto use_a = [&](const PackJob& j) { packed.a = j.dst; packed.a_stride_m = 1; packed.a_stride_k = j.pitch; packed.a_stride_l = j.dst_l; };
+    auto use_b = [&](const PackJob& j) { packed.b = j.dst; packed.b_stride_n = 1; packed.b_stride_k = j.pitch; packed.b_stride_l = j.dst_l; };
+    if (pack.a) { if (plan.swapped) use_b(*next); else use_a(*next); }
+    if (pack.b) {
+        if (!pack.shared) ++next;
+        if (!pack.a) next = pack.job;
+        if (plan.swapped) use_a(*next); else use_b(*next);
+    }
+    if (int rc = make_plan(&packed, &plan)) return rc;
+    return launch_plan(plan, st);
 }
 
 extern "C" int64_t kermac_b200_build_tile_count(const KmBuildArgs* args) {

@@ -23,7 +23,8 @@ namespace {
 
 // Entry points of libkermac_b200.so, handed over by bind(): the library that ctypes loaded is the one called.
 struct Library {
-    int (*build)(const KmBuildArgs*, void*)               = nullptr;
+    int (*build)(const KmBuildArgs*, void*, int64_t, void*) = nullptr;
+    int64_t (*build_scratch)(const KmBuildArgs*)          = nullptr;
     int (*grad)(const KmGradArgs*, void*)                 = nullptr;
     int64_t (*grad_scratch)(const KmGradArgs*)            = nullptr;
     int (*matvec)(const KmMatvecArgs*, void*)             = nullptr;
@@ -164,7 +165,18 @@ PyObject* build(KmBuildArgs& args, const Chain& chain, PyObject* pa, PyObject* p
     args.inner_power    = chain.inner_power;
     args.outer_power    = chain.outer_power;
     args.kernel_type    = chain.kernel_type;
-    const int rc = g_lib.build(&args, c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream());
+    // Scratch only makes the call faster, so a full device does without it.  It belongs to the current stream,
+    // the one the launch goes to, and returns to torch's allocator in stream order.
+    at::Tensor scratch;
+    const int64_t need = g_lib.build_scratch(&args);
+    if (need > 0) {
+        try {
+            scratch = new_float({need / 4}, device);
+        } catch (const c10::OutOfMemoryError&) {
+        }
+    }
+    const int rc = g_lib.build(&args, scratch.defined() ? scratch.data_ptr() : nullptr, scratch.defined() ? need : 0,
+                               c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream());
     return finish(rc, made, pout != Py_None ? pout : nullptr);
 }
 
@@ -337,11 +349,17 @@ PyObject* call_kernel_matvec(PyObject*, PyObject* const* v, Py_ssize_t n) {
     args.inner_power    = chain.inner_power;
     args.outer_power    = chain.outer_power;
     args.kernel_type    = chain.kernel_type;
+    // A device too full for all of the scratch does without: only an explicit split cannot.
     at::Tensor scratch;
-    const int64_t need = g_lib.matvec_scratch(&args);
+    int64_t need = g_lib.matvec_scratch(&args);
     if (need > 0) {
-        scratch            = new_float({need / 4}, device);
-        args.scratch       = static_cast<float*>(scratch.data_ptr());
+        try {
+            scratch = new_float({(need + 3) / 4}, device);
+        } catch (const c10::OutOfMemoryError&) {
+            need = args.split_m > 1 ? 4 * static_cast<int64_t>(args.split_m) * L * N * O : 0;
+            if (need > 0) scratch = new_float({need / 4}, device);
+        }
+        args.scratch       = need > 0 ? static_cast<float*>(scratch.data_ptr()) : nullptr;
         args.scratch_bytes = need;
     }
     const int rc = g_lib.matvec(&args, c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream());
@@ -412,11 +430,11 @@ PyObject* call_cdist_grad(PyObject*, PyObject* const* v, Py_ssize_t n) {
     return finish(rc, made, v[4] != Py_None ? v[4] : nullptr);
 }
 
-// bind((addresses of the five entry points), (InnerOperator, PowerType, KernelType))
+// bind((addresses of the six entry points), (InnerOperator, PowerType, KernelType))
 PyObject* call_bind(PyObject*, PyObject* args) {
-    unsigned long long build_fn, grad_fn, grad_scratch_fn, matvec_fn, matvec_scratch_fn;
+    unsigned long long build_fn, build_scratch_fn, grad_fn, grad_scratch_fn, matvec_fn, matvec_scratch_fn;
     PyObject* types[3];
-    if (!PyArg_ParseTuple(args, "(KKKKK)(OOO)", &build_fn, &grad_fn, &grad_scratch_fn, &matvec_fn, &matvec_scratch_fn,
+    if (!PyArg_ParseTuple(args, "(KKKKKK)(OOO)", &build_fn, &build_scratch_fn, &grad_fn, &grad_scratch_fn, &matvec_fn, &matvec_scratch_fn,
                           &types[0], &types[1], &types[2]))
         return nullptr;
     const char* names[5] = {"_inner_operator", "_inner_power", "_outer_power", "_kernel_type", "_value_"};
@@ -430,6 +448,7 @@ PyObject* call_bind(PyObject*, PyObject* args) {
     g_lib.grad_scratch   = reinterpret_cast<decltype(g_lib.grad_scratch)>(grad_scratch_fn);
     g_lib.matvec         = reinterpret_cast<decltype(g_lib.matvec)>(matvec_fn);
     g_lib.matvec_scratch = reinterpret_cast<decltype(g_lib.matvec_scratch)>(matvec_scratch_fn);
+    g_lib.build_scratch  = reinterpret_cast<decltype(g_lib.build_scratch)>(build_scratch_fn);
     g_lib.build          = reinterpret_cast<decltype(g_lib.build)>(build_fn);
     Py_RETURN_NONE;
 }
