@@ -358,20 +358,24 @@ __global__ void __launch_bounds__(G_THREADS, grad_min_blocks(OT, NT)) grad_kerne
     }
 }
 
-// out[l][o][n][m] = sum over splits of partial[split][l][o][n][m] (dense partials).
+// out[l][o][n][m] = sum over splits of partial[split][l][o][n][m] (dense partials), in split order.  Bound by
+// reading the partials: indices are 32-bit wherever they fit, because the 64-bit divisions take longer than the
+// loads, and four splits are loaded ahead of the adds.
+template <typename Index>
 __global__ void __launch_bounds__(256) grad_reduce_kernel(const float* __restrict__ partial, float* __restrict__ out,
                                                           int M, int N, int O, int L, int splits, long long split_stride,
                                                           long long o_sn, long long o_so, long long o_sl) {
-    const long long total = (long long)L * O * N * M;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
+    const Index total = (Index)L * O * N * M;
+    const Index step  = (Index)gridDim.x * blockDim.x;
+    for (Index i = blockIdx.x * (Index)blockDim.x + threadIdx.x; i < total; i += step) {
         float s = 0.0f;
+#pragma unroll 4
         for (int sp = 0; sp < splits; ++sp) s += partial[sp * split_stride + i];
-        long long r = i;
-        const int m = (int)(r % M); r /= M;
-        const int n = (int)(r % N); r /= N;
-        const int o = (int)(r % O); r /= O;
-        const int l = (int)r;
-        out[l * o_sl + o * o_so + n * o_sn + m] = s;
+        Index r = i;
+        const Index m = r % M; r /= M;
+        const Index n = r % N; r /= N;
+        const Index o = r % O; r /= O;
+        out[(long long)r * o_sl + (long long)o * o_so + (long long)n * o_sn + m] = s;
     }
 }
 
@@ -405,6 +409,43 @@ struct GradPlan {
     int splits_wanted;
     long long partial_elems;   // elements of one dense partial result
 };
+
+// Preferred k split: the smallest within 0.5 % of the least estimated time.  An SM works through its share of
+// the blocks, ceil(blocks / SMs), two at a time, or one by one 10 % slower per slab (the tensor-core kernel: one
+// at a time); a slab of 32 k takes about the time below, a block 2.5 us besides, and the partial results of a
+// split are written and read back at about 5 TB/s.  Measured on B200, us, against the rule before (whole waves,
+// at least 8 slabs a block, at most 64 splits), for K, M, N, O, p:
+//   1000, 200, 50, 4, 1.5:  101 (2 splits) -> 17 (32)     2000, 64, 64, 8, 1:     54 (5) -> 17 (63)
+//   500, 64, 16, 4, 1:      68 (1) -> 13 (16)             30000, 64, 16, 16, 1.7: 74 (59) -> 46 (134)
+//   500, 100, 30, 32, 1:    35 (1) -> 15 (16)             8000, 500, 20, 4, 1.7:  175 (31) -> 156 (36)
+//   30000, 4096, 256, 4, 1: 6244 (8) -> 6237 (4)          64, 1000, 1000, 16, 1.5: 57 (1) either way
+int preferred_split(const GradPlan& plan, int norm_type, bool square_root) {
+    const GradParams& p    = plan.p;
+    const long long blocks = (long long)p.tiles_m * p.tiles_n * p.o_chunks * p.L;
+    const long long slabs  = ceil_div_ll(p.K, G_BK);
+    const long long sms    = sm_count();
+    const double bytes     = 4.0 * p.L * p.O * p.N * p.M;
+    if (blocks <= 0 || slabs <= 1) return 1;
+    double slab_us = 2.0;
+    if (!plan.tensor) {
+        slab_us = 0.6 + 0.16 * plan.nt * (1 + plan.ot);
+        if (norm_type == KM_NORM_P) slab_us += (square_root ? 0.5 : 1.4) * plan.nt;
+    }
+    auto cost = [&](long long s) {
+        const long long per_split = ceil_div_ll(slabs, s);
+        const long long share     = ceil_div_ll(blocks * ceil_div_ll(slabs, per_split), sms);
+        const double units        = plan.tensor ? (double)share : 0.9 * share + ((share & 1) ? 0.1 : 0.0);
+        return units * per_split * slab_us + 2.5 * share + (s > 1 ? 3.0 + (2.0 * s + 1.0) * bytes / 5e6 : 0.0);
+    };
+    // more than 16 blocks per SM gain nothing, and partial results stay within 512 MB
+    long long last = 1;
+    while (last < slabs && blocks * (last + 1) <= 16 * sms && bytes * (last + 1) <= 512e6) ++last;
+    double least = cost(1);
+    for (long long s = 2; s <= last; ++s) least = cost(s) < least ? cost(s) : least;
+    for (long long s = 1; s <= last; ++s)
+        if (cost(s) <= 1.005 * least) return (int)s;
+    return 1;
+}
 
 int make_grad_plan(const KmGradArgs* a, GradPlan* plan) {
     if (!a) return fail(KM_ERR_NULL_POINTER, "args is NULL");
@@ -454,27 +495,7 @@ int make_grad_plan(const KmGradArgs* a, GradPlan* plan) {
     if ((long long)p.tiles_m * p.tiles_n > (1LL << 26)) return fail(KM_ERR_TOO_LARGE, "too many output tiles");
     if (p.o_chunks > 65535) return fail(KM_ERR_TOO_LARGE, "too many output channels");
 
-    // Preferred k split.  Thread blocks run two per SM, in waves of `slots`; a launch of `blocks`
-    // blocks takes ceil(blocks / slots) waves however full the last one is.  Among the splits the
-    // k range allows (at least 8 slabs of k per block, at most 64 splits) take the smallest one
-    // whose waves are within 2 % of the best filled; a launch that already fills its waves to 90 %
-    // is left alone (every split costs a partial result written and read back).
-    const long long blocks = (long long)p.tiles_m * p.tiles_n * p.o_chunks * p.L;
-    const long long slots  = (long long)(plan->tensor ? gt_blocks_per_sm(plan->ot) : grad_min_blocks(plan->ot, plan->nt)) * sm_count();
-    auto fill = [&](long long s) {
-        const long long b = blocks * s;
-        return (double)b / (double)(ceil_div_ll(b, slots) * slots);
-    };
-    int want = 1;
-    if (blocks > 0 && fill(1) < 0.90) {
-        int max_s = (int)(p.K / (8 * G_BK));
-        if (max_s > 64) max_s = 64;
-        double best = fill(1);
-        for (int s = 2; s <= max_s; ++s) best = fill(s) > best ? fill(s) : best;
-        for (int s = 1; s <= max_s; ++s)
-            if (fill(s) >= best - 0.02) { want = s; break; }
-    }
-    plan->splits_wanted = want;
+    plan->splits_wanted = preferred_split(*plan, a->norm_type, !a->p.ptr && a->p.value == 1.5f);
     plan->partial_elems = (long long)p.L * p.O * p.N * p.M;
     return 0;
 }
@@ -560,8 +581,10 @@ extern "C" int kermac_b200_cdist_grad(const KmGradArgs* args, void* stream) {
     }
     if (splits > 1) {
         const long long total = plan.partial_elems;
-        int blocks = (int)(ceil_div_ll(total, 256) < 4LL * sm_count() ? ceil_div_ll(total, 256) : 4LL * sm_count());
-        grad_reduce_kernel<<<blocks, 256, 0, st>>>(p.E, args->out, p.M, p.N, p.O, p.L, splits, plan.partial_elems,
+        int blocks = (int)(ceil_div_ll(total, 256) < 8LL * sm_count() ? ceil_div_ll(total, 256) : 8LL * sm_count());
+        // (below 2^31 the grid stride cannot overflow 32 unsigned bits)
+        auto reduce = total < (1LL << 31) ? grad_reduce_kernel<unsigned int> : grad_reduce_kernel<long long>;
+        reduce<<<blocks, 256, 0, st>>>(p.E, args->out, p.M, p.N, p.O, p.L, splits, plan.partial_elems,
                                                    args->out_stride_n, args->out_stride_o, args->out_stride_l);
         if (int rc = cuda_status(cudaGetLastError(), "launch of grad_reduce_kernel")) return rc;
     }
