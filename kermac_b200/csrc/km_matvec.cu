@@ -19,6 +19,7 @@
 #include "km_build_tma.cuh"
 #include "km_host.h"
 #include "km_mbar.cuh"
+#include "km_pack.h"
 #include "km_tcgen05.cuh"
 
 namespace km {
@@ -644,7 +645,56 @@ struct MatvecPlan {
     bool tma;                 // tensor kernel with TMA operand staging
     int splits_wanted;
     long long partial_elems;
+    PackJob pack[2];          // operands worth rewriting k-major first
+    int packs;
+    bool pack_a, pack_b;
+    long long pack_floats[2];
 };
+
+// Preferred m split: the smallest within 0.5 % of the least estimated time.  An SM works through its share of the
+// blocks two at a time, or one by one about 13 % slower per chunk, so what counts is the largest share,
+// ceil(blocks / SMs), times the chunks of a block; a block costs about 1.5 us besides and the reduction 3 us and
+// a little per partial result.  A chunk of 128 x 128 pairs takes about 4.5 + 0.155 K us.  Measured with the
+// operands contiguous along the points, us, against the rule before (whole waves of two blocks per SM, at least
+// 8 chunks a block, at most 32 splits):
+//   M 10007  N 1009  K 27:  72 (10 splits) -> 49 (16)       M 1000   N 300  K 27: 66 (1) -> 17 (8)
+//   M 10007  N 1009  K 200: 287 (10) -> 169 (79)            M 100000 N 100  K 64: 332 (32) -> 94 (261)
+//   M 20000  N 20000 K 64:  1962 (1) -> 1873 (16)           M 131072 N 65536 K 64: 4 splits either way
+int preferred_split(const MatvecParams& p) {
+    const long long blocks = (long long)p.tiles_n * p.o_chunks * p.L;
+    const long long chunks = ceil_div_ll(p.M, MV_TILE);
+    const long long sms    = sm_count();
+    const long long result = (long long)p.L * p.N * p.O * 4;
+    if (blocks <= 0 || chunks <= 1) return 1;
+    auto cost = [&](long long s) {
+        const long long per_split = ceil_div_ll(chunks, s);
+        const long long share     = ceil_div_ll(blocks * ceil_div_ll(chunks, per_split), sms);
+        return (0.9 * share + ((share & 1) ? 0.12 : 0.0)) * per_split * (4.5 + 0.155 * p.K) + 1.5 * share +
+               (s > 1 ? 3.0 + 0.05 * s : 0.0);
+    };
+    // more than 32 blocks per SM gain nothing, and partial results stay within 512 MB
+    long long last = 1;
+    while (last < chunks && blocks * (last + 1) <= 32 * sms && result * (last + 1) <= (512LL << 20)) ++last;
+    double least = cost(1);
+    for (long long s = 2; s <= last; ++s) least = cost(s) < least ? cost(s) : least;
+    for (long long s = 1; s <= last; ++s)
+        if (cost(s) <= 1.005 * least) return (int)s;
+    return 1;
+}
+
+// How the operands are staged: 16-byte copies, and TMA where the inner step gains from it.
+void choose_staging(MatvecPlan* plan) {
+    const MatvecParams& p = plan->p;
+    plan->avec = (p.a_sm == 1) && aligned16(p.A) && (p.a_sk % 4 == 0 || p.K <= 1) && (p.a_sl % 4 == 0);
+    plan->bvec = (p.b_sn == 1) && aligned16(p.B) && (p.b_sk % 4 == 0 || p.K <= 1) && (p.b_sl % 4 == 0);
+    // Measured on B200 (K=64, M=N=131072, O=16): TMA staging takes the (b-a)^2 walk from 345 to
+    // 323 ms per 262144^2 pairs; for |b-a| and |b-a|^p it changes nothing (90.9 vs 90.9 ms,
+    // 448 vs 450 ms), so those keep the cp.async pipeline, which accepts every layout.
+    const bool tma_inner = (p.inner_id == IN_DIFF_SQUARE || p.inner_id == IN_DOT_NOOP);
+    plan->tma = plan->tensor && tma_inner && p.K >= 1 && p.M > 0 && p.N > 0 &&
+                tma_operand_ok(p.A, p.a_sm, p.a_sk, p.a_sl, p.K, p.L) &&
+                tma_operand_ok(p.B, p.b_sn, p.b_sk, p.b_sl, p.K, p.L);
+}
 
 int make_matvec_plan(const KmMatvecArgs* a, MatvecPlan* plan) {
     if (!a) return fail(KM_ERR_NULL_POINTER, "args is NULL");
@@ -693,36 +743,30 @@ int make_matvec_plan(const KmMatvecArgs* a, MatvecPlan* plan) {
     p.tiles_n  = (int)ceil_div_ll(p.N, MV_TILE);
     p.o_chunks = (int)ceil_div_ll(p.O > 0 ? p.O : 1, ot);
     if (p.o_chunks > 65535) return fail(KM_ERR_TOO_LARGE, "too many output channels");
-    plan->avec = (p.a_sm == 1) && aligned16(p.A) && (p.a_sk % 4 == 0 || p.K <= 1) && (p.a_sl % 4 == 0);
-    plan->bvec = (p.b_sn == 1) && aligned16(p.B) && (p.b_sk % 4 == 0 || p.K <= 1) && (p.b_sl % 4 == 0);
-    // Measured on B200 (K=64, M=N=131072, O=16): TMA staging takes the (b-a)^2 walk from 345 to
-    // 323 ms per 262144^2 pairs; for |b-a| and |b-a|^p it changes nothing (90.9 vs 90.9 ms,
-    // 448 vs 450 ms), so those keep the cp.async pipeline, which accepts every layout.
-    const bool tma_inner = (p.inner_id == IN_DIFF_SQUARE || p.inner_id == IN_DOT_NOOP);
-    plan->tma = plan->tensor && tma_inner && p.K >= 1 && p.M > 0 && p.N > 0 &&
-                tma_operand_ok(p.A, p.a_sm, p.a_sk, p.a_sl, p.K, p.L) &&
-                tma_operand_ok(p.B, p.b_sn, p.b_sk, p.b_sl, p.K, p.L);
-
-    // Preferred m split: fill whole waves of 2 blocks per SM when the row tiles alone
-    // leave more than ~10 % of a wave idle.
-    const long long blocks = (long long)p.tiles_n * p.o_chunks * p.L;
-    const long long slots  = 2LL * sm_count();
-    int want = 1;
-    if (blocks > 0) {
-        const double waves = (double)blocks / (double)slots;
-        const double eff   = waves / (double)ceil_div_ll(blocks, slots);
-        if (eff < 0.9) {
-            // smallest split that brings the efficiency above 0.95, capped by chunk count
-            const int max_split = (int)ceil_div_ll(p.M > 0 ? p.M : 1, 8 * MV_TILE);
-            for (int s = 2; s <= 32 && s <= max_split; ++s) {
-                const double w = (double)(blocks * s) / (double)slots;
-                if (w / (double)ceil_div_ll(blocks * s, slots) >= 0.95) { want = s; break; }
-                want = s;
-            }
-        }
-    }
-    plan->splits_wanted = want;
+    choose_staging(plan);
+    plan->splits_wanted = preferred_split(p);
     plan->partial_elems = (long long)p.L * p.N * p.O;
+
+    // An operand that is not contiguous along its points is copied word by word, once per 128 x 128 tile.
+    // Measured on B200 with rows / contiguous points, us: laplace L2 10007 x 1009 x 200 362 / 287,
+    // 20000 x 20000 x 64 2494 / 1962; laplace L1 2663 / 2245; so a pair and feature costs about 2e-14 s less
+    // (|.| 1.6e-14; the fractional power, which takes ten times as long, is left out of the account).
+    plan->packs  = 0;
+    plan->pack_a = !plan->avec;
+    plan->pack_b = !plan->bvec;
+    plan->pack_floats[0] = plan->pack_floats[1] = 0;
+    if (p.K >= 1 && p.M > 0 && p.N > 0 && (plan->pack_a || plan->pack_b) && p.inner_id != IN_DIFF_POW) {
+        if (plan->pack_a) {
+            plan->pack_floats[0] = plan_pack(&plan->pack[0], p.A, p.M, p.K, p.L, p.a_sm, p.a_sk, p.a_sl);
+            ++plan->packs;
+        }
+        if (plan->pack_b) {
+            const int i = plan->packs++;
+            plan->pack_floats[i] = plan_pack(&plan->pack[i], p.B, p.N, p.K, p.L, p.b_sn, p.b_sk, p.b_sl);
+        }
+        const double gain = (p.inner_id == IN_DIFF_ABS ? 1.6e-14 : 2e-14) * p.o_chunks * p.L;
+        if ((double)p.M * p.N * p.K * gain < pack_seconds(plan->pack_floats[0] + plan->pack_floats[1])) plan->packs = 0;
+    }
     return 0;
 }
 
@@ -739,13 +783,20 @@ int matvec_take_wait_flag() {
 }
 }  // namespace km
 
+namespace km {
+namespace {
+// The packed operands follow the partial results in the scratch.
+int64_t pack_offset(int64_t partial_bytes) { return (partial_bytes + 127) & ~int64_t(127); }
+}  // namespace
+}  // namespace km
+
 extern "C" int64_t kermac_b200_kernel_matvec_scratch_bytes(const KmMatvecArgs* args) {
     using namespace km;
     MatvecPlan plan;
     if (make_matvec_plan(args, &plan)) return 0;
-    int splits = args->split_m > 0 ? args->split_m : plan.splits_wanted;
-    if (splits <= 1) return 0;
-    return (int64_t)splits * plan.partial_elems * 4;
+    const int splits      = args->split_m > 0 ? args->split_m : plan.splits_wanted;
+    const int64_t partial = splits > 1 ? (int64_t)splits * plan.partial_elems * 4 : 0;
+    return plan.packs ? pack_offset(partial) + (plan.pack_floats[0] + plan.pack_floats[1]) * 4 : partial;
 }
 
 extern "C" int kermac_b200_kernel_matvec(const KmMatvecArgs* args, void* stream) {
@@ -765,6 +816,25 @@ extern "C" int kermac_b200_kernel_matvec(const KmMatvecArgs* args, void* stream)
                 return fail(KM_ERR_BAD_SHAPE, "split_m=%d needs %lld bytes of scratch, got %lld", splits, (long long)need,
                             (long long)(args->scratch ? args->scratch_bytes : 0));
             splits = 1;
+        }
+    }
+    if (plan.packs) {
+        // scratch that holds the partial results only, or is not aligned, leaves the operands where they are
+        const int64_t offset = pack_offset(splits > 1 ? (int64_t)splits * plan.partial_elems * 4 : 0);
+        const int64_t need   = offset + (plan.pack_floats[0] + plan.pack_floats[1]) * 4;
+        if (args->scratch && aligned16(args->scratch) && args->scratch_bytes >= need) {
+            plan.pack[0].dst = reinterpret_cast<float*>(static_cast<char*>(args->scratch) + offset);
+            plan.pack[1].dst = plan.pack[0].dst + plan.pack_floats[0];
+            if (int rc = launch_pack(plan.pack, plan.packs, p.K, st)) return rc;
+            if (plan.pack_a) {
+                const PackJob& j = plan.pack[0];
+                p.A = j.dst; p.a_sm = 1; p.a_sk = j.pitch; p.a_sl = j.dst_l;
+            }
+            if (plan.pack_b) {
+                const PackJob& j = plan.pack[plan.packs - 1];
+                p.B = j.dst; p.b_sn = 1; p.b_sk = j.pitch; p.b_sl = j.dst_l;
+            }
+            choose_staging(&plan);
         }
     }
     const int chunks = (int)ceil_div_ll(p.M > 0 ? p.M : 1, MV_TILE);

@@ -161,8 +161,13 @@ def kernel_matvec(
     need = int(_native.lib().kermac_b200_kernel_matvec_scratch_bytes(ctypes.byref(args)))
     scratch = None
     if need > 0:
-        scratch = torch.empty(need // 4, dtype=torch.float32, device=a.device)
-        args.scratch, args.scratch_bytes = scratch.data_ptr(), need
+        try:
+            scratch = torch.empty(need // 4, dtype=torch.float32, device=a.device)
+        except torch.cuda.OutOfMemoryError:      # all of it only makes the call faster; an explicit split needs its part
+            need = 4 * args.split_m * args.l * args.n * args.o if args.split_m > 1 else 0
+            scratch = torch.empty(need // 4, dtype=torch.float32, device=a.device) if need else None
+        if scratch is not None:
+            args.scratch, args.scratch_bytes = scratch.data_ptr(), need
     if debug:
         print(f'(Kermac Debug) Launching kernel_matvec split scratch bytes={need}')
     _native.launch_matvec(args, stream_ptr)

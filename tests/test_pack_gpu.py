@@ -64,3 +64,25 @@ def test_one_matrix_is_packed_once_and_stays_symmetric():
     other = torch.empty_like(out)
     _call(x, x, other, 2.0, scratch_bytes=0)
     assert torch.equal(out, other)
+
+
+@pytest.mark.parametrize("desc", ["l1", "l2"])
+@pytest.mark.parametrize("layouts", [("rows", "rows"), ("cols", "off"), ("off", "cols")])
+@pytest.mark.parametrize("shape", [((), 10007, 1009, 27, 5), ((), 5000, 6001, 40, 17), ((3,), 4100, 2000, 65, 2)])
+def test_matvec_on_packed_operands(shape, layouts, desc):
+    # the operands as given against the same points already contiguous along the points: the same kernel
+    # arithmetic and the same split over m, so the same bits
+    lead, M, N, K, O = shape
+    descriptor = kermac.kernel_descriptor_laplace_l1 if desc == "l1" else kermac.kernel_descriptor_laplace_l2
+    gen = torch.Generator().manual_seed(K)
+    a, c = _points(gen, lead, M, K, layouts[0]), torch.randn(*lead, O, M, generator=gen).cuda()
+    for b in (_points(gen, lead, N, K, layouts[1]), _points(gen, (), N, K, layouts[1])):
+        def aligned(x):
+            buf = torch.zeros(*x.shape[:-2], K, (x.shape[-2] + 3) // 4 * 4, device="cuda")
+            buf[..., :x.shape[-2]] = x.transpose(-1, -2)
+            return buf[..., :x.shape[-2]].transpose(-1, -2)
+        got = kermac.kernel_matvec(descriptor, a, b, c, bandwidth=8.0)
+        assert torch.equal(got, kermac.kernel_matvec(descriptor, aligned(a), aligned(b), c, bandwidth=8.0))
+        split = kermac.kernel_matvec(descriptor, a, b, c, bandwidth=8.0, split_m=3)
+        assert torch.allclose(got, split, rtol=0.0, atol=float(got.abs().max()) * 2e-6)    # sums of M terms, regrouped
+    assert _native.device_error_flag() == 0
