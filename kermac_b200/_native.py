@@ -185,6 +185,15 @@ def lib() -> C.CDLL:
 _call = None
 
 
+def _bind_torch_call(call, handle) -> None:
+    """Hands the C-ABI entry points of `handle` and the enum classes to the extension."""
+    from .build_a_kernel import InnerOperator, KernelType, PowerType
+    names = ("build_kernel_scratch", "build_scratch_bytes", "cdist_grad", "cdist_grad_scratch_bytes", "kernel_matvec",
+             "kernel_matvec_scratch_bytes")
+    addresses = tuple(C.cast(getattr(handle, "kermac_b200_" + name), C.c_void_p).value for name in names)
+    call.bind(addresses, (InnerOperator, PowerType, KernelType))
+
+
 def torch_call():
     """The bound `_torch_call` extension, or False where it cannot be loaded."""
     global _call
@@ -200,14 +209,7 @@ def torch_call():
                                   "about 20 us more; rebuild with `make -C kermac_b200/csrc`", RuntimeWarning)
                     _call = False
                     return _call
-                from .build_a_kernel import InnerOperator, KernelType, PowerType
-                address = lambda fn: C.cast(fn, C.c_void_p).value       # noqa: E731
-                _torch_call.bind((address(handle.kermac_b200_build_kernel_scratch),
-                                  address(handle.kermac_b200_build_scratch_bytes), address(handle.kermac_b200_cdist_grad),
-                                  address(handle.kermac_b200_cdist_grad_scratch_bytes),
-                                  address(handle.kermac_b200_kernel_matvec),
-                                  address(handle.kermac_b200_kernel_matvec_scratch_bytes)),
-                                 (InnerOperator, PowerType, KernelType))
+                _bind_torch_call(_torch_call, handle)
                 _call = _torch_call
     return _call
 

@@ -117,6 +117,17 @@ PyObject* finish(int rc, const at::Tensor& result, PyObject* given) {
     return THPVariable_Wrap(result);
 }
 
+// Releases the interpreter lock for its scope: a launch waits when the queue is full, a first launch loads its
+// module, and torch's allocator may synchronise, while a data loader, a Python host callback in the stream or the
+// thread of another GPU needs the lock.  Inside, nothing touches a Python object or a tensor the caller owns.
+struct Unlocked {
+    PyThreadState* state = PyEval_SaveThread();
+    Unlocked() = default;
+    Unlocked(const Unlocked&) = delete;
+    Unlocked& operator=(const Unlocked&) = delete;
+    ~Unlocked() { PyEval_RestoreThread(state); }
+};
+
 at::Tensor new_float(c10::IntArrayRef shape, int device) {
     return at::Tensor(at::detail::empty_cuda(shape, at::kFloat, c10::Device(c10::kCUDA, static_cast<c10::DeviceIndex>(device)),
                                              std::nullopt));
@@ -135,15 +146,14 @@ PyObject* build(KmBuildArgs& args, const Chain& chain, PyObject* pa, PyObject* p
     if (!standard_layout(*a.t) || !standard_layout(*b.t)) return decline();
     const int64_t M = a.t->size(-2), K = a.t->size(-1), N = b.t->size(-2);
     if (b.t->size(-1) != K) return decline();
-    at::Tensor made;
-    if (pout != Py_None) {
+    const bool given = pout != Py_None;
+    if (given) {
         if (!read_operand(pout, 2, device, c) || !merge_batch(L, c.batch) || !standard_layout(*c.t)) return decline();
         if (c.t->size(-2) != M || c.t->size(-1) != N || (c.batch != L && L != 1)) return decline();
-    } else {
-        made = new_float({L, M, N}, device);
-        c.t  = &made;
-        c.batch_stride = L != 1 ? made.stride(0) : 0;
-        if (!standard_layout(made)) return decline();
+        args.out = static_cast<float*>(c.t->data_ptr());
+        args.out_stride_m = c.t->stride(-2);
+        args.out_stride_n = c.t->stride(-1);
+        args.out_stride_l = c.batch_stride;
     }
     args.m = static_cast<int32_t>(M);
     args.n = static_cast<int32_t>(N);
@@ -157,27 +167,35 @@ PyObject* build(KmBuildArgs& args, const Chain& chain, PyObject* pa, PyObject* p
     args.b_stride_n = b.t->stride(-2);
     args.b_stride_k = b.t->stride(-1);
     args.b_stride_l = b.batch_stride;
-    args.out = static_cast<float*>(c.t->data_ptr());
-    args.out_stride_m = c.t->stride(-2);
-    args.out_stride_n = c.t->stride(-1);
-    args.out_stride_l = c.batch_stride;
     args.inner_operator = chain.inner_operator;
     args.inner_power    = chain.inner_power;
     args.outer_power    = chain.outer_power;
     args.kernel_type    = chain.kernel_type;
-    // Scratch only makes the call faster, so a full device does without it.  It belongs to the current stream,
-    // the one the launch goes to, and returns to torch's allocator in stream order.
-    at::Tensor scratch;
-    const int64_t need = g_lib.build_scratch(&args);
-    if (need > 0) {
-        try {
-            scratch = new_float({need / 4}, device);
-        } catch (const c10::OutOfMemoryError&) {
+    at::Tensor made;
+    int rc;
+    {
+        Unlocked unlocked;
+        if (!given) {
+            made = new_float({L, M, N}, device);
+            args.out = static_cast<float*>(made.data_ptr());
+            args.out_stride_m = made.stride(-2);
+            args.out_stride_n = made.stride(-1);
+            args.out_stride_l = L != 1 ? made.stride(0) : 0;
         }
+        // Scratch only makes the call faster, so a full device does without it.  It belongs to the current stream,
+        // the one the launch goes to, and returns to torch's allocator in stream order.
+        at::Tensor scratch;
+        const int64_t need = g_lib.build_scratch(&args);
+        if (need > 0) {
+            try {
+                scratch = new_float({need / 4}, device);
+            } catch (const c10::OutOfMemoryError&) {
+            }
+        }
+        rc = g_lib.build(&args, scratch.defined() ? scratch.data_ptr() : nullptr, scratch.defined() ? need : 0,
+                         c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream());
     }
-    const int rc = g_lib.build(&args, scratch.defined() ? scratch.data_ptr() : nullptr, scratch.defined() ? need : 0,
-                               c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream());
-    return finish(rc, made, pout != Py_None ? pout : nullptr);
+    return finish(rc, made, given ? pout : nullptr);
 }
 
 bool build_overridden() {
@@ -316,14 +334,14 @@ PyObject* call_kernel_matvec(PyObject*, PyObject* const* v, Py_ssize_t n) {
     if (!standard_layout(*a.t) || !standard_layout(*b.t) || !standard_layout(*c.t) || c.t->stride(-1) != 1) return decline();
     const int64_t M = a.t->size(-2), K = a.t->size(-1), N = b.t->size(-2), O = c.t->size(-2);
     if (b.t->size(-1) != K || c.t->size(-1) != M) return decline();
-    at::Tensor made;
-    if (v[4] != Py_None) {
+    const bool given = v[4] != Py_None;
+    if (given) {
         if (!read_operand(v[4], 2, device, y) || !merge_batch(L, y.batch)) return decline();
         if (y.t->size(-2) != N || y.t->size(-1) != O || (y.batch != L && L != 1)) return decline();
-    } else {
-        made = new_float({L, N, O}, device);
-        y.t  = &made;
-        y.batch_stride = L != 1 ? made.stride(0) : 0;
+        args.y = static_cast<float*>(y.t->data_ptr());
+        args.y_stride_n = y.t->stride(-2);
+        args.y_stride_o = y.t->stride(-1);
+        args.y_stride_l = y.batch_stride;
     }
     args.m = static_cast<int32_t>(M);
     args.n = static_cast<int32_t>(N);
@@ -341,29 +359,37 @@ PyObject* call_kernel_matvec(PyObject*, PyObject* const* v, Py_ssize_t n) {
     args.c = static_cast<const float*>(c.t->data_ptr());
     args.ldc        = c.t->stride(-2);
     args.c_stride_l = c.batch_stride;
-    args.y = static_cast<float*>(y.t->data_ptr());
-    args.y_stride_n = y.t->stride(-2);
-    args.y_stride_o = y.t->stride(-1);
-    args.y_stride_l = y.batch_stride;
     args.inner_operator = chain.inner_operator;
     args.inner_power    = chain.inner_power;
     args.outer_power    = chain.outer_power;
     args.kernel_type    = chain.kernel_type;
-    // A device too full for all of the scratch does without: only an explicit split cannot.
-    at::Tensor scratch;
-    int64_t need = g_lib.matvec_scratch(&args);
-    if (need > 0) {
-        try {
-            scratch = new_float({(need + 3) / 4}, device);
-        } catch (const c10::OutOfMemoryError&) {
-            need = args.split_m > 1 ? 4 * static_cast<int64_t>(args.split_m) * L * N * O : 0;
-            if (need > 0) scratch = new_float({need / 4}, device);
+    at::Tensor made;
+    int rc;
+    {
+        Unlocked unlocked;
+        if (!given) {
+            made = new_float({L, N, O}, device);
+            args.y = static_cast<float*>(made.data_ptr());
+            args.y_stride_n = made.stride(-2);
+            args.y_stride_o = made.stride(-1);
+            args.y_stride_l = L != 1 ? made.stride(0) : 0;
         }
-        args.scratch       = need > 0 ? static_cast<float*>(scratch.data_ptr()) : nullptr;
-        args.scratch_bytes = need;
+        // A device too full for all of the scratch does without: only an explicit split cannot.
+        at::Tensor scratch;
+        int64_t need = g_lib.matvec_scratch(&args);
+        if (need > 0) {
+            try {
+                scratch = new_float({(need + 3) / 4}, device);
+            } catch (const c10::OutOfMemoryError&) {
+                need = args.split_m > 1 ? 4 * static_cast<int64_t>(args.split_m) * L * N * O : 0;
+                if (need > 0) scratch = new_float({need / 4}, device);
+            }
+            args.scratch       = need > 0 ? static_cast<float*>(scratch.data_ptr()) : nullptr;
+            args.scratch_bytes = need;
+        }
+        rc = g_lib.matvec(&args, c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream());
     }
-    const int rc = g_lib.matvec(&args, c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream());
-    return finish(rc, made, v[4] != Py_None ? v[4] : nullptr);
+    return finish(rc, made, given ? v[4] : nullptr);
 }
 
 // cdist_grad(a, b, c, d, out, p, contraction code)
@@ -383,17 +409,17 @@ PyObject* call_cdist_grad(PyObject*, PyObject* const* v, Py_ssize_t n) {
     const at::Tensor &a = *op[0].t, &b = *op[1].t, &c = *op[2].t, &d = *op[3].t;
     const int64_t K = a.size(-2), M = a.size(-1), N = b.size(-2), O = c.size(-2);
     if (b.size(-1) != K || c.size(-1) != K || d.size(-2) != N || d.size(-1) != M) return decline();
-    at::Tensor made;
+    const bool given = v[4] != Py_None;
     Operand out;
-    if (v[4] != Py_None) {
+    if (given) {
         if (!read_operand(v[4], 3, device, out) || !merge_batch(L, out.batch)) return decline();
         const at::Tensor& e = *out.t;
         if (e.size(-3) != O || e.size(-2) != N || e.size(-1) != M || e.stride(-1) != 1) return decline();
         if (out.batch != L) return decline();
-    } else {
-        made  = new_float({L, O, N, M}, device);
-        out.t = &made;
-        out.batch_stride = L != 1 ? made.stride(0) : 0;
+        args.out = static_cast<float*>(e.data_ptr());
+        args.out_stride_n = e.stride(-2);
+        args.out_stride_o = e.stride(-3);
+        args.out_stride_l = out.batch_stride;
     }
     args.m = static_cast<int32_t>(M);
     args.n = static_cast<int32_t>(N);
@@ -412,22 +438,30 @@ PyObject* call_cdist_grad(PyObject*, PyObject* const* v, Py_ssize_t n) {
     args.d = static_cast<const float*>(d.data_ptr());
     args.ldd        = d.stride(-2);
     args.d_stride_l = op[3].batch_stride;
-    args.out = static_cast<float*>(out.t->data_ptr());
-    args.out_stride_n = out.t->stride(-2);
-    args.out_stride_o = out.t->stride(-3);
-    args.out_stride_l = out.batch_stride;
     const double p = PyFloat_AS_DOUBLE(v[5]);
     args.norm_type = p == 1.0 ? KM_NORM_L1 : p == 2.0 ? KM_NORM_L2 : KM_NORM_P;
     args.p.value   = static_cast<float>(p);
-    at::Tensor scratch;
-    const int64_t need = g_lib.grad_scratch(&args);
-    if (need > 0) {
-        scratch            = new_float({need / 4}, device);
-        args.scratch       = static_cast<float*>(scratch.data_ptr());
-        args.scratch_bytes = need;
+    at::Tensor made;
+    int rc;
+    {
+        Unlocked unlocked;
+        if (!given) {
+            made = new_float({L, O, N, M}, device);
+            args.out = static_cast<float*>(made.data_ptr());
+            args.out_stride_n = made.stride(-2);
+            args.out_stride_o = made.stride(-3);
+            args.out_stride_l = L != 1 ? made.stride(0) : 0;
+        }
+        at::Tensor scratch;
+        const int64_t need = g_lib.grad_scratch(&args);
+        if (need > 0) {
+            scratch            = new_float({need / 4}, device);
+            args.scratch       = static_cast<float*>(scratch.data_ptr());
+            args.scratch_bytes = need;
+        }
+        rc = g_lib.grad(&args, c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream());
     }
-    const int rc = g_lib.grad(&args, c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream());
-    return finish(rc, made, v[4] != Py_None ? v[4] : nullptr);
+    return finish(rc, made, given ? v[4] : nullptr);
 }
 
 // bind((addresses of the six entry points), (InnerOperator, PowerType, KernelType))

@@ -1,6 +1,11 @@
 """The extension that takes ordinary calls straight to the C-ABI: same results as the ctypes marshalling
 (which `debug=True` still uses), and anything out of the ordinary is declined, so that the Python layer's own
 checks and exceptions apply."""
+import ctypes
+import subprocess
+import threading
+import time
+
 import pytest
 import torch
 
@@ -69,3 +74,50 @@ def test_exceptions_of_the_python_layer_still_apply():
         kermac.cdist(a, b.cpu())
     with pytest.raises(ValueError, match="contraction"):
         kermac.cdist_grad(torch.zeros(3, 4, device="cuda"), b, b[:2], torch.zeros(5, 4, device="cuda"), contraction="no")
+
+
+SLOW_ENTRY_POINTS = """
+#include <unistd.h>
+#include <stdint.h>
+int kermac_b200_build_kernel_scratch(const void* a, void* s, int64_t n, void* st) { usleep(300000); return 0; }
+int64_t kermac_b200_build_scratch_bytes(const void* a) { return 0; }
+int kermac_b200_cdist_grad(const void* a, void* st) { usleep(300000); return 0; }
+int64_t kermac_b200_cdist_grad_scratch_bytes(const void* a) { return 0; }
+int kermac_b200_kernel_matvec(const void* a, void* st) { usleep(300000); return 0; }
+int64_t kermac_b200_kernel_matvec_scratch_bytes(const void* a) { return 0; }
+"""
+
+
+@pytest.mark.gpu
+def test_other_python_threads_run_while_a_call_is_in_its_native_part(tmp_path):
+    # entry points that only sleep stand in for a launch that waits on a full queue
+    (tmp_path / "slow.c").write_text(SLOW_ENTRY_POINTS)
+    subprocess.run(["gcc", "-shared", "-fPIC", str(tmp_path / "slow.c"), "-o", str(tmp_path / "slow.so")], check=True)
+    a, b, c = (torch.zeros(n, 4, device="cuda") for n in (5, 6, 3))
+    z, cm = torch.zeros(6, 5, device="cuda"), torch.zeros(2, 5, device="cuda")
+    call = _native.torch_call()
+    calls = (lambda: call.cdist(a, b, None, 2.0, False),
+             lambda: call.run_kernel(kermac.kernel_descriptor_l1_norm, a, b, *[None] * 7, 0, 0),
+             lambda: call.cdist_grad(a.t().contiguous(), b, c, z, None, 2.0, 0),
+             lambda: call.kernel_matvec(kermac.kernel_descriptor_l1_norm, a, b, cm, *[None] * 7, 0, 0, 0, None))
+    ticks, stop = [], threading.Event()
+
+    def tick():
+        while not stop.is_set():
+            ticks.append(time.perf_counter())
+            time.sleep(0.005)
+
+    other = threading.Thread(target=tick)
+    _native._bind_torch_call(call, ctypes.CDLL(str(tmp_path / "slow.so")))
+    try:
+        other.start()
+        for one in calls:
+            began = time.perf_counter()
+            assert one() is not None
+            ended = time.perf_counter()
+            assert ended - began >= 0.3
+            assert sum(began + 0.05 < t < ended - 0.05 for t in ticks) >= 5
+    finally:
+        stop.set()
+        other.join()
+        _native._bind_torch_call(call, _native.lib())
