@@ -185,9 +185,21 @@ def lib() -> C.CDLL:
 _call = None
 
 
+def _check_torch_version(call) -> None:
+    """ImportError unless the extension was compiled against the torch that is loaded: it reads torch's C++ objects
+    through inlined accessors, which another torch may lay out differently."""
+    import torch
+    built_for = getattr(call, "torch_version", "an unknown torch")
+    if built_for != torch.__version__:
+        raise ImportError(f"built for torch {built_for}, this is {torch.__version__}")
+
+
 def _bind_torch_call(call, handle) -> None:
     """Hands the C-ABI entry points of `handle` and the enum classes to the extension."""
-    from .build_a_kernel import InnerOperator, KernelType, PowerType
+    from .build_a_kernel import _INNER_CODE, _KERNEL_CODE, _POWER_CODE, InnerOperator, KernelType, PowerType
+    for kind, codes in ((InnerOperator, _INNER_CODE), (PowerType, _POWER_CODE), (KernelType, _KERNEL_CODE)):
+        if any(codes[member] != member.value - 1 for member in kind):
+            raise NativeLibraryError(f"{kind.__name__} does not number its members like the C-ABI")
     names = ("build_kernel_scratch", "build_scratch_bytes", "cdist_grad", "cdist_grad_scratch_bytes", "kernel_matvec",
              "kernel_matvec_scratch_bytes")
     addresses = tuple(C.cast(getattr(handle, "kermac_b200_" + name), C.c_void_p).value for name in names)
@@ -203,6 +215,7 @@ def torch_call():
             if _call is None:
                 try:
                     from . import _torch_call
+                    _check_torch_version(_torch_call)
                 except ImportError as exc:
                     import warnings
                     warnings.warn(f"kermac_b200._torch_call is not usable ({exc}): calls go through ctypes and cost "

@@ -1,4 +1,6 @@
-// The call path from torch tensors to the C-ABI, as a CPython extension (kermac_b200/_torch_call.so).
+// The call path from torch tensors to the C-ABI, as a CPython extension (kermac_b200/_torch_call*.so).
+// It reads torch's C++ objects, so it serves the one CPython its file name carries and the one torch version it was
+// compiled against; _native.torch_call() compares the latter.
 //
 // A call of cdist / run_kernel / cdist_grad / kernel_matvec on a small problem is bound by the host:
 // checking three tensors, filling an argument struct through ctypes and asking torch for an output took
@@ -238,7 +240,7 @@ PyObject* call_cdist(PyObject*, PyObject* const* v, Py_ssize_t n) {
 }
 
 // The four enum members of a KernelDescriptor as C-ABI codes.  InnerOperator, PowerType and KernelType
-// number their members from 1 in the order of the C enums; bind() checked that.
+// number their members from 1 in the order of the C enums; _native checks that before it calls bind().
 PyObject* g_enum_types[3] = {nullptr, nullptr, nullptr};
 PyObject* g_names[5]      = {nullptr, nullptr, nullptr, nullptr, nullptr};
 
@@ -509,4 +511,8 @@ PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_torch_call", "torch tensors to 
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__torch_call(void) { return PyModule_Create(&g_module); }
+PyMODINIT_FUNC PyInit__torch_call(void) {
+    PyObject* module = PyModule_Create(&g_module);
+    if (module && PyModule_AddStringConstant(module, "torch_version", KM_TORCH_VERSION) < 0) Py_CLEAR(module);
+    return module;
+}

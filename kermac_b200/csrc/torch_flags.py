@@ -1,7 +1,8 @@
 """What the Makefile needs to know about Python and torch to build _torch_call.
 
   torch_flags.py id        one line that changes when the Python or the torch it is built for does
-  torch_flags.py cflags    compiler flags (headers, ABI)
+  torch_flags.py suffix    file name ending that only this Python imports (needs no torch)
+  torch_flags.py cflags    compiler flags (headers, ABI, torch's version as a macro)
   torch_flags.py ldflags   library folders
 """
 import importlib.metadata
@@ -14,7 +15,11 @@ def torch_id():
     spec = importlib.util.find_spec("torch")          # located, not imported: this runs on every make
     if spec is None:
         sys.exit("torch is not installed for " + sys.executable)
-    return " ".join((sys.executable, sys.version.split()[0], importlib.metadata.version("torch"), str(spec.origin)))
+    return " ".join((sysconfig.get_paths()["include"], sys.version.split()[0], importlib.metadata.version("torch"), str(spec.origin)))
+
+
+def suffix():
+    return sysconfig.get_config_var("EXT_SUFFIX")
 
 
 def cflags():
@@ -22,7 +27,8 @@ def cflags():
     from torch.utils import cpp_extension
     folders = cpp_extension.include_paths() + [sysconfig.get_paths()["include"]]
     return " ".join(["-isystem " + folder for folder in folders] +
-                    [f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}"])
+                    [f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+                     f"-DKM_TORCH_VERSION='\"{torch.__version__}\"'"])
 
 
 def ldflags():
@@ -31,4 +37,4 @@ def ldflags():
 
 
 if __name__ == "__main__":
-    print({"id": torch_id, "cflags": cflags, "ldflags": ldflags}[sys.argv[1]]())
+    print({"id": torch_id, "suffix": suffix, "cflags": cflags, "ldflags": ldflags}[sys.argv[1]]())

@@ -8,7 +8,7 @@ import subprocess
 import pytest
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
-CALL = "../_torch_call.so"
+CALL = "../_torch_call.fake-abi.so"
 
 
 @pytest.fixture
@@ -27,7 +27,8 @@ def tree(tmp_path):
 
 def _python(tree, version, fails_on="nothing"):
     fake = tree / "python"
-    fake.write_text(f'#!/bin/sh\n[ "$2" = {fails_on} ] && exit 1\n[ "$2" = id ] && echo "torch {version}" || echo "-Dflag_{version}"\n')
+    fake.write_text(f'#!/bin/sh\n[ "$2" = {fails_on} ] && exit 1\ncase "$2" in\n  id) echo "torch {version}" ;;\n'
+                    f'  suffix) echo .fake-abi.so ;;\n  *) echo "-Dflag_{version}" ;;\nesac\n')
     fake.chmod(0o755)
     return str(fake)
 
@@ -48,7 +49,7 @@ def test_the_library_is_built_without_torch(tree, target):
     assert run.returncode == 0, run.stderr
     assert (tree / "kermac_b200" / "libkermac_b200.so").exists()
     assert not _compiled(tree, "cxx") and not list((tree / "kermac_b200" / "csrc" / "build").glob("torch*"))
-    run = _make(tree, "false", CALL)
+    run = _make(tree, "false", "../_torch_call")            # (no Python, no file name ending)
     assert run.returncode != 0 and "needs torch" in run.stderr
 
 

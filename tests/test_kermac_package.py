@@ -6,6 +6,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import zipfile
 
 import pytest
@@ -78,10 +79,13 @@ def test_wheel_carries_both_packages_and_the_library(tmp_path):
     assert res.returncode == 0, res.stdout[-2000:] + res.stderr[-2000:]
     built = [f for f in os.listdir(wheels) if f.endswith(".whl")]
     assert len(built) == 1 and "linux" in built[0]
+    python = f"cp{sys.version_info.major}{sys.version_info.minor}"        # the extension is this CPython's only
+    assert f"-{python}-{python}" in built[0]
     site = tmp_path / "site"
     with zipfile.ZipFile(wheels / built[0]) as z:
         names = [n.split("purelib/")[-1].split("platlib/")[-1] for n in z.namelist()]
     assert "kermac_b200/libkermac_b200.so" in names
+    assert [n for n in names if "_torch_call" in n] == ["kermac_b200/_torch_call" + sysconfig.get_config_var("EXT_SUFFIX")]
     assert "kermac/__init__.py" in names and "kermac/linalg/__init__.py" in names
     assert not any(n.startswith("kermac_b200/csrc") for n in names)
     res = subprocess.run([sys.executable, "-m", "pip", "install", "--no-deps", "--no-index", "--target", str(site),

@@ -24,6 +24,23 @@ def test_declines_what_is_not_an_ordinary_call():
     assert call.cdist_grad(a, b, b, a, None, 2.0, None) is None
 
 
+def test_an_extension_of_another_torch_is_not_used(monkeypatch):
+    assert _native.torch_call().torch_version == torch.__version__
+    monkeypatch.setattr(_native, "_call", None)
+    monkeypatch.setattr(torch, "__version__", "0.0.1")
+    with pytest.warns(RuntimeWarning, match="built for torch"):
+        assert _native.torch_call() is False
+
+
+def test_enum_classes_that_do_not_match_the_c_abi_are_refused(monkeypatch):
+    from kermac_b200 import build_a_kernel
+    swapped = dict(build_a_kernel._POWER_CODE)
+    swapped[kermac.PowerType.ABS], swapped[kermac.PowerType.SQUARE] = _native.POW_SQUARE, _native.POW_ABS
+    monkeypatch.setattr(build_a_kernel, "_POWER_CODE", swapped)
+    with pytest.raises(_native.NativeLibraryError, match="PowerType"):
+        _native._bind_torch_call(_native.torch_call(), _native.lib())
+
+
 def _col(t):
     return t.transpose(-1, -2).contiguous().transpose(-1, -2)
 
