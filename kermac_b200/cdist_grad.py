@@ -164,8 +164,11 @@ def cdist_grad(
     need = int(library.kermac_b200_cdist_grad_scratch_bytes(ctypes.byref(args)))
     scratch = None
     if need > 0:
-        scratch = torch.empty(need // 4, dtype=torch.float32, device=a.device)
-        args.scratch, args.scratch_bytes = scratch.data_ptr(), need
+        try:
+            scratch = torch.empty(need // 4, dtype=torch.float32, device=a.device)
+            args.scratch, args.scratch_bytes = scratch.data_ptr(), need
+        except torch.cuda.OutOfMemoryError:      # without room for the partial sums: a single pass over k
+            need = 0
     if debug:
         print(f'(Kermac Debug) Launching cdist_grad norm_type={args.norm_type} split scratch bytes={need}')
     _native.launch_grad(args, stream_ptr)

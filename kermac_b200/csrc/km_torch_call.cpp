@@ -454,12 +454,16 @@ PyObject* call_cdist_grad(PyObject*, PyObject* const* v, Py_ssize_t n) {
             args.out_stride_o = made.stride(-3);
             args.out_stride_l = L != 1 ? made.stride(0) : 0;
         }
+        // A device too full for the partial sums takes a single pass over k.
         at::Tensor scratch;
         const int64_t need = g_lib.grad_scratch(&args);
         if (need > 0) {
-            scratch            = new_float({need / 4}, device);
-            args.scratch       = static_cast<float*>(scratch.data_ptr());
-            args.scratch_bytes = need;
+            try {
+                scratch            = new_float({need / 4}, device);
+                args.scratch       = static_cast<float*>(scratch.data_ptr());
+                args.scratch_bytes = need;
+            } catch (const c10::OutOfMemoryError&) {
+            }
         }
         rc = g_lib.grad(&args, c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)).stream());
     }

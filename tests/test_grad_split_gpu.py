@@ -4,6 +4,7 @@ single pass over k (the same terms, regrouped) and against the float64 oracle.
 Bound of the regrouping: each of the K additions of the single pass rounds by at most 2^-24 of a partial sum, which
 stays about below the largest entry; independent, they add up to 2^-24 sqrt(K / 3) of it (one sigma).  Held to
 2 * 2^-24 sqrt(K), 3.5 sigma of that."""
+import contextlib
 import ctypes
 import math
 
@@ -15,6 +16,18 @@ from kermac_b200 import _native
 from oracle import kermac_oracle as ko
 
 pytestmark = pytest.mark.gpu
+
+
+@contextlib.contextmanager
+def full_device():
+    """torch's allocator refuses whatever it does not hold already."""
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.set_per_process_memory_fraction(torch.cuda.memory_reserved() / torch.cuda.get_device_properties(0).total_memory)
+    try:
+        yield
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
 
 
 def _single_pass(a, b, c, d, p):
@@ -47,3 +60,18 @@ def test_split_sums_match_a_single_pass(shape, p):
     assert float((got - want).abs().max()) <= 2.0 ** -23 * math.sqrt(K) * float(want.abs().max())
     assert ko.rel_err_signed(got, ko.cdist_grad_ref(a.cpu(), b.cpu(), c.cpu(), d.cpu(), p=p)[0]) < 5e-5
     assert _native.device_error_flag() == 0
+
+
+def test_a_full_device_takes_a_single_pass():
+    K, M, N, O = 3000, 4096, 320, 4                              # one partial result is 21 MB
+    gen = torch.Generator().manual_seed(1)
+    a, b = torch.rand(K, M, generator=gen).cuda(), torch.randn(N, K, generator=gen).cuda()
+    c, d = torch.randn(O, K, generator=gen).cuda(), torch.randn(N, M, generator=gen).cuda()
+    want, splits = _single_pass(a, b, c, d, 1.0)
+    assert splits > 1, "the case must be one that splits"
+    for debug in (False, True):                                  # the native call path and the ctypes one
+        out = torch.full((O, N, M), float("nan"), device="cuda")
+        with full_device():
+            kermac.cdist_grad(a, b, c, d, out=out, p=1.0, debug=debug)
+        assert torch.equal(out, want)
+        assert not torch.equal(kermac.cdist_grad(a, b, c, d, out=out, p=1.0, debug=debug), want)      # split again
