@@ -47,24 +47,31 @@ struct BuildPlan {
 //   an operand that both can only copy word by word: few tiles; for |.| and |.|^p also a short k loop
 //       square  1000^2 x 27: 33.7 / 11.2   4000^2 x 27: 66.0 / 64.8   4000^2 x 129: 206 / 245
 //       |.|     1000^2 x 27: 32.6 / 9.3    4001 x 4003 x 64: 140 / 118   8001 x 8003 x 300: 1727 / 1911
-//       |.|^1.3 1000^2 x 27: 44.8 / 21.7   4001 x 4003 x 64: 440 / 425   8001 x 8003 x 300: 7543 / 7636
 //   both operands contiguous along the points: a short k loop, or few tiles:
 //       square  2048^2 x 64: 28.9 / 22.8   2048^2 x 512: 156 / 140   4000^2 x 512: 521 / 509
 //               4000^2 x 1024: 1029 / 1045   16384^2 x 128: 2148 / 2127   16384^2 x 256: 4111 / 4159
 //       |.|     2048^2 x 64: 33.0 / 24.8   2048^2 x 512: 171 / 158   4000^2 x 512: 581 / 569
 //               4000^2 x 1024: 1124 / 1142   16384^2 x 64: 1383 / 1279   16384^2 x 128: 2375 / 2400
-//       |.|^1.3 2048^2 x 64: 125 / 107   2048^2 x 512: 923 / 814   4000^2 x 1024: 6278 / 6081
-//               16384^2 x 128: 12559 / 12527   16384^2 x 256: 24802 / 24864
-// The line is drawn by the whole problem, not by the launch's tile range: the two kernels spread the two
-// forms of the fractional power differently over a tile, and ranges must add up to the full launch's bits.
+//   |.|^1.3, operands not held as aligned rows: a short k loop, or up to 2048 tiles:
+//       contiguous points 2048^2 x 512: 923 / 814   4000^2 x 1024: 6276 / 6079   4736 x 4096 x 600: 4217 / 4229
+//               4400^2 x 600: 4732 / 4359   5760^2 x 600: 7340 / 7240   16384^2 x 128: 12559 / 12527   x 256: 24802 / 24864
+//       word by word 1000^2 x 27: 44.8 / 21.7   4001 x 4000 x 600: 3909 / 3835   5501 x 5500 x 600: 7209 / 7069
+//               8001 x 8003 x 300: 7543 / 7636
+//       with itself 4400^2 x 600: 2765 / 2264   5700^2 x 600: 3858 / 3704
+// The line is drawn by the whole problem, not by the launch's tile range, so that ranges add up to the full
+// launch's bits.  For |.|^p, whose two forms of the exponential the two kernels spread differently over a tile, it
+// must not depend either on whether operands have been packed (the caller's scratch) or on symmetry (which a range
+// switches off): it counts every tile, and is the same for contiguous points as for operands copied word by word
+// (packed rows are rows that the 64 x 64 kernel reads as well, so they are never packed).
 bool small_preferred(const BuildParams& p, bool avec, bool bvec, bool awide, bool bwide) {
+    const bool rows = awide && bwide && !(avec && bvec);
+    if (p.inner_id == IN_DIFF_POW) return rows || p.K <= 128 || (long long)p.tiles_m * p.tiles_n * p.L <= 2048;
     const long long tiles =
         (p.symmetric ? (long long)p.tiles_n * (p.tiles_n + 1) / 2 : (long long)p.tiles_m * p.tiles_n) * p.L;
-    if (!awide || !bwide)
-        return tiles <= 512 || ((p.inner_id == IN_DIFF_ABS || p.inner_id == IN_DIFF_POW) && p.K <= 128);
-    if (!avec || !bvec) return true;
+    if (!awide || !bwide) return tiles <= 512 || (p.inner_id == IN_DIFF_ABS && p.K <= 128);
+    if (rows) return true;
     if (p.K <= (p.inner_id == IN_DIFF_ABS ? 96 : 128)) return true;
-    return tiles <= 512 || (tiles <= 1024 && (p.K <= 512 || p.inner_id == IN_DIFF_POW));
+    return tiles <= 512 || (tiles <= 1024 && p.K <= 512);
 }
 
 int make_plan(const KmBuildArgs* a, BuildPlan* plan) {

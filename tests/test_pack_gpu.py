@@ -55,6 +55,17 @@ def test_packed_operands_give_the_same_bits(layouts, shape):
     assert _native.device_error_flag() == 0
 
 
+@pytest.mark.parametrize("shape", [(3000, 3000, 301), (4001, 4003, 200), (6001, 5003, 130)])
+def test_fractional_powers_do_not_depend_on_the_scratch(shape):
+    M, N, K = shape                                             # below and above the line between the kernels
+    gen = torch.Generator().manual_seed(K)
+    a, b = _points(gen, (), M, K, "off"), _points(gen, (), N, K, "off")
+    out, other = torch.empty(M, N, device="cuda"), torch.empty(M, N, device="cuda")
+    assert _call(a, b, out, 1.3) > 0, "the case must be one that packs"
+    _call(a, b, other, 1.3, scratch_bytes=0)
+    assert torch.equal(out, other)
+
+
 def test_one_matrix_is_packed_once_and_stays_symmetric():
     x = torch.randn(8001, 96, generator=torch.Generator().manual_seed(1)).cuda()
     out = torch.empty(8001, 8001, device="cuda")

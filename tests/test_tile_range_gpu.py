@@ -57,6 +57,38 @@ def test_tile_ranges_reproduce_the_full_launch(p, layout):
     assert _native.device_error_flag() == 0
 
 
+def test_ranges_of_fractional_powers_match_a_full_call_that_packs():
+    # rows that can only be copied word by word: cdist packs them first, ranges read them where they lie
+    M, N, K = 3000, 3000, 301
+    g = torch.Generator().manual_seed(22)
+    a, b = torch.randn(M, K, generator=g).cuda(), torch.randn(N, K, generator=g).cuda()
+    whole = kermac.cdist(a, b, p=1.3)[0]
+    parts = torch.full_like(whole, -3.0)
+    total = _launch(a, b, torch.empty_like(whole), 1.3)
+    for first, count in tile_ranges(total, 8):
+        _launch(a, b, parts, 1.3, first, count)
+    assert torch.equal(parts, whole)
+
+
+@pytest.mark.parametrize("p", [1.0, 2.0, 1.3])
+def test_ranges_of_a_matrix_with_itself(p):
+    # the full launch computes the tiles on and above the diagonal and mirrors them, ranges compute every tile: a
+    # mirrored fractional power takes the exponential's other route here and there and agrees to rounding
+    M, K = 4400, 136
+    x = torch.randn(K, M, generator=torch.Generator().manual_seed(23)).cuda().t()
+    whole, parts = (torch.full((M, M), -3.0, device="cuda").t() for _ in range(2))
+    total = _launch(x, x, whole, p)
+    for first, count in tile_ranges(total, 8):
+        _launch(x, x, parts, p, first, count)
+    if p == 1.3:
+        assert torch.allclose(parts, whole, rtol=2e-6, atol=0.0)
+        tile = torch.arange(M, device="cuda") // 64             # the kernel chosen here works in 64 x 64 tiles
+        computed = tile[:, None] <= tile[None, :]
+        assert torch.equal(parts[computed], whole[computed])
+    else:
+        assert torch.equal(parts, whole)
+
+
 def test_empty_range_is_a_no_op():
     a = torch.rand(64, 300, device="cuda").t()
     out = torch.full((300, 300), -3.0, device="cuda").t()
