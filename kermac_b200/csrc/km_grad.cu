@@ -14,6 +14,7 @@
 //   - blocks that share a tile of the weight matrix a (the n-tiles of one m-column and
 //     k range) are neighbours in launch order, so a is read from DRAM once;
 //   - p = 1.5 takes |x|^(p-1) as one sqrt.approx instead of the lg2 / ex2 pair.
+#include <algorithm>
 #include <mutex>
 
 #include "km_common.cuh"
@@ -431,20 +432,16 @@ int preferred_split(const GradPlan& plan, int norm_type, bool square_root) {
         slab_us = 0.6 + 0.16 * plan.nt * (1 + plan.ot);
         if (norm_type == KM_NORM_P) slab_us += (square_root ? 0.5 : 1.4) * plan.nt;
     }
-    auto cost = [&](long long s) {
-        const long long per_split = ceil_div_ll(slabs, s);
-        const long long share     = ceil_div_ll(blocks * ceil_div_ll(slabs, per_split), sms);
-        const double units        = plan.tensor ? (double)share : 0.9 * share + ((share & 1) ? 0.1 : 0.0);
+    auto cost = [&](long long s, long long per_split) {
+        const long long share = ceil_div_ll(blocks * s, sms);
+        const double units    = plan.tensor ? (double)share : 0.9 * share + ((share & 1) ? 0.1 : 0.0);
         return units * per_split * slab_us + 2.5 * share + (s > 1 ? 3.0 + (2.0 * s + 1.0) * bytes / 5e6 : 0.0);
     };
     // more than 16 blocks per SM gain nothing, and partial results stay within 512 MB
-    long long last = 1;
-    while (last < slabs && blocks * (last + 1) <= 16 * sms && bytes * (last + 1) <= 512e6) ++last;
-    double least = cost(1);
-    for (long long s = 2; s <= last; ++s) least = cost(s) < least ? cost(s) : least;
-    for (long long s = 1; s <= last; ++s)
-        if (cost(s) <= 1.005 * least) return (int)s;
-    return 1;
+    const double cap = 512e6 / (bytes > 0.0 ? bytes : 1.0);
+    long long last   = std::min(slabs, 16 * sms / blocks);
+    if ((double)last > cap) last = (long long)cap;
+    return cheapest_split(slabs, last, cost);
 }
 
 int make_grad_plan(const KmGradArgs* a, GradPlan* plan) {

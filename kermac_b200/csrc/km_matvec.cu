@@ -13,6 +13,7 @@
 //
 // The reference has no such kernel: callers materialise run_kernel(...)
 // (src/kermac/build_a_kernel.py:158-394) and multiply afterwards.
+#include <algorithm>
 #include <cstring>
 
 #include "km_build_cpasync.cuh"
@@ -666,20 +667,14 @@ int preferred_split(const MatvecParams& p) {
     const long long sms    = sm_count();
     const long long result = (long long)p.L * p.N * p.O * 4;
     if (blocks <= 0 || chunks <= 1) return 1;
-    auto cost = [&](long long s) {
-        const long long per_split = ceil_div_ll(chunks, s);
-        const long long share     = ceil_div_ll(blocks * ceil_div_ll(chunks, per_split), sms);
+    auto cost = [&](long long s, long long per_split) {
+        const long long share = ceil_div_ll(blocks * s, sms);
         return (0.9 * share + ((share & 1) ? 0.12 : 0.0)) * per_split * (4.5 + 0.155 * p.K) + 1.5 * share +
                (s > 1 ? 3.0 + 0.05 * s : 0.0);
     };
     // more than 32 blocks per SM gain nothing, and partial results stay within 512 MB
-    long long last = 1;
-    while (last < chunks && blocks * (last + 1) <= 32 * sms && result * (last + 1) <= (512LL << 20)) ++last;
-    double least = cost(1);
-    for (long long s = 2; s <= last; ++s) least = cost(s) < least ? cost(s) : least;
-    for (long long s = 1; s <= last; ++s)
-        if (cost(s) <= 1.005 * least) return (int)s;
-    return 1;
+    const long long last = std::min({chunks, 32 * sms / blocks, (512LL << 20) / std::max(result, 1LL)});
+    return cheapest_split(chunks, last, cost);
 }
 
 // How the operands are staged: 16-byte copies, and TMA where the inner step gains from it.
