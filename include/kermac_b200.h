@@ -253,7 +253,8 @@ int kermac_b200_kernel_matvec(const KmMatvecArgs* args, void* stream);
 int64_t kermac_b200_kernel_matvec_scratch_bytes(const KmMatvecArgs* args);
 
 /* Writes a description of the kernel variant and grid that kermac_b200_build_kernel
- * would launch for `args` into buf (NUL terminated, truncated to buf_len). */
+ * would launch for `args` into buf (NUL terminated, truncated to buf_len), and, where it differs, what
+ * kermac_b200_build_kernel_scratch launches with the scratch it asks for. */
 int kermac_b200_describe_variant(const KmBuildArgs* args, char* buf, int32_t buf_len);
 
 /*

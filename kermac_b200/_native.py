@@ -258,8 +258,15 @@ def hyper(value) -> KmHyper:
     return h
 
 
-def launch_build(args: KmBuildArgs, stream_ptr: int) -> None:
-    check(lib().kermac_b200_build_kernel(C.byref(args), C.c_void_p(stream_ptr)), "kermac_b200_build_kernel")
+def launch_build(args: KmBuildArgs, stream_ptr: int, scratch=None) -> None:
+    """`scratch`: a tensor of build_scratch_bytes() that belongs to the stream, or None to do without."""
+    ptr, size = (None, 0) if scratch is None else (scratch.data_ptr(), scratch.numel() * scratch.element_size())
+    check(lib().kermac_b200_build_kernel_scratch(C.byref(args), ptr, size, C.c_void_p(stream_ptr)),
+          "kermac_b200_build_kernel")
+
+
+def build_scratch_bytes(args: KmBuildArgs) -> int:
+    return int(lib().kermac_b200_build_scratch_bytes(C.byref(args)))
 
 
 def build_tile_count(args: KmBuildArgs) -> int:

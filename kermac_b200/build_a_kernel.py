@@ -339,6 +339,18 @@ def run_kernel(
     stream_ptr = _current_stream_for(a.device)
     if debug:
         print(f'(Kermac Debug) Launching kernel: {_native.describe_build(args)}')
-    _native.launch_build(args, stream_ptr)
+    scratch, need = None, _native.build_scratch_bytes(args)
+    if need > 0:
+        try:
+            scratch = torch.empty(need // 4, dtype=torch.float32, device=a.device)
+        except torch.cuda.OutOfMemoryError:      # it only makes the call faster
+            pass
+    if debug:
+        print(f'(Kermac Debug) scratch bytes={need if scratch is not None else 0}')
+    if scratch is None:
+        _native.launch_build(args, stream_ptr)
+    else:
+        _native.launch_build(args, stream_ptr, scratch)
+    del scratch
     del keep_alive
     return out

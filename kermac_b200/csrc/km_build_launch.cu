@@ -228,6 +228,21 @@ void plan_pack_operands(const BuildPlan& plan, PackPlan* pack) {
     if (pairs * p.K * gain < 1.5 * pack_seconds(pack->floats[0] + pack->floats[1])) pack->n = 0;
 }
 
+// The same call on the operands packed into `scratch` (plan.swapped: the kernel's A is the caller's b).
+KmBuildArgs packed_arguments(const KmBuildArgs& args, const BuildPlan& plan, PackPlan* pack, void* scratch) {
+    pack->job[0].dst = static_cast<float*>(scratch);
+    pack->job[1].dst = pack->job[0].dst + pack->floats[0];
+    KmBuildArgs packed = args;
+    auto use_a = [&](const PackJob& j) { packed.a = j.dst; packed.a_stride_m = 1; packed.a_stride_k = j.pitch; packed.a_stride_l = j.dst_l; };
+    auto use_b = [&](const PackJob& j) { packed.b = j.dst; packed.b_stride_n = 1; packed.b_stride_k = j.pitch; packed.b_stride_l = j.dst_l; };
+    if (pack->a) { if (plan.swapped) use_b(pack->job[0]); else use_a(pack->job[0]); }
+    if (pack->b) {
+        const PackJob& j = pack->job[pack->a && !pack->shared ? 1 : 0];
+        if (plan.swapped) use_a(j); else use_b(j);
+    }
+    return packed;
+}
+
 const char* const kInnerNames[IN_COUNT] = {"diff_abs", "diff_square", "diff_pow", "diff_noop", "diff_sqrt",
                                            "dot_noop", "dot_abs",     "dot_square", "dot_sqrt", "dot_pow"};
 
@@ -298,20 +313,8 @@ extern "C" int kermac_b200_build_kernel_scratch(const KmBuildArgs* args, void* s
     const int64_t need = (int64_t)(pack.floats[0] + pack.floats[1]) * 4;
     if (!pack.n || !scratch || !aligned16(scratch) || scratch_bytes < need) return launch_plan(plan, st);
 
-    pack.job[0].dst = static_cast<float*>(scratch);
-    pack.job[1].dst = pack.job[0].dst + pack.floats[0];
+    KmBuildArgs packed = packed_arguments(*args, plan, &pack, scratch);
     if (int rc = launch_pack(pack.job, pack.n, plan.p.K, st)) return rc;
-    // the same call on the packed operands (plan.swapped: the kernel's A is the caller's b)
-    KmBuildArgs packed = *args;
-    const PackJob* next = pack.job;
-    auto use_a = [&](const PackJob& j) { packed.a = j.dst; packed.a_stride_m = 1; packed.a_stride_k = j.pitch; packed.a_stride_l = j.dst_l; };
-    auto use_b = [&](const PackJob& j) { packed.b = j.dst; packed.b_stride_n = 1; packed.b_stride_k = j.pitch; packed.b_stride_l = j.dst_l; };
-    if (pack.a) { if (plan.swapped) use_b(*next); else use_a(*next); }
-    if (pack.b) {
-        if (!pack.shared) ++next;
-        if (!pack.a) next = pack.job;
-        if (plan.swapped) use_a(*next); else use_b(*next);
-    }
     if (int rc = make_plan(&packed, &plan)) return rc;
     return launch_plan(plan, st);
 }
@@ -332,11 +335,21 @@ extern "C" int kermac_b200_describe_variant(const KmBuildArgs* args, char* buf, 
     BuildPlan plan;
     if (int rc = make_plan(args, &plan)) return rc;
     const BuildParams& p = plan.p;
-    snprintf(buf, (size_t)buf_len,
+    auto name  = [](const BuildPlan& q) { return q.variant == KM_VARIANT_TMA ? "tma" : "cpasync"; };
+    int length = snprintf(buf, (size_t)buf_len,
              "build_kernel variant=%s inner=%s outer_power=%d kernel_type=%d exchanged=%d a_vec16=%d b_vec16=%d "
              "out_vec16=%d tiles=%dx%d batches=%d symmetric=%d tile_range=%d+%d kernel_tile=%d",
-             plan.variant == KM_VARIANT_TMA ? "tma" : "cpasync", kInnerNames[p.inner_id], p.outer_power, p.kernel_type,
+             name(plan), kInnerNames[p.inner_id], p.outer_power, p.kernel_type,
              plan.swapped ? 1 : 0, plan.avec ? 1 : 0, plan.bvec ? 1 : 0, p.c_vec4, p.tiles_m, p.tiles_n, p.L, p.symmetric,
              p.tile_first, p.tile_count, plan.small ? 64 : BUILD_TILE);
+    // what kermac_b200_build_kernel_scratch does with as much scratch as it asks for (any aligned address stands for it)
+    PackPlan pack;
+    plan_pack_operands(plan, &pack);
+    if (!pack.n || length < 0 || length >= buf_len) return 0;
+    const long long bytes = (pack.floats[0] + pack.floats[1]) * 4;
+    KmBuildArgs packed    = packed_arguments(*args, plan, &pack, reinterpret_cast<void*>(uintptr_t{256}));
+    if (int rc = make_plan(&packed, &plan)) return rc;
+    snprintf(buf + length, (size_t)(buf_len - length), "; with %lld bytes of scratch: operands packed, variant=%s kernel_tile=%d",
+             bytes, name(plan), plan.small ? 64 : BUILD_TILE);
     return 0;
 }

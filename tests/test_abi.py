@@ -208,6 +208,20 @@ def test_describe_variant_reports_the_plan():
     assert "variant=cpasync" in _native.describe_build(col) and "a_vec16=1" in _native.describe_build(col)
 
 
+def test_describe_variant_reports_what_scratch_changes():
+    lib = _native.lib()
+    rows = _build_args(m=8000, n=8000, k=512, a_stride_m=512, b_stride_n=512, out_stride_n=8000, b=0x2000,
+                       inner_power=_native.POW_SQUARE)
+    text = _native.describe_build(rows)
+    need = lib.kermac_b200_build_scratch_bytes(ctypes.byref(rows))
+    assert need == 2 * 8000 * 512 * 4
+    plain, packed = text.split("; ")
+    assert plain.startswith("build_kernel variant=cpasync") and plain.endswith("kernel_tile=64")
+    assert packed == f"with {need} bytes of scratch: operands packed, variant=tma kernel_tile=128"
+    rows.m = rows.n = 300                          # too small to pack
+    assert ";" not in _native.describe_build(rows) and lib.kermac_b200_build_scratch_bytes(ctypes.byref(rows)) == 0
+
+
 def test_grad_rejects_bad_arguments():
     lib = _native.lib()
     g = _native.KmGradArgs()

@@ -20,11 +20,17 @@ pytestmark = pytest.mark.gpu
 
 @contextlib.contextmanager
 def full_device():
-    """torch's allocator refuses whatever it does not hold already."""
+    """torch's allocator has no more than 1 MB to give."""
     torch.cuda.synchronize()
     torch.cuda.empty_cache()
     torch.cuda.set_per_process_memory_fraction(torch.cuda.memory_reserved() / torch.cuda.get_device_properties(0).total_memory)
+    held, size = [], 1 << 30                                     # what is free inside the segments in use
     try:
+        while size >= 1 << 20:
+            try:
+                held.append(torch.empty(size, dtype=torch.uint8, device="cuda"))
+            except torch.cuda.OutOfMemoryError:
+                size //= 2
         yield
     finally:
         torch.cuda.set_per_process_memory_fraction(1.0)

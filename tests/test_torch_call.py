@@ -11,6 +11,7 @@ import torch
 
 import kermac_b200 as kermac
 from kermac_b200 import _native
+from test_grad_split_gpu import full_device
 
 
 def test_declines_what_is_not_an_ordinary_call():
@@ -76,6 +77,27 @@ def test_same_bits_as_the_ctypes_marshalling(L, layout, capsys):
         assert "Kermac Debug" in capsys.readouterr().out
         assert fast.shape == slow.shape and torch.equal(fast, slow)
     assert kermac.cdist(a, b, out=out) is out
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("p", [1.0, 2.0, 1.3])
+def test_both_paths_pack_large_row_operands(p, capsys, monkeypatch):
+    a, b = torch.randn(6001, 701, device="cuda"), torch.randn(6001, 701, device="cuda")
+    with_scratch = []
+    launch = _native.launch_build
+    monkeypatch.setattr(_native, "launch_build", lambda args, stream, scratch=None:
+                        (with_scratch.append(scratch is not None), launch(args, stream, scratch)))
+    fast, slow = kermac.cdist(a, b, p=p), kermac.cdist(a, b, p=p, debug=True)
+    assert with_scratch == [True] and torch.equal(fast, slow)
+    printed = capsys.readouterr().out
+    size = 2 * 6016 * 701 * 4
+    assert f"with {size} bytes of scratch: operands packed" in printed and f"scratch bytes={size}" in printed
+    for debug in (False, True):                              # a full device does without, for the same bits
+        slow.fill_(-1.0)
+        with full_device():
+            kermac.cdist(a, b, out=slow, p=p, debug=debug)
+        assert torch.equal(fast, slow)
+    assert with_scratch == [True, False] and "scratch bytes=0" in capsys.readouterr().out
 
 
 @pytest.mark.gpu
