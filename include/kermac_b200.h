@@ -134,7 +134,7 @@ typedef struct KmBuildArgs {
 int kermac_b200_build_kernel(const KmBuildArgs* args, void* stream);
 
 /* The same call with device scratch, which pays where a or b is held as rows (k contiguous): large problems
- * rewrite such operands k-major first.  kermac_b200_build_scratch_bytes says how much the call would use (0:
+ * rewrite such operands k-major first, which takes (m + n) * k * l floats, 1 GiB at most.  kermac_b200_build_scratch_bytes says how much the call would use (0:
  * none, or the arguments are rejected); without it (NULL, too small, not 16-byte aligned) the call is
  * kermac_b200_build_kernel.  The scratch may be reused once the stream has passed the call.  No reference
  * counterpart. */

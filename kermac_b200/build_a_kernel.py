@@ -319,6 +319,10 @@ def run_kernel(
     is None a (L, M, N) tensor is allocated.  Launches on torch's current stream and
     returns without synchronising.
 
+    A large problem whose points are held as rows copies them into scratch from torch's allocator first: the size of
+    a and b, at most 1 GiB, given back when the call returns and done without where the device is full.  Like every
+    allocation by torch it has to be captured through torch.cuda.graph.
+
     The TMA-staged kernels wait on their copies with a bound; if such a wait ever runs out the
     affected tiles are not written and a device flag is raised.  Nothing here reads it: poll
     `kermac_b200._native.device_error_flag()` at your own synchronisation points (0 = clean).

@@ -28,7 +28,7 @@ def cdist(
     """out[m, n] = (sum_k |b[n, k] - a[m, k]|^p)^(1/p), or the raw sum with `skip_epilogue`.
 
     In storage terms (the reference README's c-style loop): a[K, M], b[K, N], out[N, M]
-    when every tensor is contiguous along m / n.
+    when every tensor is contiguous along m / n.  Large problems on row-held points use scratch as `run_kernel` does.
 
     Args:
         a: (M, K) or (L, M, K) float32 CUDA tensor, either majorness.

@@ -225,7 +225,8 @@ void plan_pack_operands(const BuildPlan& plan, PackPlan* pack) {
         pack->floats[pack->n] = plan_pack(&pack->job[pack->n], p.B, p.N, p.K, p.L, p.b_sn, p.b_sk, p.b_sl);
         ++pack->n;
     }
-    if (pairs * p.K * gain < 1.5 * pack_seconds(pack->floats[0] + pack->floats[1])) pack->n = 0;
+    const long long floats = pack->floats[0] + pack->floats[1];
+    if (pairs * p.K * gain < 1.5 * pack_seconds(floats) || floats * 4 > PACK_MAX_BYTES) pack->n = 0;
 }
 
 // The same call on the operands packed into `scratch` (plan.swapped: the kernel's A is the caller's b).

@@ -760,7 +760,8 @@ int make_matvec_plan(const KmMatvecArgs* a, MatvecPlan* plan) {
             plan->pack_floats[i] = plan_pack(&plan->pack[i], p.B, p.N, p.K, p.L, p.b_sn, p.b_sk, p.b_sl);
         }
         const double gain = (p.inner_id == IN_DIFF_ABS ? 1.6e-14 : 2e-14) * p.o_chunks * p.L;
-        if ((double)p.M * p.N * p.K * gain < pack_seconds(plan->pack_floats[0] + plan->pack_floats[1])) plan->packs = 0;
+        const long long floats = plan->pack_floats[0] + plan->pack_floats[1];
+        if ((double)p.M * p.N * p.K * gain < pack_seconds(floats) || floats * 4 > PACK_MAX_BYTES) plan->packs = 0;
     }
     return 0;
 }

@@ -20,6 +20,10 @@ long long plan_pack(PackJob* job, const float* src, int count, int K, int L, lon
 // Packs one or two operands in one launch; K >= 1.
 int launch_pack(const PackJob* jobs, int n, int K, cudaStream_t stream);
 
+// Packing takes at most this much scratch (0.6 % of the device), so that a call on a few points against very many
+// does not take a copy of its data set from a caller who counts on the memory; larger operands are read as they lie.
+constexpr long long PACK_MAX_BYTES = 1LL << 30;
+
 // Seconds a pack of `floats` elements adds to a call.
 double pack_seconds(long long floats);
 

@@ -141,6 +141,9 @@ def kernel_matvec(
     products per term, fp32-level accuracy), "fp32" (packed FP32 FMAs) or "auto" / None
     (the environment variable KERMAC_B200_CONTRACTION, else the library default: tensor).
 
+    Partial sums (at most 512 MB unless `split_m` asks for more) and copies of points that are held as rows (at most
+    1 GiB) take scratch from torch's allocator for the duration of the call.
+
     The tensor-core kernel waits on its copies and on the tensor cores with a bound; a wait that
     runs out leaves the affected rows unwritten and raises a device flag that nothing here reads:
     poll `kermac_b200._native.device_error_flag()` at your own synchronisation points.

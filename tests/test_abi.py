@@ -222,6 +222,22 @@ def test_describe_variant_reports_what_scratch_changes():
     assert ";" not in _native.describe_build(rows) and lib.kermac_b200_build_scratch_bytes(ctypes.byref(rows)) == 0
 
 
+@pytest.mark.parametrize("m, packs", [(4000000, True), (5000000, False)])       # 1.02 and 1.28 GB of rows, k = 64
+def test_packing_stops_at_a_gibibyte(m, packs):
+    lib = _native.lib()
+    rows = _build_args(m=m, n=1000, k=64, a_stride_m=64, b_stride_n=64, out_stride_n=m, b=0x2000,
+                       inner_power=_native.POW_SQUARE)
+    need = lib.kermac_b200_build_scratch_bytes(ctypes.byref(rows))
+    assert need == ((m + 1024) * 64 * 4 if packs else 0)
+    g = _native.KmMatvecArgs()
+    g.m, g.n, g.k, g.o, g.l = m, 1000, 64, 4, 1
+    g.a, g.b, g.c, g.y = 0x1000, 0x2000, 0x3000, 0x4000
+    g.a_stride_m, g.a_stride_k, g.b_stride_n, g.b_stride_k = 64, 1, 64, 1
+    g.ldc, g.y_stride_n, g.y_stride_o, g.inner_power = m, 4, 1, _native.POW_SQUARE
+    need = lib.kermac_b200_kernel_matvec_scratch_bytes(ctypes.byref(g))
+    assert (need > m * 64 * 4) == packs and need < 1536 << 20
+
+
 def test_grad_rejects_bad_arguments():
     lib = _native.lib()
     g = _native.KmGradArgs()
