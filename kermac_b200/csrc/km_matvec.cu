@@ -649,6 +649,7 @@ struct MatvecPlan {
     PackJob pack[2];          // operands worth rewriting k-major first
     int packs;
     bool pack_a, pack_b;
+    bool pack_shared;         // b is the same matrix as a: one copy serves both
     long long pack_floats[2];
 };
 
@@ -750,12 +751,13 @@ int make_matvec_plan(const KmMatvecArgs* a, MatvecPlan* plan) {
     plan->pack_a = !plan->avec;
     plan->pack_b = !plan->bvec;
     plan->pack_floats[0] = plan->pack_floats[1] = 0;
+    plan->pack_shared = p.A == p.B && p.M == p.N && p.a_sm == p.b_sn && p.a_sk == p.b_sk && p.a_sl == p.b_sl;
     if (p.K >= 1 && p.M > 0 && p.N > 0 && (plan->pack_a || plan->pack_b) && p.inner_id != IN_DIFF_POW) {
         if (plan->pack_a) {
             plan->pack_floats[0] = plan_pack(&plan->pack[0], p.A, p.M, p.K, p.L, p.a_sm, p.a_sk, p.a_sl);
             ++plan->packs;
         }
-        if (plan->pack_b) {
+        if (plan->pack_b && !plan->pack_shared) {
             const int i = plan->packs++;
             plan->pack_floats[i] = plan_pack(&plan->pack[i], p.B, p.N, p.K, p.L, p.b_sn, p.b_sk, p.b_sl);
         }

@@ -238,6 +238,19 @@ def test_packing_stops_at_a_gibibyte(m, packs):
     assert (need > m * 64 * 4) == packs and need < 1536 << 20
 
 
+def test_matvec_packs_one_matrix_once():
+    lib = _native.lib()
+    g = _native.KmMatvecArgs()
+    g.m = g.n = 20000
+    g.k, g.o, g.l, g.split_m = 65, 4, 1, 1
+    g.a, g.b, g.c, g.y = 0x1000, 0x2000, 0x3000, 0x4000
+    g.a_stride_m, g.a_stride_k, g.b_stride_n, g.b_stride_k = 65, 1, 65, 1
+    g.ldc, g.y_stride_n, g.y_stride_o, g.inner_power = 20000, 4, 1, _native.POW_SQUARE
+    assert lib.kermac_b200_kernel_matvec_scratch_bytes(ctypes.byref(g)) == 2 * 20000 * 65 * 4
+    g.b = g.a
+    assert lib.kermac_b200_kernel_matvec_scratch_bytes(ctypes.byref(g)) == 20000 * 65 * 4
+
+
 def test_grad_rejects_bad_arguments():
     lib = _native.lib()
     g = _native.KmGradArgs()

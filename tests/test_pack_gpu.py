@@ -94,6 +94,9 @@ def test_matvec_on_packed_operands(shape, layouts, desc):
             return buf[..., :x.shape[-2]].transpose(-1, -2)
         got = kermac.kernel_matvec(descriptor, a, b, c, bandwidth=8.0)
         assert torch.equal(got, kermac.kernel_matvec(descriptor, aligned(a), aligned(b), c, bandwidth=8.0))
+        x = aligned(a)                                         # one matrix on both sides: one copy serves both
+        assert torch.equal(kermac.kernel_matvec(descriptor, a, a, c, bandwidth=8.0),
+                           kermac.kernel_matvec(descriptor, x, x, c, bandwidth=8.0))
         split = kermac.kernel_matvec(descriptor, a, b, c, bandwidth=8.0, split_m=3)
         assert torch.allclose(got, split, rtol=0.0, atol=float(got.abs().max()) * 2e-6)    # sums of M terms, regrouped
     assert _native.device_error_flag() == 0
