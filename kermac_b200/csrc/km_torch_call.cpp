@@ -313,6 +313,14 @@ PyObject* call_run_kernel(PyObject*, PyObject* const* v, Py_ssize_t n) {
     return build(args, chain, v[1], v[2], v[3], L, device);
 }
 
+bool read_contraction(PyObject* o, int32_t& code) {
+    if (!PyUnicode_CheckExact(o)) return false;
+    const char* const names[] = {"auto", "fp32", "tensor"};       // KM_CONTRACT_*
+    for (code = KM_CONTRACT_AUTO; code <= KM_CONTRACT_TENSOR; ++code)
+        if (PyUnicode_CompareWithASCIIString(o, names[code]) == 0) return true;
+    return false;
+}
+
 // kernel_matvec(descriptor, a, b, c, out, p, inner_p, outer_p, bandwidth, epsilon, regularization, offset_x,
 //               offset_y, split_m, contraction)
 PyObject* call_kernel_matvec(PyObject*, PyObject* const* v, Py_ssize_t n) {
@@ -328,7 +336,11 @@ PyObject* call_kernel_matvec(PyObject*, PyObject* const* v, Py_ssize_t n) {
         return decline();
     if (!read_int32(v[11], args.reg_off_x) || !read_int32(v[12], args.reg_off_y) || !read_int32(v[13], args.split_m))
         return decline();
-    if (v[14] != Py_None || env_set("KERMAC_B200_CONTRACTION")) return decline();   // the library's own choice only
+    if (v[14] == Py_None) {
+        if (env_set("KERMAC_B200_CONTRACTION")) return decline();
+    } else if (!read_contraction(v[14], args.contraction)) {
+        return decline();
+    }
     Operand a, b, c, y;
     if (!read_operand(v[1], 2, device, a) || !read_operand(v[2], 2, device, b) || !read_operand(v[3], 2, device, c))
         return decline();

@@ -80,6 +80,25 @@ def test_same_bits_as_the_ctypes_marshalling(L, layout, capsys):
 
 
 @pytest.mark.gpu
+def test_a_named_contraction_takes_the_native_path(capsys):
+    g = torch.Generator().manual_seed(6)
+    a, b, c = (torch.randn(*s, generator=g).cuda() for s in ((500, 9), (70, 9), (3, 500)))
+    call, tail = _native.torch_call(), (None,) * 3 + (8.0, None, None, 0, 0, 0)
+    desc = kermac.kernel_descriptor_laplace_l2
+    seen = {}
+    for name in (None, "auto", "tensor", "fp32"):
+        seen[name] = call.kernel_matvec(desc, a, b, c, None, *tail, name)
+        assert torch.equal(seen[name], kermac.kernel_matvec(desc, a, b, c, bandwidth=8.0, contraction=name, debug=True))
+    assert torch.equal(seen["auto"], seen["tensor"]) and not torch.equal(seen["fp32"], seen["tensor"])
+    for name in ("fp64", "FP32", 1):                         # other spellings are the Python layer's business
+        assert call.kernel_matvec(desc, a, b, c, None, *tail, name) is None
+    assert torch.equal(kermac.kernel_matvec(desc, a, b, c, bandwidth=8.0, contraction="FP32"), seen["fp32"])
+    for name in ("fp64", 1):
+        with pytest.raises(ValueError, match="contraction"):
+            kermac.kernel_matvec(desc, a, b, c, bandwidth=8.0, contraction=name)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("p", [1.0, 2.0, 1.3])
 def test_both_paths_pack_large_row_operands(p, capsys, monkeypatch):
     a, b = torch.randn(6001, 701, device="cuda"), torch.randn(6001, 701, device="cuda")
