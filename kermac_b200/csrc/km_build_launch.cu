@@ -44,14 +44,32 @@ struct BuildPlan {
 //       square  2 x 1000^2 x 64: 22.9 / 18.8   8000^2 x 96: 580 / 431   16384^2 x 256: 5330 / 4695
 //       |.|     2 x 1000^2 x 64: 28.9 / 17.6   8000^2 x 96: 637 / 429   16384^2 x 256: 5947 / 4671
 //       |.|^1.3 2 x 1000^2 x 64: 74.0 / 65.9   8000^2 x 96: 2413 / 2230 16384^2 x 256: 26139 / 24770
-//   an operand that both can only copy word by word: few tiles; for |.| and |.|^p also a short k loop
-//       square  1000^2 x 27: 33.7 / 11.2   4000^2 x 27: 66.0 / 64.8   4000^2 x 129: 206 / 245
-//       |.|     1000^2 x 27: 32.6 / 9.3    4001 x 4003 x 64: 140 / 118   8001 x 8003 x 300: 1727 / 1911
-//   both operands contiguous along the points: a short k loop, or few tiles:
-//       square  2048^2 x 64: 28.9 / 22.8   2048^2 x 512: 156 / 140   4000^2 x 512: 521 / 509
-//               4000^2 x 1024: 1029 / 1045   16384^2 x 128: 2148 / 2127   16384^2 x 256: 4111 / 4159
-//       |.|     2048^2 x 64: 33.0 / 24.8   2048^2 x 512: 171 / 158   4000^2 x 512: 581 / 569
-//               4000^2 x 1024: 1124 / 1142   16384^2 x 64: 1383 / 1279   16384^2 x 128: 2375 / 2400
+// Otherwise the gain is in how evenly tiles fall on the 148 SMs: an SM's share is ceil(4 T / 148) quarter tiles, or
+// ceil(T / 148) whole ones.  The 64 x 64 kernel is the faster one where quarters make the largest share smaller by
+// more than its longer k step costs, and where the k loop is short in any case (T: 128 x 128 tiles).
+//   an operand that both can only copy word by word (the longer step costs most here: the square above 512 tiles
+//   and |.| with a long k loop are left to the 128 x 128 kernel):
+//       square  share 2/4  8000 x 55 (T 63) x 371: 82 / 64   x 701: 144 / 114
+//               share 3/4  1279^2 (T 100) x 127: 39.1 / 33.0   x 259: 63.7 / 63.8   x 371: 84 / 88
+//                          2301^2 (T 324) x 127: 86.1 / 84.2   x 259: 159 / 164
+//               share 7/8  2801^2 (T 484) x 33: 47.3 / 45.3   x 65: 71.9 / 74.0   x 701: 522 / 643
+//               share 1    1401 x 1301 (T 121) x 33: 20.7 / 17.2   x 65: 27.5 / 26.8   x 97: 33.0 / 35.0   x 701: 146 / 203
+//       |.|     share 3/4  1279^2 x 259: 72 / 57   x 701: 162 / 140   2301^2 x 701: 428 / 383
+//               share 7/8  2801^2 x 259: 231 / 226   x 371: 314 / 317   x 701: 564 / 583
+//               share 1    1401 x 1301 x 127: 45.2 / 38.1   x 259: 72.0 / 71.9   x 701: 162 / 179
+//               4001 x 4003 (T 1024) x 65: 156 / 128   x 127: 225 / 217   x 259: 405 / 427   8001 x 8003 x 65: 540 / 490
+//       with itself (quarters below the diagonal are left out as well, T counts what is launched)
+//               square  2001^2 (T 136) x 701: 298 / 201   3601^2 (T 435) x 97: 96 / 88   x 259: 190 / 209
+//               |.|     2801^2 (T 253) x 701: 326 / 307   3601^2 x 372: 283 / 278   x 701: 494 / 508
+//   both operands contiguous along the points:
+//       square  share 7/8  2000^2 (T 256) x 200: 67.8 / 59.7   x 700: 209 / 191   2800^2 (T 484) x 1024: 589 / 530
+//               share 1    1536^2 (T 144) x 256: 46.4 / 45.4   x 512: 84.3 / 86.1   x 1024: 158 / 166
+//                          2688^2 (T 441) x 256: 121 / 119   x 512: 230 / 233   x 1024: 451 / 459
+//               4000^2 (T 1024) x 256: 273 / 268   x 512: 520 / 527   16384^2 x 128: 2145 / 2124   x 256: 4109 / 4153
+//       |.|     share 7/8  2000^2 x 200: 74.0 / 67.3   x 700: 232 / 216   2800^2 x 1024: 647 / 601
+//               share 1    1536^2 x 256: 51.6 / 50.2   x 512: 92.5 / 94.8   2112^2 (T 289) x 372: 129 / 133   x 1024: 332 / 352
+//               with itself 1536^2 x 700: 131 / 103   4000^2 (T 528) x 372: 266 / 229
+//               4000^2 x 256: 303 / 293   x 512: 580 / 576   16384^2 x 96: 1858 / 1825   x 128: 2374 / 2397
 //   |.|^1.3, operands not held as aligned rows: a short k loop, or up to 2048 tiles:
 //       contiguous points 2048^2 x 512: 923 / 814   4000^2 x 1024: 6276 / 6079   4736 x 4096 x 600: 4217 / 4229
 //               4400^2 x 600: 4732 / 4359   5760^2 x 600: 7340 / 7240   16384^2 x 128: 12559 / 12527   x 256: 24802 / 24864
@@ -66,11 +84,21 @@ struct BuildPlan {
 bool small_preferred(const BuildParams& p, bool avec, bool bvec, bool awide, bool bwide) {
     const bool rows = awide && bwide && !(avec && bvec);
     if (p.inner_id == IN_DIFF_POW) return rows || p.K <= 128 || (long long)p.tiles_m * p.tiles_n * p.L <= 2048;
+    if (rows) return true;
     const long long tiles =
         (p.symmetric ? (long long)p.tiles_n * (p.tiles_n + 1) / 2 : (long long)p.tiles_m * p.tiles_n) * p.L;
-    if (!awide || !bwide) return tiles <= 512 || (p.inner_id == IN_DIFF_ABS && p.K <= 128);
-    if (rows) return true;
-    if (p.K <= (p.inner_id == IN_DIFF_ABS ? 96 : 128)) return true;
+    const bool absolute = p.inner_id == IN_DIFF_ABS;
+    const long long sms = sm_count(), quarters = ceil_div_ll(4 * tiles, sms), whole = 4 * ceil_div_ll(tiles, sms);
+    if (!awide || !bwide) {
+        if (absolute && p.K <= 128) return true;
+        if (p.symmetric) return tiles <= sms || (tiles <= 512 && p.K <= (absolute ? 512 : 192));
+        if (tiles > 512) return false;
+        if (absolute) return 4 * quarters <= 3 * whole || p.K <= 256;
+        return 2 * quarters <= whole || p.K <= (4 * quarters <= 3 * whole ? 192 : 48);
+    }
+    if (p.K <= (absolute ? 96 : 128)) return true;
+    // (many waves even out by themselves)
+    if (p.K > 256 && quarters == whole && tiles <= 5 * sms && !p.symmetric) return false;
     return tiles <= 512 || (tiles <= 1024 && p.K <= 512);
 }
 

@@ -1,6 +1,9 @@
-"""The automatic splits of cdist_grad (over k) and kernel_matvec (over m), as their scratch sizes show them: the
-planner looks at a few candidates only, and has to find what trying every split finds.  No GPU: the planner then
-assumes 148 SMs."""
+"""What the planners choose, without a GPU (they then assume 148 SMs).
+
+Splits: the automatic ones of cdist_grad (over k) and kernel_matvec (over m), as their scratch sizes show them: the
+planner looks at a few candidates only, and has to find what trying every split finds.
+
+Tiles: the 64 x 64 build kernel is taken where it measured faster than the 128 x 128 one and not elsewhere."""
 import ctypes
 import math
 import random
@@ -115,3 +118,38 @@ def test_planning_stays_cheap_for_long_sums():
             plan()
             best = min(best, time.perf_counter() - began)
         assert best < 20e-6        # (every split tried: 33 and 58 us where this takes 8 and 5)
+
+
+# us on B200, 128 x 128 / 64 x 64 kernel, for the square step
+@pytest.mark.parametrize("layout, shape, tile", [
+    ("unaligned", (1, 8000, 55, 701), 64),         # 144 / 110
+    ("unaligned", (1, 1279, 1279, 127), 64),       # 39 / 33
+    ("unaligned", (2, 7954, 55, 33), 64),          # 18.7 / 16.6
+    ("unaligned", (2, 7954, 55, 371), 128),        # 82 / 107
+    ("unaligned", (1, 2001, 2001, 371), 128),      # 148 / 176
+    ("unaligned", (1, 2801, 2801, 129), 128),      # 117 / 127
+    ("aligned", (1, 1536, 1536, 256), 64),         # 47.3 / 45.3
+    ("aligned", (1, 1536, 1536, 700), 128),        # 111 / 115
+    ("aligned", (1, 2112, 2112, 1024), 128),       # 302 / 313
+    ("aligned", (1, 2000, 2000, 700), 64),         # 209 / 195
+    ("aligned", (1, 2800, 2800, 700), 64),         # 408 / 371
+    ("aligned with itself", (1, 1536, 1536, 700), 64),     # 113 / 90
+    ("unaligned with itself", (1, 2001, 2001, 701), 64),   # 298 / 201
+    ("unaligned with itself", (1, 3601, 3601, 259), 128),  # 190 / 209
+    ("rows", (1, 1536, 1536, 1024), 64),           # rows that both kernels read: always the 64 x 64 one
+])
+def test_build_tile_sizes(layout, shape, tile):
+    L, M, N, K = shape
+    a = _native.KmBuildArgs()
+    a.m, a.n, a.k, a.l = M, N, K, L
+    a.a, a.b, a.out = 0x100000, 0x200000, 0x300000
+    if layout == "rows":
+        a.a_stride_m, a.a_stride_k, a.b_stride_n, a.b_stride_k = K, 1, K, 1
+    else:
+        pitch = 4 if layout.startswith("aligned") else 5
+        a.b = a.a if "itself" in layout else a.b
+        a.a_stride_m, a.a_stride_k, a.b_stride_n, a.b_stride_k = 1, _ceil(M, 8) * 8 + pitch, 1, _ceil(N, 8) * 8 + pitch
+    a.a_stride_l, a.b_stride_l = (M + 16) * (K + 16) // 4 * 4 * 8, (N + 16) * (K + 16) // 4 * 4 * 8
+    a.out_stride_m, a.out_stride_n, a.out_stride_l = 1, M, M * N
+    a.inner_power, a.outer_power = _native.POW_SQUARE, _native.POW_SQRT
+    assert _native.describe_build(a).split(";")[0].endswith(f"kernel_tile={tile}")
