@@ -6,7 +6,7 @@
 // 128 x 128 kernels' work and blocks hide one another's staging and stores.  The price is 3 shared
 // loads and 8 duplicate moves for 16 packed pairs instead of 4 and 8 for 32, which the square and |.|
 // steps pay once the k loop is long; the fractional power is bound by its own dependency chain and is
-// faster here at every size.  small_preferred() in km_build_launch.cu has the measured line.
+// faster here for few tiles and level for many.  small_preferred() in km_build_launch.cu has the measured line.
 //
 // Operands are staged k-major ([k][64]) whatever their layout, in slabs of 16 k rows:
 //   TMA = true    both operands contiguous along the tile dimension and 16-byte aligned: tiled TMA

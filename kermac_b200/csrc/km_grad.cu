@@ -9,8 +9,8 @@
 //   - differences, weights and channel FMAs run on packed pairs along m;
 //   - the contracted k range can be split over several thread blocks, whose partial
 //     tiles go to caller-provided scratch and are summed in a fixed order by a
-//     second kernel, so results do not depend on scheduling.  The split is chosen so
-//     that the thread blocks fill whole waves of the machine (two blocks per SM);
+//     second kernel, so results do not depend on scheduling.  The split is the one with
+//     the least estimated time (preferred_split);
 //   - blocks that share a tile of the weight matrix a (the n-tiles of one m-column and
 //     k range) are neighbours in launch order, so a is read from DRAM once;
 //   - p = 1.5 takes |x|^(p-1) as one sqrt.approx instead of the lg2 / ex2 pair.

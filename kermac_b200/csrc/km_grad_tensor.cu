@@ -591,7 +591,6 @@ int grad_tensor_launch(const GradTensorParams& p, int norm_kind, cudaStream_t st
 // Row groups per block: as many as tensor memory holds (two A buffers of 32 columns and two accumulator
 // sets of 2 OT columns per row group).
 int gt_rg_for(int ot) { return ot == 64 ? 2 : 4; }
-int gt_blocks_per_sm(int ot) { return ot == 64 ? GtShape<64, 2>::BLOCKS_PER_SM : ot == 32 ? GtShape<32, 4>::BLOCKS_PER_SM : GtShape<16, 4>::BLOCKS_PER_SM; }
 
 int grad_tensor_take_wait_flag() {
     int v = 0, zero = 0;

@@ -38,7 +38,6 @@ constexpr int GT_BK = 32;          // k rows per staged slab; k ranges of a spli
 inline int gt_ot_for(int o) { return o > 32 ? 64 : (o > 16 ? 32 : 16); }
 int gt_rg_for(int ot);                                 // row groups of 128 pairs per thread block
 inline int gt_tn_for(int ot) { return 4 * gt_rg_for(ot); }
-int gt_blocks_per_sm(int ot);
 constexpr int GT_NORM_SQRT = 3;
 struct GradTensorParams {
     int M, N, O, K, L;

@@ -5,7 +5,8 @@
 // A call of cdist / run_kernel / cdist_grad / kernel_matvec on a small problem is bound by the host:
 // checking three tensors, filling an argument struct through ctypes and asking torch for an output took
 // 22 - 35 us in Python against 4 - 10 us of GPU time.  The functions here do the same work on the
-// tensors' C++ objects (about 4 us including the launch).
+// tensors' C++ objects (5 to 7 us including the launch, by the machine; 10 to 12 us for a call that splits or packs: it
+// plans twice, takes scratch and launches two or three kernels).
 //
 // They accept what a correct, ordinary call passes and nothing else: for anything they do not recognise
 // (wrong types, shapes or devices, environment overrides, tensor-valued p, ...) they return None without
