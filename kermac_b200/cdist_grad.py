@@ -141,9 +141,9 @@ def cdist_grad(
     for p = 1, as in the reference's kernel (include/p_norm_gradient.cuh:373-394).
 
     `contraction` (not in the reference) selects where the products with `c` run: "fp32" as
-    packed FP32 FMAs, "tensor" on the tcgen05 tensor cores (three tf32 products per term,
-    fp32-level accuracy), "auto" the tensor cores from 17 channels and 256 k on.  The tensor-core
-    kernel bounds its waits; one that runs out is reported by
+    packed FP32 FMAs, "tensor" on the tcgen05 tensor cores (every factor split so that
+    fp32-level accuracy is kept), "auto" the tensor cores from 17 channels and 256 k on, for p = 1 and
+    many rows n from 5 channels on.  The tensor-core kernels bound their waits; one that runs out is reported by
     `kermac_b200._native.device_error_flag()`.
 
     Raises:

@@ -186,7 +186,7 @@ int encode_operand(CUtensorMap* map, const float* base, int extent, int K, int L
 }
 
 int encode_box(CUtensorMap* map, const float* base, int inner, int outer, int L, long long s_outer, long long s_l,
-               int box_inner, int box_outer) {
+               int box_inner, int box_outer, bool swizzle_128b) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return fail(KM_ERR_INTERNAL, "cuTensorMapEncodeTiled is not available from this driver");
     const cuuint64_t row_bytes = (static_cast<cuuint64_t>(inner) * 4 + 15) & ~static_cast<cuuint64_t>(15);
@@ -199,8 +199,8 @@ int encode_box(CUtensorMap* map, const float* base, int inner, int outer, int L,
     cuuint32_t box[3]          = {static_cast<cuuint32_t>(box_inner), static_cast<cuuint32_t>(box_outer), 1};
     cuuint32_t estr[3]         = {1, 1, 1};
     CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(base), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                    CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle_128b ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                    CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(KM_ERR_INTERNAL, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
     return 0;
 }
@@ -257,8 +257,8 @@ int encode_tma_operand(CUtensorMap* map, const float* base, int extent, int K, i
     return encode_operand(map, base, extent, K, L, s_k, s_l, box_k);
 }
 int encode_tma_box(CUtensorMap* map, const float* base, int inner, int outer, int L, long long s_outer, long long s_l,
-                   int box_inner, int box_outer) {
-    return encode_box(map, base, inner, outer, L, s_outer, s_l, box_inner, box_outer);
+                   int box_inner, int box_outer, bool swizzle_128b) {
+    return encode_box(map, base, inner, outer, L, s_outer, s_l, box_inner, box_outer, swizzle_128b);
 }
 bool tma_operand_ok(const float* base, long long s_t, long long s_k, long long s_l, int K, int L) {
     return operand_tma_ok(base, s_t, s_k, s_l, K, L);
@@ -348,7 +348,8 @@ extern "C" int kermac_b200_device_error_flag(void) {
     if (v) cudaMemcpyToSymbol(km::g_tma_wait_expired, &zero, sizeof(int));
     const int mv = km::matvec_take_wait_flag();
     const int gv = km::grad_tensor_take_wait_flag();
+    const int hv = km::grad_sign_take_wait_flag();
     const int sv = km::small_take_wait_flag();
-    if (mv < 0 || gv < 0 || sv < 0) return KM_ERR_INTERNAL;
-    return (v || mv || gv || sv) ? 1 : 0;
+    if (mv < 0 || gv < 0 || hv < 0 || sv < 0) return KM_ERR_INTERNAL;
+    return (v || mv || gv || hv || sv) ? 1 : 0;
 }

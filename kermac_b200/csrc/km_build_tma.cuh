@@ -23,9 +23,10 @@ int encode_tma_operand(CUtensorMap* map, const float* base, int extent, int K, i
                        int box_k);
 // Describes an fp32 matrix (inner extent contiguous, `outer` rows s_outer elements apart, L batch entries
 // s_l apart, s_l == 0 for a broadcast one) as a rank-3 tensor with a box of box_inner x box_outer x 1.
-// The base must be 16-byte aligned, s_outer and s_l multiples of 4 elements, box_inner * 4 a multiple of 16.
+// The base must be 16-byte aligned, s_outer and s_l multiples of 4 elements, box_inner * 4 a multiple of 16
+// (128 with the 128-byte swizzle, which stores 16-byte chunk c of row r at chunk position c ^ (r % 8)).
 int encode_tma_box(CUtensorMap* map, const float* base, int inner, int outer, int L, long long s_outer, long long s_l,
-                   int box_inner, int box_outer);
+                   int box_inner, int box_outer, bool swizzle_128b = false);
 // True when an operand with these strides can be described that way.
 bool tma_operand_ok(const float* base, long long s_t, long long s_k, long long s_l, int K, int L);
 

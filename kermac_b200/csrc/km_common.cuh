@@ -75,6 +75,31 @@ __device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
     return r;
 }
 
+// ---------------------------------------------------------------- bf16 pieces
+// An fp32 value is the sum of three bf16 ones: the upper half of its bits, of what is left (exact, at most 16
+// significant bits) and of what is left then (at most 8).
+// The upper halves of two floats as a bf16 pair, the first in the low half.
+__device__ __forceinline__ uint32_t upper_halves(u64 v) {
+    uint32_t lo = static_cast<uint32_t>(v), hi = static_cast<uint32_t>(v >> 32), w;
+    asm("prmt.b32 %0, %1, %2, 0x7632;" : "=r"(w) : "r"(lo), "r"(hi));
+    return w;
+}
+__device__ __forceinline__ u64 bf16_remainder2(u64 v) { return sub2(v, v & 0xFFFF0000FFFF0000ull); }
+// The pieces where that goes wrong (the remainders are NaN then): an infinite value has no remainder, and every NaN
+// has to stay one.
+__device__ __forceinline__ void bf16_pieces_special(u64 v, uint32_t& w1, uint32_t& w2, uint32_t& w3) {
+    float x[2], r[2];
+    unpack2(v, x[0], x[1]);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        x[i] = x[i] == x[i] ? x[i] : __int_as_float(0x7FFFFFFF);
+        r[i] = fabsf(x[i]) == __int_as_float(0x7F800000) ? 0.0f : x[i] - __uint_as_float(__float_as_uint(x[i]) & 0xFFFF0000u);
+    }
+    w1 = upper_halves(pack2(x[0], x[1]));
+    w2 = upper_halves(pack2(r[0], r[1]));
+    w3 = upper_halves(bf16_remainder2(pack2(r[0], r[1])));
+}
+
 // ---------------------------------------------------------------- exp2 on the FP32 pipe
 // The fractional-power inner step costs two MUFU operations per element (lg2, ex2)
 // and the MUFU pipe has 16 lanes per SM against 128 FP32 lanes, so a kernel that

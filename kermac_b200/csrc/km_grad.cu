@@ -407,6 +407,7 @@ struct GradPlan {
     GradParams p;
     int ot, nt;
     bool tensor;               // channel contraction on the tensor cores (km_grad_tensor.cu)
+    bool sign;                 // p = 1 with the signs as a matrix operand (km_grad_sign.cu)
     int splits_wanted;
     long long partial_elems;   // elements of one dense partial result
 };
@@ -427,7 +428,7 @@ int preferred_split(const GradPlan& plan, int norm_type, bool square_root) {
     const long long sms    = sm_count();
     const double bytes     = 4.0 * p.L * p.O * p.N * p.M;
     if (blocks <= 0 || slabs <= 1) return 1;
-    double slab_us = 2.0;
+    double slab_us = plan.sign ? 1.0 : 2.0;
     if (!plan.tensor) {
         slab_us = 0.6 + 0.16 * plan.nt * (1 + plan.ot);
         if (norm_type == KM_NORM_P) slab_us += (square_root ? 0.5 : 1.4) * plan.nt;
@@ -442,6 +443,34 @@ int preferred_split(const GradPlan& plan, int norm_type, bool square_root) {
     long long last   = std::min(slabs, 16 * sms / blocks);
     if ((double)last > cap) last = (long long)cap;
     return cheapest_split(slabs, last, cost);
+}
+
+// Whether p = 1 takes the kernel with the signs as a matrix operand (km_grad_sign.cu).  A block of it costs the same
+// for 1 to 128 rows n and a multiple of its channel tile, so the three kernels are compared by their tiles times what a
+// slab of 32 k of a tile takes on an SM, us.  Measured on B200 at K = 30000, M = 4096, N = 256, ms (the choice before
+// in brackets): 4 channels 6.24 [FP32 6.23], 8: 6.86 [FP32 10.6], 16: 8.87 [FP32 20.3], 32: 11.9 [weights 22.0],
+// 64: 23.8 [weights 29.5]; where b or c cannot be copied 16 bytes at a time 10.1 at 4 and 20.5 at 32.  Few k leave a
+// block mostly waiting for its first slabs (64 x 1000 x 1000 x 16: 96 us against 56), so at least 256.
+bool sign_preferred(const KmGradArgs* a) {
+    if (a->norm_type != KM_NORM_L1 || a->k < 1 || a->contraction == KM_CONTRACT_FP32) return false;
+    if (a->contraction == KM_CONTRACT_TENSOR) return a->n >= 96;      // the other tensor-core kernel for fewer rows
+    if (a->n < 64 || a->k < 8 * G_BK) return false;
+    const bool vec = aligned16(a->b) && aligned16(a->c) && a->ldb % 4 == 0 && a->ldc % 4 == 0 && a->b_stride_l % 4 == 0 &&
+                     a->c_stride_l % 4 == 0;
+    const int ot         = gs_ot_for(a->o);
+    const double slab_us = (ot == 4 ? 0.96 : ot == 8 ? 1.06 : ot == 16 ? 0.68 : 0.92) * (vec ? 1.0 : 1.65);
+    const double sign    = slab_us * ceil_div_ll(a->m, gs_mt_for(ot)) * ceil_div_ll(a->n, GS_TN) * ceil_div_ll(a->o, ot);
+    double other;
+    if (a->o >= KM_GRAD_TENSOR_MIN_O) {
+        const int wt = gt_ot_for(a->o);
+        other = (wt == 64 ? 1.14 : 1.7) * ceil_div_ll(a->m, GT_TM) * ceil_div_ll(a->n, gt_tn_for(wt)) * ceil_div_ll(a->o, wt);
+    } else {
+        int ft = 1;
+        while (ft < a->o && ft < 16) ft *= 2;
+        const int nt = nt_for(ft);
+        other = 0.9 * (0.6 + 0.16 * nt * (1 + ft)) * ceil_div_ll(a->m, G_TM) * ceil_div_ll(a->n, 16 * nt) * ceil_div_ll(a->o, ft);
+    }
+    return 1.05 * sign < other;
 }
 
 int make_grad_plan(const KmGradArgs* a, GradPlan* plan) {
@@ -482,11 +511,13 @@ int make_grad_plan(const KmGradArgs* a, GradPlan* plan) {
     // 64).  The tensor kernel needs at least one slab of k.
     plan->tensor = a->k > 0 && (a->contraction == KM_CONTRACT_TENSOR ||
                                 (a->contraction == KM_CONTRACT_AUTO && a->o >= KM_GRAD_TENSOR_MIN_O && a->k >= 8 * G_BK));
-    if (plan->tensor) ot = gt_ot_for(a->o);
+    plan->sign = sign_preferred(a);
+    if (plan->sign) plan->tensor = true;
+    if (plan->tensor) ot = plan->sign ? gs_ot_for(a->o) : gt_ot_for(a->o);
     plan->ot = ot;
     plan->nt = nt_for(ot);
-    p.tiles_m  = (int)ceil_div_ll(p.M, plan->tensor ? GT_TM : G_TM);
-    p.tiles_n  = (int)ceil_div_ll(p.N, plan->tensor ? gt_tn_for(ot) : 16 * plan->nt);
+    p.tiles_m  = (int)ceil_div_ll(p.M, plan->sign ? gs_mt_for(ot) : plan->tensor ? GT_TM : G_TM);
+    p.tiles_n  = (int)ceil_div_ll(p.N, plan->sign ? GS_TN : plan->tensor ? gt_tn_for(ot) : 16 * plan->nt);
     p.o_chunks = (int)ceil_div_ll(p.O > 0 ? p.O : 1, ot);
     p.a_vec    = aligned16(p.A) && p.lda % 4 == 0 && p.a_sl % 4 == 0;
     if ((long long)p.tiles_m * p.tiles_n > (1LL << 26)) return fail(KM_ERR_TOO_LARGE, "too many output tiles");
@@ -560,7 +591,9 @@ extern "C" int kermac_b200_cdist_grad(const KmGradArgs* args, void* stream) {
         t.tiles_m = p.tiles_m; t.tiles_n = p.tiles_n; t.o_chunks = p.o_chunks; t.splits = p.splits;
         t.k_per_split = p.k_per_split; t.split_stride = p.split_stride;
         t.c_vec = aligned16(p.C) && p.ldc % 4 == 0 && p.c_sl % 4 == 0;
-        if (int rc = grad_tensor_launch(t, sqrt_route ? GT_NORM_SQRT : args->norm_type, st)) return rc;
+        t.e_vec = p.e_vec;
+        if (int rc = plan.sign ? grad_sign_launch(t, st) : grad_tensor_launch(t, sqrt_route ? GT_NORM_SQRT : args->norm_type, st))
+            return rc;
     } else {
     GradChoice choice = {nullptr, 0};
     switch (args->norm_type) {

@@ -53,11 +53,20 @@ struct GradTensorParams {
     int k_per_split;
     long long split_stride;
     int c_vec;                                      // c rows can be read 16 bytes at a time
+    int e_vec;                                      // rows of the destination can be written 16 bytes at a time
 };
 int grad_tensor_launch(const GradTensorParams& p, int norm_kind, cudaStream_t st);
 // Reads back and clears the wait-ran-out flag of the tensor-core gradient kernel; the device
 // must already be synchronised.  0 / 1, or -1 on error.
 int grad_tensor_take_wait_flag();
+
+// The form for p = 1, where the signs are an exact matrix operand (km_grad_sign.cu): n rows, channels and m per
+// thread block.  Takes the same parameter block (ot = gs_ot_for(O)).
+constexpr int GS_TN = 128;
+inline int gs_ot_for(int o) { return o > 16 ? 32 : (o > 8 ? 16 : (o > 4 ? 8 : 4)); }
+constexpr int gs_mt_for(int ot) { return ot >= 16 ? 4 : 8; }
+int grad_sign_launch(const GradTensorParams& p, cudaStream_t st);
+int grad_sign_take_wait_flag();
 
 inline long long ceil_div_ll(long long a, long long b) { return (a + b - 1) / b; }
 

@@ -1,5 +1,5 @@
 // Inline-PTX helpers for the 5th-generation tensor cores of sm_100a: tensor-memory
-// allocation, shared-memory matrix descriptors, tcgen05.mma (kind::tf32, one CTA),
+// allocation, shared-memory matrix descriptors, tcgen05.mma (kind::tf32 and bf16, one CTA),
 // commit to an mbarrier and accumulator read-back.
 #pragma once
 
@@ -23,6 +23,16 @@ __device__ __forceinline__ uint64_t smem_desc_k_major_sw128(uint32_t smem_addr) 
 // N >> 3 in [17,23), M >> 4 in [24,29).
 __host__ __device__ constexpr uint32_t instr_desc_tf32(int M, int N) {
     return (1u << 4) | (2u << 7) | (2u << 10) | (static_cast<uint32_t>(N >> 3) << 17) | (static_cast<uint32_t>(M >> 4) << 24);
+}
+
+// The same for an operand stored as 64-byte rows with the 64-byte swizzle: row r at r * 64 bytes, its 16-byte chunk c
+// at chunk position c ^ ((r / 2) % 4), 8-row groups 512 bytes apart, tiles 512-byte aligned (layout type 4).
+__device__ __forceinline__ uint64_t smem_desc_k_major_sw64(uint32_t smem_addr) {
+    return static_cast<uint64_t>((smem_addr & 0x3FFFFu) >> 4) | (1ull << 16) | (32ull << 32) | (1ull << 46) | (4ull << 61);
+}
+// Instruction descriptor for D(f32) += A(bf16) * B(bf16) (format 1), both operands K-major.
+__host__ __device__ constexpr uint32_t instr_desc_bf16(int M, int N) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (static_cast<uint32_t>(N >> 3) << 17) | (static_cast<uint32_t>(M >> 4) << 24);
 }
 
 // Executed by one whole warp.  Writes the allocation's base address to *dst_smem.
@@ -74,6 +84,23 @@ __device__ __forceinline__ void mma_tf32_a_tmem(uint32_t d_tmem, uint32_t a_tmem
         ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(static_cast<uint32_t>(accumulate))
         : "memory");
 }
+// D(f32) (+)= A * B with bf16 operands, 16 k per instruction: A in tensor memory (two k per 32-bit column, the
+// even one in the low half), B in shared memory.
+__device__ __forceinline__ void mma_bf16_a_tmem(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, bool accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(static_cast<uint32_t>(accumulate))
+        : "memory");
+}
+// True on one lane of the (converged) warp.  What it guards stays warp-uniform code, so descriptors and addresses
+// are computed once per warp.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
 // Warp-wide: lane i writes 16 consecutive 32-bit columns of tensor-memory lane (taddr.lane + i).
 // Complete only after wait_st().
 __device__ __forceinline__ void st_32x32b_x16(uint32_t taddr, const uint32_t (&r)[16]) {
@@ -92,6 +119,24 @@ __device__ __forceinline__ void ld_32x32b_x16(uint32_t taddr, uint32_t (&r)[16])
         : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
           "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr)
+        : "memory");
+}
+
+// Three groups of 16 columns, one wait.
+__device__ __forceinline__ void ld3_32x32b_x16(uint32_t t0, uint32_t t1, uint32_t t2, uint32_t (&r0)[16], uint32_t (&r1)[16],
+                                               uint32_t (&r2)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%48];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%49];\n\t"
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%32, %33, %34, %35, %36, %37, %38, %39, %40, %41, %42, %43, %44, %45, %46, %47}, [%50];\n\t"
+        "tcgen05.wait::ld.sync.aligned;"
+        : "=r"(r0[0]), "=r"(r0[1]), "=r"(r0[2]), "=r"(r0[3]), "=r"(r0[4]), "=r"(r0[5]), "=r"(r0[6]), "=r"(r0[7]),
+          "=r"(r0[8]), "=r"(r0[9]), "=r"(r0[10]), "=r"(r0[11]), "=r"(r0[12]), "=r"(r0[13]), "=r"(r0[14]), "=r"(r0[15]),
+          "=r"(r1[0]), "=r"(r1[1]), "=r"(r1[2]), "=r"(r1[3]), "=r"(r1[4]), "=r"(r1[5]), "=r"(r1[6]), "=r"(r1[7]),
+          "=r"(r1[8]), "=r"(r1[9]), "=r"(r1[10]), "=r"(r1[11]), "=r"(r1[12]), "=r"(r1[13]), "=r"(r1[14]), "=r"(r1[15]),
+          "=r"(r2[0]), "=r"(r2[1]), "=r"(r2[2]), "=r"(r2[3]), "=r"(r2[4]), "=r"(r2[5]), "=r"(r2[6]), "=r"(r2[7]),
+          "=r"(r2[8]), "=r"(r2[9]), "=r"(r2[10]), "=r"(r2[11]), "=r"(r2[12]), "=r"(r2[13]), "=r"(r2[14]), "=r"(r2[15])
+        : "r"(t0), "r"(t1), "r"(t2)
         : "memory");
 }
 
