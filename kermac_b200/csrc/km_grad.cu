@@ -409,6 +409,7 @@ struct GradPlan {
     bool tensor;               // channel contraction on the tensor cores (km_grad_tensor.cu)
     bool sign;                 // p = 1 with the signs as a matrix operand (km_grad_sign.cu)
     int splits_wanted;
+    int sign_splits;           // where the sign kernel runs: how many of them it takes
     long long partial_elems;   // elements of one dense partial result
 };
 
@@ -511,13 +512,12 @@ int make_grad_plan(const KmGradArgs* a, GradPlan* plan) {
     // 64).  The tensor kernel needs at least one slab of k.
     plan->tensor = a->k > 0 && (a->contraction == KM_CONTRACT_TENSOR ||
                                 (a->contraction == KM_CONTRACT_AUTO && a->o >= KM_GRAD_TENSOR_MIN_O && a->k >= 8 * G_BK));
-    plan->sign = sign_preferred(a);
-    if (plan->sign) plan->tensor = true;
-    if (plan->tensor) ot = plan->sign ? gs_ot_for(a->o) : gt_ot_for(a->o);
+    plan->sign = false;
+    if (plan->tensor) ot = gt_ot_for(a->o);
     plan->ot = ot;
     plan->nt = nt_for(ot);
-    p.tiles_m  = (int)ceil_div_ll(p.M, plan->sign ? gs_mt_for(ot) : plan->tensor ? GT_TM : G_TM);
-    p.tiles_n  = (int)ceil_div_ll(p.N, plan->sign ? GS_TN : plan->tensor ? gt_tn_for(ot) : 16 * plan->nt);
+    p.tiles_m  = (int)ceil_div_ll(p.M, plan->tensor ? GT_TM : G_TM);
+    p.tiles_n  = (int)ceil_div_ll(p.N, plan->tensor ? gt_tn_for(ot) : 16 * plan->nt);
     p.o_chunks = (int)ceil_div_ll(p.O > 0 ? p.O : 1, ot);
     p.a_vec    = aligned16(p.A) && p.lda % 4 == 0 && p.a_sl % 4 == 0;
     if ((long long)p.tiles_m * p.tiles_n > (1LL << 26)) return fail(KM_ERR_TOO_LARGE, "too many output tiles");
@@ -525,6 +525,16 @@ int make_grad_plan(const KmGradArgs* a, GradPlan* plan) {
 
     plan->splits_wanted = preferred_split(*plan, a->norm_type, !a->p.ptr && a->p.value == 1.5f);
     plan->partial_elems = (long long)p.L * p.O * p.N * p.M;
+    if (sign_preferred(a) && ceil_div_ll(p.M, 4) * ceil_div_ll(p.N, GS_TN) <= (1LL << 26)) {
+        // its split stays within the one above, and so within the scratch that callers were told of: its blocks are no
+        // larger than the other kernels' (512 results per channel against 512 to 4096), it rarely wants more
+        plan->sign = plan->tensor = true;
+        plan->ot   = gs_ot_for(a->o);
+        p.tiles_m  = (int)ceil_div_ll(p.M, gs_mt_for(plan->ot));
+        p.tiles_n  = (int)ceil_div_ll(p.N, GS_TN);
+        p.o_chunks = (int)ceil_div_ll(p.O, plan->ot);
+        plan->sign_splits = std::min(plan->splits_wanted, preferred_split(*plan, a->norm_type, false));
+    }
     return 0;
 }
 
@@ -559,6 +569,7 @@ extern "C" int kermac_b200_cdist_grad(const KmGradArgs* args, void* stream) {
             splits = 1;   // automatic mode falls back to a single pass
         }
     }
+    if (plan.sign && args->split_k == 0) splits = std::min(splits, plan.sign_splits);
     int slabs       = (int)ceil_div_ll(p.K > 0 ? p.K : 1, G_BK);
     p.k_per_split   = (int)ceil_div_ll(slabs, splits) * G_BK;
     splits          = (int)ceil_div_ll(p.K > 0 ? p.K : 1, p.k_per_split);
