@@ -164,7 +164,7 @@ int64_t kermac_b200_build_tile_count(const KmBuildArgs* args);
  * in fp32: fp32-level accuracy, not the FP32 kernel's bits).  For KM_NORM_L1 and 96 or more rows n the
  * signs themselves are the matrix operand and the products c * a are split, into three bf16 pieces that lose
  * nothing.  KM_CONTRACT_AUTO takes the tensor cores from 17 channels and 256 k on, and for KM_NORM_L1 from 64
- * rows and 256 k on wherever that is estimated to be the faster form (5 channels, for many rows).  The weights
+ * rows and 256 k on wherever that is estimated to be the faster form (3 channels on, for many rows).  The weights
  * a * g(d - b) are computed in FP32 either way.  A bounded wait inside a tensor-core kernel that runs out raises
  * kermac_b200_device_error_flag().
  */

@@ -143,7 +143,7 @@ def cdist_grad(
     `contraction` (not in the reference) selects where the products with `c` run: "fp32" as
     packed FP32 FMAs, "tensor" on the tcgen05 tensor cores (every factor split so that
     fp32-level accuracy is kept), "auto" the tensor cores from 17 channels and 256 k on, for p = 1 and
-    many rows n from 5 channels on.  The tensor-core kernels bound their waits; one that runs out is reported by
+    many rows n from 3 channels on.  The tensor-core kernels bound their waits; one that runs out is reported by
     `kermac_b200._native.device_error_flag()`.
 
     Raises:

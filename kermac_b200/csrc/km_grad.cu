@@ -449,8 +449,8 @@ int preferred_split(const GradPlan& plan, int norm_type, bool square_root) {
 // Whether p = 1 takes the kernel with the signs as a matrix operand (km_grad_sign.cu).  A block of it costs the same
 // for 1 to 128 rows n and a multiple of its channel tile, so the three kernels are compared by their tiles times what a
 // slab of 32 k of a tile takes on an SM, us.  Measured on B200 at K = 30000, M = 4096, N = 256, ms (the choice before
-// in brackets): 4 channels 6.24 [FP32 6.23], 8: 6.86 [FP32 10.6], 16: 8.87 [FP32 20.3], 32: 11.9 [weights 22.0],
-// 64: 23.8 [weights 29.5]; where b or c cannot be copied 16 bytes at a time 10.1 at 4 and 20.5 at 32.  Few k leave a
+// // in brackets): 2 channels 5.49 [FP32 4.45], 4: 5.49 [FP32 6.23], 8: 5.98 [FP32 10.6], 16: 8.87 [FP32 20.3], 32: 11.9 [weights 22.0],
+// 64: 23.8 [weights 29.5]; where b or c cannot be copied 16 bytes at a time 9.4 at 4, 17.2 at 16 and 20.5 at 32.  Few k leave a
 // block mostly waiting for its first slabs (64 x 1000 x 1000 x 16: 96 us against 56), so at least 256.
 bool sign_preferred(const KmGradArgs* a) {
     if (a->norm_type != KM_NORM_L1 || a->k < 1 || a->contraction == KM_CONTRACT_FP32) return false;
@@ -459,7 +459,7 @@ bool sign_preferred(const KmGradArgs* a) {
     const bool vec = aligned16(a->b) && aligned16(a->c) && a->ldb % 4 == 0 && a->ldc % 4 == 0 && a->b_stride_l % 4 == 0 &&
                      a->c_stride_l % 4 == 0;
     const int ot         = gs_ot_for(a->o);
-    const double slab_us = (ot == 4 ? 0.96 : ot == 8 ? 1.06 : ot == 16 ? 0.68 : 0.92) * (vec ? 1.0 : 1.65);
+    const double slab_us = (ot == 4 ? 0.85 : ot == 8 ? 0.92 : ot == 16 ? 0.68 : 0.92) * (vec ? 1.0 : 1.8);
     const double sign    = slab_us * ceil_div_ll(a->m, gs_mt_for(ot)) * ceil_div_ll(a->n, GS_TN) * ceil_div_ll(a->o, ot);
     double other;
     if (a->o >= KM_GRAD_TENSOR_MIN_O) {
@@ -469,7 +469,7 @@ bool sign_preferred(const KmGradArgs* a) {
         int ft = 1;
         while (ft < a->o && ft < 16) ft *= 2;
         const int nt = nt_for(ft);
-        other = 0.9 * (0.6 + 0.16 * nt * (1 + ft)) * ceil_div_ll(a->m, G_TM) * ceil_div_ll(a->n, 16 * nt) * ceil_div_ll(a->o, ft);
+        other = (ft == 1 ? 2.24 : ft == 2 ? 2.74 : ft == 4 ? 3.84 : ft == 8 ? 3.27 : 3.13) * ceil_div_ll(a->m, G_TM) * ceil_div_ll(a->n, 16 * nt) * ceil_div_ll(a->o, ft);
     }
     return 1.05 * sign < other;
 }

@@ -14,8 +14,8 @@
 //
 // Work decomposition: a thread block owns 128 rows n, MT columns m and up to OT channels.
 //   16 generating warps (4 groups of 4): a thread owns one row n (a tensor-memory lane); a group takes
-//      16 k of a slab of 32 for four m and writes their signs (8 columns of packed bf16 pairs per m)
-//      with tcgen05.st into a ring of A buffers, one slab each;
+//      16 k of every second slab of 32, reads them once for all m and writes the signs (8 columns of packed
+//      bf16 pairs per m) with tcgen05.st into a ring of A buffers, one slab each;
 //   8 product warps (4 with few channels): P_m for the slab, split and parked in shared memory as the B operand (K-major rows
 //      of 64 bytes, 64-byte swizzle; row = piece * OT + channel);
 //   2 warps (4 with few channels) issue the MMAs, one accumulator of 3 OT columns (rounded up to 16) per m;
@@ -29,15 +29,15 @@
 // The product warps have no global loads of their own: their fence to the asynchronous units waits for
 // every memory operation of the thread, and behind loads in flight it made each slab as long as a load.
 // What bounds it (B200, K = 30000, M = 4096, N = 256; ms, in brackets the kernel that took these calls before):
-// 8 channels 6.9 (10.6), 16: 8.9 (20.3), 32: 11.9 (22.0), 64: 23.8 (29.5); at 4 channels, 6.2, it is level with
-// the FP32 kernel.  The MMAs alone would take 2.5 ms at 32 channels (an MMA of 128 rows x N columns holds the
-// tensor pipe N / 2 cycles, also with the stores to tensor memory beside it), the ALU pipe (permutes and logic, half
-// rate) about 3.5.  At 32 channels a slab of 4 m takes some 1600 cycles: the product warps compute for 920 of
-// them (their instructions issue once in four to five cycles beside the generating warps) and a wait for a phase that
-// is long complete costs 100 to 250.  On the way here (ms at 4 / 32 channels): one thread issuing all MMAs 18.5 / -;
-// every role handing over per 16 k by its own barrier, four issuing warps 6.7 / 14.5; global loads taken from the
-// product warps 7.0 / 14.2; eight product warps and carried copy addresses 7.5 / 12.4; all MMAs of a slab in one
-// elected block 6.2 / 11.9.
+// 4 channels 5.5 (6.2), 8: 6.0 (10.6), 16: 8.9 (20.3), 32: 11.9 (22.0), 64: 23.8 (29.5).  The MMAs alone would
+// take 2.5 ms at 32 channels (an MMA of 128 rows x N columns holds the tensor pipe N / 2 cycles, also with the
+// stores to tensor memory beside it), the ALU pipe (permutes and logic, half rate) about 3.5.  At 32 channels a slab of
+// 4 m takes some 1600 cycles: the product warps compute for 920 of them (their instructions issue once in four to
+// five cycles beside the generating warps) and a wait for a phase that is long complete costs 100 to 250.  On the way
+// here (ms at 4 / 32 channels): one thread issuing all MMAs 18.5 / -; every role handing over per 16 k by its own
+// barrier, four issuing warps 6.7 / 14.5; global loads taken from the product warps 7.0 / 14.2; eight product warps
+// and carried copy addresses 7.5 / 12.4; all MMAs of a slab in one elected block 6.2 / 11.9; 16 k of all eight m
+// per group and slab instead of four 5.5 / 11.9.
 // Hand-over is by mbarriers, one round per slab; every wait is bounded, and a wait that runs out sets a
 // flag (kermac_b200_device_error_flag) and lets the block run to its end without its results.
 #include <cstring>
@@ -66,7 +66,6 @@ constexpr int GS_CHAIN    = 16;     // slabs per accumulation chain
 
 template <int OT, int MT, bool TMA>
 struct GsShape {
-    static constexpr int ITEMS     = MT / 2;                           // (16 k, four m) parts of a slab: one group each
     static constexpr int COLS      = (3 * OT + 15) / 16 * 16;          // MMA width: pieces x channels
     static constexpr int P_BYTES   = COLS * GS_BK * 2;                 // split products of one m and slab
     static constexpr int A_OFF     = MT * COLS;                        // tensor-memory columns before the A buffers
@@ -89,7 +88,7 @@ struct GsShape {
     static constexpr int OCTS      = OT >= 8 ? OT / 8 : 1;             // product warps per m: eight channels each
     static constexpr int MSUB      = OT >= 8 ? 1 : 8 / OT;             // m that a product warp takes at a time
     static constexpr int STAGGER   = GS_CHAIN / MT;                    // slabs between the chain cuts of two m
-    static_assert(MT % 4 == 0 && GS_CHAIN % MT == 0 && ITEMS <= GS_GROUPS && NB >= 2 && GS_P_SLOTS <= GS_DONE &&
+    static_assert(MT % 4 == 0 && GS_CHAIN % MT == 0 && NB >= 2 && GS_P_SLOTS <= GS_DONE &&
                   SMEM <= 227 * 1024, "shape");
 };
 
@@ -146,14 +145,14 @@ grad_sign_kernel(const __grid_constant__ GradTensorParams p, const __grid_consta
     if (tid == 0) {
         for (int st = 0; st < GS_B_STAGES; ++st) {
             mbar_init(bfull(st), TMA ? 1 : 32);
-            mbar_init(bempty(st), 4 * S::ITEMS);
+            mbar_init(bempty(st), 8);                  // a slab is read by two groups of four warps
         }
         for (int sl = 0; sl < GS_AC_SLOTS; ++sl) {
             mbar_init(acfull(sl), 32);
             mbar_init(acempty(sl), S::PROD);
         }
         for (int sl = 0; sl < GS_P_SLOTS; ++sl) mbar_init(pfull(sl), S::PROD);
-        for (int b = 0; b < S::NB; ++b) mbar_init(afull(b), 4 * S::ITEMS);
+        for (int b = 0; b < S::NB; ++b) mbar_init(afull(b), 8);
         for (int i = 0; i < GS_DONE; ++i) mbar_init(done(i), S::ISSUERS);
         for (int m = 0; m < MT; ++m) {
             mbar_init(dfull(m), 1);
@@ -186,18 +185,17 @@ grad_sign_kernel(const __grid_constant__ GradTensorParams p, const __grid_consta
         const int row = 32 * q + lane;
         const int n   = n0 + row;
         const float* D = p.D + (long long)l * p.d_sl;
-        // this group's part of a slab: 16 k, four m; with two parts a slab the groups take turns at the slabs
-        const int hf = group & 1, quad = S::ITEMS == 4 ? group >> 1 : 0;
-        u64 dd[4];
+        // this group's part of a slab: 16 k; two groups make up a slab, the other two the next one
+        const int hf = group & 1;
+        u64 dd[MT];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const int m   = m0 + 4 * quad + i;
-            const float v = (n < p.N && m < p.M) ? D[(long long)n * p.ldd + m] : 0.0f;
+        for (int i = 0; i < MT; ++i) {
+            const float v = (n < p.N && m0 + i < p.M) ? D[(long long)n * p.ldd + m0 + i] : 0.0f;
             dd[i] = pack2(v, v);
         }
-        const uint32_t t_row = tmem + (static_cast<uint32_t>(32 * q) << 16) + S::A_OFF + (hf * MT + 4 * quad) * (GS_KA / 2);
+        const uint32_t t_row = tmem + (static_cast<uint32_t>(32 * q) << 16) + S::A_OFF + hf * MT * (GS_KA / 2);
         const unsigned char* brow = tiles + S::OFF_B + row * (GS_BK * 4);
-        for (int s = S::ITEMS == 4 ? 0 : group >> 1; s < nslabs; s += GS_GROUPS / S::ITEMS) {
+        for (int s = group >> 1; s < nslabs; s += GS_GROUPS / 2) {
             const int st = s % GS_B_STAGES;
             wait(bfull(st), (s / GS_B_STAGES) & 1);
             __syncwarp();
@@ -214,7 +212,7 @@ grad_sign_kernel(const __grid_constant__ GradTensorParams p, const __grid_consta
             __syncwarp();
             tc::fence_after_sync();
 #pragma unroll
-            for (int i = 0; i < 4; i += 2) {
+            for (int i = 0; i < MT; i += 2) {
                 uint32_t w[16];
 #pragma unroll
                 for (int j = 0; j < 16; ++j) w[j] = sign_pair(sub2(dd[i + (j >> 3)], b2[j & 7]));
