@@ -291,9 +291,9 @@ def grad(args, ctx):
     line["roofline"]["inner_step_ceiling_lane_ops"] = step_packed
     line["roofline"]["frac_of_inner_step_ceiling"] = (1.0 + O) * triples / (ms1 * 1e-3) / step_packed
     line["roofline"]["inner_step_ceiling_scalar_fma_lane_ops"] = step_scalar
-    # 32 and 64 channels: the tensor-core kernel (the automatic choice from 17 channels on) next to the FP32 kernel.
-    # Its bound is the tensor pipe at the rate narrow MMAs get: a 128 x 8 tf32 MMA of up to 64 output
-    # columns holds the pipe ~45 cycles; two of them (head and remainder of the weights) per 128 pairs x 8 k.
+    # (these two are ceilings of the FP32 kernel; the automatic choice for p = 1 and many rows is the sign kernel)
+    # 32 and 64 channels: the tensor-core form for p = 1 (the signs as the matrix operand) next to the FP32 kernel.
+    # Its tensor-pipe bound: one bf16 MMA of 128 rows x 96 columns (three pieces of 32 channels) x 16 k per 128 n and m.
     few = max(2, args.steps // 3)
     mma_rates = [_native.measure_pipe(kind, 4096)[0] for kind in (8, 9, 10, 11)]   # 128 x {32, 64, 128, 256} x 8
     for O2 in (32, 64):
@@ -304,21 +304,19 @@ def grad(args, ctx):
         fp_out = out2.clone()
         t_tc = _timed(run(lambda: kermac.cdist_grad(ad, bd, c2, dd, out=out2, p=1.0, contraction="tensor")), few, 1,
                       ctx.barrier) - t_flush
-        # per 128 pairs x 8 k: one MMA of 2 O2 columns (heads) and one of O2 columns (remainders)
-        per_step = float(M) * N / 128.0 * (K / 8.0)
-        wide, narrow = (mma_rates[1], mma_rates[0]) if O2 == 32 else (mma_rates[2], mma_rates[1])
-        t_bound = per_step / wide + per_step / narrow
+        # an MMA holds the tensor pipe N / 2 cycles, as the 256-column one whose rate was measured does
+        mmas = float(M) * N / 128.0 * (K / 16.0) * (O2 // 32)
+        t_bound = mmas * (96.0 / 256.0) / mma_rates[3]
         line[f"O={O2}"] = {"fp32_kernel_ms": t_fp, "tensor_kernel_ms": t_tc, "ratio": t_fp / t_tc,
                            "max_abs_diff_over_max": float((out2 - fp_out).abs().max() / fp_out.abs().max()),
                            "device_error_flag": _native.device_error_flag(),
-                           "roofline": {"bound": "tensor", "achieved": 2.0 * per_step / (t_tc * 1e-3) / 1e9,
-                                        "peak": 2.0 * per_step / t_bound / 1e9, "unit": "G narrow-MMA/s",
+                           "roofline": {"bound": "tensor", "achieved": mmas / (t_tc * 1e-3) / 1e9,
+                                        "peak": mmas / t_bound / 1e9, "unit": "G MMA/s (128 x 96 x 16 bf16)",
                                         "frac": t_bound / (t_tc * 1e-3), "traffic": None,
                                         "peak_source": "measured on this device by kermac_b200_measure_pipe kinds 8-11",
                                         "mma_per_s_n32_n64_n128_n256": mma_rates,
-                                        "note": "tcgen05.mma kind::tf32 128 x N x 8 holds the tensor pipe ~45 cycles up to "
-                                                "N = 64 and N / 2 cycles from 128 on; per 128 pairs x 8 k one of 2 O columns "
-                                                "(heads of the weights) and one of O columns (remainders)"}}
+                                        "note": "tcgen05.mma of 128 rows x N columns holds the tensor pipe N / 2 cycles; the "
+                                                "kernel is bound by forming signs and products, not by the MMAs"}}
         del c2, out2, fp_out
     if not args.no_ref_gpu:
         from baseline import ref_kernels
