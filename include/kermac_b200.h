@@ -188,6 +188,10 @@ int kermac_b200_cdist_grad(const KmGradArgs* args, void* stream);
  * this problem (0 when no split is useful). */
 int64_t kermac_b200_cdist_grad_scratch_bytes(const KmGradArgs* args);
 
+/* Writes which kernel kermac_b200_cdist_grad would launch for `args`, and its tiling, into buf (NUL terminated,
+ * truncated to buf_len). */
+int kermac_b200_describe_grad(const KmGradArgs* args, char* buf, int32_t buf_len);
+
 /*
  * Same computation and arguments as kermac_b200_cdist_grad, for callers that cannot
  * allocate device memory where they call it (a plugin inside another runtime's fixed

@@ -28,6 +28,7 @@ EXPORTED_SYMBOLS = (
     "kermac_b200_cdist_grad",
     "kermac_b200_cdist_grad_scratch_bytes",
     "kermac_b200_cdist_grad_static",
+    "kermac_b200_describe_grad",
     "kermac_b200_kernel_matvec",
     "kermac_b200_kernel_matvec_scratch_bytes",
     "kermac_b200_describe_variant",
@@ -134,6 +135,8 @@ def _declare(lib: C.CDLL) -> None:
     lib.kermac_b200_cdist_grad_scratch_bytes.restype = C.c_int64
     lib.kermac_b200_cdist_grad_static.argtypes = [C.POINTER(KmGradArgs), C.c_void_p]
     lib.kermac_b200_cdist_grad_static.restype = C.c_int
+    lib.kermac_b200_describe_grad.argtypes = [C.POINTER(KmGradArgs), C.c_char_p, C.c_int32]
+    lib.kermac_b200_describe_grad.restype = C.c_int
     lib.kermac_b200_kernel_matvec.argtypes = [C.POINTER(KmMatvecArgs), C.c_void_p]
     lib.kermac_b200_kernel_matvec.restype = C.c_int
     lib.kermac_b200_kernel_matvec_scratch_bytes.argtypes = [C.POINTER(KmMatvecArgs)]
@@ -309,6 +312,12 @@ def launch_matvec(args: KmMatvecArgs, stream_ptr: int) -> None:
 def describe_build(args: KmBuildArgs) -> str:
     buf = C.create_string_buffer(512)
     check(lib().kermac_b200_describe_variant(C.byref(args), buf, 512), "kermac_b200_describe_variant")
+    return buf.value.decode()
+
+
+def describe_grad(args: KmGradArgs) -> str:
+    buf = C.create_string_buffer(256)
+    check(lib().kermac_b200_describe_grad(C.byref(args), buf, 256), "kermac_b200_describe_grad")
     return buf.value.decode()
 
 

@@ -525,7 +525,9 @@ int make_grad_plan(const KmGradArgs* a, GradPlan* plan) {
 
     plan->splits_wanted = preferred_split(*plan, a->norm_type, !a->p.ptr && a->p.value == 1.5f);
     plan->partial_elems = (long long)p.L * p.O * p.N * p.M;
-    if (sign_preferred(a) && ceil_div_ll(p.M, 4) * ceil_div_ll(p.N, GS_TN) <= (1LL << 26)) {
+    // (its tiles and channel chunks are smaller than the ones checked above: calls that would need too many keep theirs)
+    if (sign_preferred(a) && ceil_div_ll(p.M, 4) * ceil_div_ll(p.N, GS_TN) <= (1LL << 26) &&
+        ceil_div_ll(p.O, gs_ot_for(a->o)) <= 65535) {
         // its split stays within the one above, and so within the scratch that callers were told of: its blocks are no
         // larger than the other kernels' (512 results per channel against 512 to 4096), it rarely wants more
         plan->sign = plan->tensor = true;
@@ -548,6 +550,17 @@ extern "C" int64_t kermac_b200_cdist_grad_scratch_bytes(const KmGradArgs* args) 
     int splits = args->split_k > 0 ? args->split_k : plan.splits_wanted;
     if (splits <= 1) return 0;
     return (int64_t)splits * plan.partial_elems * 4;
+}
+
+extern "C" int kermac_b200_describe_grad(const KmGradArgs* args, char* buf, int32_t buf_len) {
+    using namespace km;
+    if (!buf || buf_len <= 0) return fail(KM_ERR_NULL_POINTER, "buf is NULL or empty");
+    GradPlan plan;
+    if (int rc = make_grad_plan(args, &plan)) return rc;
+    snprintf(buf, (size_t)buf_len, "cdist_grad kernel=%s channels=%d tiles=%dx%d chunks=%d batches=%d",
+             plan.sign ? "sign" : plan.tensor ? "weights" : "fp32", plan.ot, plan.p.tiles_m, plan.p.tiles_n, plan.p.o_chunks,
+             plan.p.L);
+    return 0;
 }
 
 extern "C" int kermac_b200_cdist_grad(const KmGradArgs* args, void* stream) {
