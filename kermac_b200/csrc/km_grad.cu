@@ -408,8 +408,8 @@ struct GradPlan {
     int ot, nt;
     bool tensor;               // channel contraction on the tensor cores (km_grad_tensor.cu)
     bool sign;                 // p = 1 with the signs as a matrix operand (km_grad_sign.cu)
-    int splits_wanted;
-    int sign_splits;           // where the sign kernel runs: how many of them it takes
+    int splits_told;           // what callers are asked scratch for: the automatic split of the kernel without signs
+    int splits;                // the automatic split of the kernel that runs, at most that
     long long partial_elems;   // elements of one dense partial result
 };
 
@@ -523,7 +523,7 @@ int make_grad_plan(const KmGradArgs* a, GradPlan* plan) {
     if ((long long)p.tiles_m * p.tiles_n > (1LL << 26)) return fail(KM_ERR_TOO_LARGE, "too many output tiles");
     if (p.o_chunks > 65535) return fail(KM_ERR_TOO_LARGE, "too many output channels");
 
-    plan->splits_wanted = preferred_split(*plan, a->norm_type, !a->p.ptr && a->p.value == 1.5f);
+    plan->splits = plan->splits_told = preferred_split(*plan, a->norm_type, !a->p.ptr && a->p.value == 1.5f);
     plan->partial_elems = (long long)p.L * p.O * p.N * p.M;
     // (its tiles and channel chunks are smaller than the ones checked above: calls that would need too many keep theirs)
     if (sign_preferred(a) && ceil_div_ll(p.M, 4) * ceil_div_ll(p.N, GS_TN) <= (1LL << 26) &&
@@ -535,7 +535,7 @@ int make_grad_plan(const KmGradArgs* a, GradPlan* plan) {
         p.tiles_m  = (int)ceil_div_ll(p.M, gs_mt_for(plan->ot));
         p.tiles_n  = (int)ceil_div_ll(p.N, GS_TN);
         p.o_chunks = (int)ceil_div_ll(p.O, plan->ot);
-        plan->sign_splits = std::min(plan->splits_wanted, preferred_split(*plan, a->norm_type, false));
+        plan->splits = std::min(plan->splits_told, preferred_split(*plan, a->norm_type, false));
     }
     return 0;
 }
@@ -547,7 +547,7 @@ extern "C" int64_t kermac_b200_cdist_grad_scratch_bytes(const KmGradArgs* args) 
     using namespace km;
     GradPlan plan;
     if (make_grad_plan(args, &plan)) return 0;
-    int splits = args->split_k > 0 ? args->split_k : plan.splits_wanted;
+    int splits = args->split_k > 0 ? args->split_k : plan.splits_told;
     if (splits <= 1) return 0;
     return (int64_t)splits * plan.partial_elems * 4;
 }
@@ -557,38 +557,24 @@ extern "C" int kermac_b200_describe_grad(const KmGradArgs* args, char* buf, int3
     if (!buf || buf_len <= 0) return fail(KM_ERR_NULL_POINTER, "buf is NULL or empty");
     GradPlan plan;
     if (int rc = make_grad_plan(args, &plan)) return rc;
-    snprintf(buf, (size_t)buf_len, "cdist_grad kernel=%s channels=%d tiles=%dx%d chunks=%d batches=%d",
+    snprintf(buf, (size_t)buf_len, "cdist_grad kernel=%s channels=%d tiles=%dx%d chunks=%d batches=%d splits=%d",
              plan.sign ? "sign" : plan.tensor ? "weights" : "fp32", plan.ot, plan.p.tiles_m, plan.p.tiles_n, plan.p.o_chunks,
-             plan.p.L);
+             plan.p.L, args->split_k > 0 ? args->split_k : plan.splits);
     return 0;
 }
 
-extern "C" int kermac_b200_cdist_grad(const KmGradArgs* args, void* stream) {
-    using namespace km;
-    GradPlan plan;
-    if (int rc = make_grad_plan(args, &plan)) return rc;
-    GradParams& p = plan.p;
-    if (p.M == 0 || p.N == 0 || p.O == 0) return 0;
-    if (int rc = require_sm100()) return rc;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
+// Launches the plan with this split; scratch holds the partial results of more than one.
+namespace km {
+namespace {
 
-    int splits = args->split_k > 0 ? args->split_k : plan.splits_wanted;
-    if (splits > 1) {
-        const int64_t need = (int64_t)splits * plan.partial_elems * 4;
-        if (!args->scratch || args->scratch_bytes < need) {
-            if (args->split_k > 1)
-                return fail(KM_ERR_BAD_SHAPE, "split_k=%d needs %lld bytes of scratch, got %lld", splits, (long long)need,
-                            (long long)(args->scratch ? args->scratch_bytes : 0));
-            splits = 1;   // automatic mode falls back to a single pass
-        }
-    }
-    if (plan.sign && args->split_k == 0) splits = std::min(splits, plan.sign_splits);
+int run_plan(const KmGradArgs* args, GradPlan& plan, int splits, void* scratch, cudaStream_t st) {
+    GradParams& p   = plan.p;
     int slabs       = (int)ceil_div_ll(p.K > 0 ? p.K : 1, G_BK);
     p.k_per_split   = (int)ceil_div_ll(slabs, splits) * G_BK;
     splits          = (int)ceil_div_ll(p.K > 0 ? p.K : 1, p.k_per_split);
     p.splits        = splits;
     if (splits > 1) {
-        p.E = static_cast<float*>(args->scratch);
+        p.E = static_cast<float*>(scratch);
         p.e_sn = p.M; p.e_so = (long long)p.N * p.M; p.e_sl = (long long)p.O * p.N * p.M;
         p.split_stride = plan.partial_elems;
         p.e_vec = aligned16(p.E) && p.M % 4 == 0;
@@ -643,6 +629,28 @@ extern "C" int kermac_b200_cdist_grad(const KmGradArgs* args, void* stream) {
         if (int rc = cuda_status(cudaGetLastError(), "launch of grad_reduce_kernel")) return rc;
     }
     return 0;
+}
+
+}  // namespace
+}  // namespace km
+
+extern "C" int kermac_b200_cdist_grad(const KmGradArgs* args, void* stream) {
+    using namespace km;
+    GradPlan plan;
+    if (int rc = make_grad_plan(args, &plan)) return rc;
+    if (plan.partial_elems == 0) return 0;
+    if (int rc = require_sm100()) return rc;
+    int splits = args->split_k > 0 ? args->split_k : plan.splits;
+    if (splits > 1) {
+        const int64_t need = (int64_t)splits * plan.partial_elems * 4;
+        if (!args->scratch || args->scratch_bytes < need) {
+            if (args->split_k > 1)
+                return fail(KM_ERR_BAD_SHAPE, "split_k=%d needs %lld bytes of scratch, got %lld", splits, (long long)need,
+                            (long long)(args->scratch ? args->scratch_bytes : 0));
+            splits = 1;   // automatic mode falls back to a single pass
+        }
+    }
+    return run_plan(args, plan, splits, args->scratch, static_cast<cudaStream_t>(stream));
 }
 
 // ---------------------------------------------------------------------------
@@ -707,34 +715,29 @@ int grad_static_scratch(float** out) {
 extern "C" int kermac_b200_cdist_grad_static(const KmGradArgs* args, void* stream) {
     using namespace km;
     if (!args) return fail(KM_ERR_NULL_POINTER, "args is NULL");
-    KmGradArgs local   = *args;
-    local.scratch      = nullptr;
-    local.scratch_bytes = 0;
     GradPlan plan;
-    if (int rc = make_grad_plan(&local, &plan)) return rc;
+    if (int rc = make_grad_plan(args, &plan)) return rc;
+    int splits = args->split_k;
     const int64_t cap      = KM_GRAD_STATIC_FLOATS * 4;
     const int64_t per_split = plan.partial_elems * 4;
-    if (local.split_k > 1) {
+    if (splits > 1) {
         // an explicit split either fits the built-in array or is refused
-        const int64_t need = (int64_t)local.split_k * per_split;
+        const int64_t need = (int64_t)splits * per_split;
         if (need > cap)
             return fail(KM_ERR_TOO_LARGE,
                         "split_k = %d needs %lld bytes of scratch but the built-in array holds %lld; pass a smaller "
                         "split_k (1 always fits), or call kermac_b200_cdist_grad with your own scratch",
-                        local.split_k, (long long)need, (long long)cap);
-    } else if (local.split_k == 0) {
+                        splits, (long long)need, (long long)cap);
+    } else if (splits == 0) {
         // automatic: the preferred split, reduced to the largest one whose partial sums fit (down to a
-        // single pass), as kermac_b200_cdist_grad does when the caller's scratch is too small
-        long long fit = per_split > 0 ? cap / per_split : plan.splits_wanted;
-        int splits    = plan.splits_wanted;
-        if (splits > fit) splits = (int)fit;
-        local.split_k = splits > 1 ? splits : 1;
+        // single pass)
+        const long long fit = per_split > 0 ? cap / per_split : plan.splits;
+        splits              = (int)std::max(1LL, std::min<long long>(plan.splits, fit));
     }
-    if (local.split_k > 1) {
-        float* ptr = nullptr;
-        if (int rc = grad_static_scratch(&ptr)) return rc;
-        local.scratch       = ptr;
-        local.scratch_bytes = cap;
-    }
-    return kermac_b200_cdist_grad(&local, stream);
+    float* scratch = nullptr;
+    if (splits > 1)
+        if (int rc = grad_static_scratch(&scratch)) return rc;
+    if (plan.partial_elems == 0) return 0;
+    if (int rc = require_sm100()) return rc;
+    return run_plan(args, plan, splits, scratch, static_cast<cudaStream_t>(stream));
 }

@@ -81,3 +81,31 @@ def test_a_full_device_takes_a_single_pass():
             kermac.cdist_grad(a, b, c, d, out=out, p=1.0, debug=debug)
         assert torch.equal(out, want)
         assert not torch.equal(kermac.cdist_grad(a, b, c, d, out=out, p=1.0, debug=debug), want)      # split again
+
+
+@pytest.mark.parametrize("O", [5, 16])
+def test_one_automatic_split_whoever_holds_the_scratch(O):
+    # The sign kernel takes fewer splits than callers are asked scratch for.  With room for its own ones, and in the
+    # library's built-in array, it sums in the same groups as in the ordinary call.
+    K, M, N = 30000, 64, 128
+    gen = torch.Generator().manual_seed(7)
+    a, b = torch.rand(K, M, generator=gen).cuda(), torch.randn(N, K, generator=gen).cuda()
+    c, d = torch.randn(O, K, generator=gen).cuda(), torch.randn(N, M, generator=gen).cuda()
+    want = kermac.cdist_grad(a, b, c, d, p=1.0)[0]
+    g = _native.KmGradArgs()
+    g.m, g.n, g.o, g.k, g.l = M, N, O, K, 1
+    g.a, g.lda, g.b, g.ldb = a.data_ptr(), M, b.data_ptr(), K
+    g.c, g.ldc, g.d, g.ldd = c.data_ptr(), K, d.data_ptr(), M
+    g.out_stride_n, g.out_stride_o, g.norm_type, g.p = M, N * M, _native.NORM_L1, _native.hyper(1.0)
+    g.out = want.data_ptr()
+    plan = dict(word.split("=") for word in _native.describe_grad(g).split()[1:])
+    need = int(plan["splits"]) * O * N * M * 4
+    assert plan["kernel"] == "sign" and int(plan["splits"]) > 1 and need < _native.lib().kermac_b200_cdist_grad_scratch_bytes(ctypes.byref(g))
+    stream = torch.cuda.current_stream().cuda_stream
+    scratch = torch.empty(need // 4, device="cuda")
+    for launch in (_native.launch_grad, _native.launch_grad_static):
+        out = torch.full((O, N, M), float("nan"), device="cuda")
+        g.out, g.scratch, g.scratch_bytes = out.data_ptr(), scratch.data_ptr(), need
+        launch(g, stream)
+        assert torch.equal(out, want)
+    assert _native.device_error_flag() == 0
