@@ -429,7 +429,7 @@ int preferred_split(const GradPlan& plan, int norm_type, bool square_root) {
     const long long sms    = sm_count();
     const double bytes     = 4.0 * p.L * p.O * p.N * p.M;
     if (blocks <= 0 || slabs <= 1) return 1;
-    double slab_us = plan.sign ? 1.0 : 2.0;
+    double slab_us = 2.0;
     if (!plan.tensor) {
         slab_us = 0.6 + 0.16 * plan.nt * (1 + plan.ot);
         if (norm_type == KM_NORM_P) slab_us += (square_root ? 0.5 : 1.4) * plan.nt;
@@ -446,32 +446,94 @@ int preferred_split(const GradPlan& plan, int norm_type, bool square_root) {
     return cheapest_split(slabs, last, cost);
 }
 
-// Whether p = 1 takes the kernel with the signs as a matrix operand (km_grad_sign.cu).  A block of it costs the same
-// for 1 to 128 rows n and a multiple of its channel tile, so the three kernels are compared by their tiles times what a
-// slab of 32 k of a tile takes on an SM, us.  Measured on B200 at K = 30000, M = 4096, N = 256, ms (the choice before
-// // in brackets): 2 channels 5.49 [FP32 4.45], 4: 5.49 [FP32 6.23], 8: 5.98 [FP32 10.6], 16: 8.87 [FP32 20.3], 32: 11.9 [weights 22.0],
-// 64: 23.8 [weights 29.5]; where b or c cannot be copied 16 bytes at a time 9.4 at 4, 17.2 at 16 and 20.5 at 32.  Few k leave a
-// block mostly waiting for its first slabs (64 x 1000 x 1000 x 16: 96 us against 56), so at least 256.
-bool sign_preferred(const KmGradArgs* a) {
-    if (a->norm_type != KM_NORM_L1 || a->k < 1 || a->contraction == KM_CONTRACT_FP32) return false;
-    if (a->contraction == KM_CONTRACT_TENSOR) return a->n >= 96;      // the other tensor-core kernel for fewer rows
-    if (a->n < 64 || a->k < 8 * G_BK) return false;
-    const bool vec = aligned16(a->b) && aligned16(a->c) && a->ldb % 4 == 0 && a->ldc % 4 == 0 && a->b_stride_l % 4 == 0 &&
-                     a->c_stride_l % 4 == 0;
-    const int ot         = gs_ot_for(a->o);
-    const double slab_us = (ot == 4 ? 0.85 : ot == 8 ? 0.92 : ot == 16 ? 0.68 : 0.92) * (vec ? 1.0 : 1.8);
-    const double sign    = slab_us * ceil_div_ll(a->m, gs_mt_for(ot)) * ceil_div_ll(a->n, GS_TN) * ceil_div_ll(a->o, ot);
-    double other;
-    if (a->o >= KM_GRAD_TENSOR_MIN_O) {
-        const int wt = gt_ot_for(a->o);
-        other = (wt == 64 ? 1.14 : 1.7) * ceil_div_ll(a->m, GT_TM) * ceil_div_ll(a->n, gt_tn_for(wt)) * ceil_div_ll(a->o, wt);
-    } else {
-        int ft = 1;
-        while (ft < a->o && ft < 16) ft *= 2;
-        const int nt = nt_for(ft);
-        other = (ft == 1 ? 2.24 : ft == 2 ? 2.74 : ft == 4 ? 3.84 : ft == 8 ? 3.27 : 3.13) * ceil_div_ll(a->m, G_TM) * ceil_div_ll(a->n, 16 * nt) * ceil_div_ll(a->o, ft);
+// What the kernels of the p = 1 gradient take, us: a slab of 32 k and the rest of a block (its set-up, first slabs, last
+// sums and stores); what rows of the result that cannot be stored 16 bytes at a time add to the latter, and rows of b or
+// c that cannot be copied 16 bytes at a time to the former (one warp of the sign kernel then copies 128 rows of b word by
+// word).  Fitted on B200 to 10558 calls (K 256 to 30000, M 9 to 4096, N 64 to 1000, O 1 to 64): 95 % of a kernel's calls
+// are within 8 to 20 % of estimated_us().
+struct P1Cost {
+    double slab, block, ragged, words;
+};
+P1Cost p1_cost(const GradPlan& plan) {
+    if (plan.sign) {
+        switch (plan.ot) {
+            case 4: return {0.84, 5.3, 0.5, 0.59};
+            case 8: return {0.91, 6.7, 1.6, 0.51};
+            case 16: return {0.68, 5.1, 1.8, 0.62};
+            default: return {0.90, 7.8, 3.3, 0.63};
+        }
     }
-    return 1.05 * sign < other;
+    if (plan.tensor) return plan.ot == 16 ? P1Cost{1.50, 3.1, 0.3, 0.0} : plan.ot == 32 ? P1Cost{1.67, 5.9, 0.3, 0.0} : P1Cost{1.17, 5.9, 0.3, 0.0};
+    const double slab = plan.ot == 1 ? 2.49 : plan.ot == 2 ? 3.05 : plan.ot == 4 ? 4.22 : plan.ot == 8 ? 3.64 : 3.51;
+    return {slab, 1.0, 2.0, 0.0};
+}
+
+// Estimated time of a p = 1 plan whose k range is cut into `s` pieces of at most `per` slabs, us.  An SM has one block of
+// a tensor-core kernel at a time, two of the FP32 kernel 10 % faster per slab than one; the sign kernel's last wave
+// overlaps a little with the others.
+double estimated_us(const GradPlan& plan, const KmGradArgs* a, long long sms, long long s, long long per) {
+    const GradParams& p    = plan.p;
+    const P1Cost cost      = p1_cost(plan);
+    const long long blocks = (long long)p.tiles_m * p.tiles_n * p.o_chunks * p.L * s;
+    const long long share  = ceil_div_ll(blocks, sms);
+    double waves = (double)share, work = (double)share, slab = cost.slab;
+    if (plan.sign) {
+        waves = work   = 0.85 * share + 0.15 * std::max(1.0, (double)blocks / sms);
+        const bool vec = aligned16(a->b) && aligned16(a->c) && a->ldb % 4 == 0 && a->ldc % 4 == 0 && a->b_stride_l % 4 == 0 &&
+                         a->c_stride_l % 4 == 0;
+        if (!vec) slab += cost.words * p.N / ((double)GS_TN * p.tiles_n);
+    } else if (!plan.tensor) {
+        work = 0.9 * share + ((share & 1) ? 0.1 : 0.0);
+    }
+    const bool stores_vec = s > 1 ? p.M % 4 == 0
+                                  : aligned16(a->out) && a->out_stride_n % 4 == 0 && a->out_stride_o % 4 == 0 &&
+                                        (p.L == 1 || a->out_stride_l % 4 == 0);
+    const double mbytes = 4e-6 * p.L * p.O * p.N * p.M;
+    // the sign kernel writes rows 16 bytes at a time, which costs more where the result does not fit L2
+    const double stores = plan.sign ? 0.2 * std::max(0.0, mbytes - 128.0) : 0.0;
+    return 3.0 + stores + work * per * slab + waves * (cost.block + (stores_vec ? 0.0 : cost.ragged)) +
+           (s > 1 ? 3.0 + 0.06 * s + 0.2 * (2 * s + 1) * mbytes : 0.0);
+}
+
+// Turns a plan for p = 1 into one for the kernel with the signs as a matrix operand (km_grad_sign.cu) where that is
+// estimated to be the faster one.  A block of it costs the same for 1 to 128 rows n, takes a multiple of its channel tile
+// and is alone on its SM, so short sums lose what many k win.  Measured on B200, us, sign kernel against the other one
+// (FP32 up to 16 channels, weights from 17 on):
+//   K      M     N     O    sign   other         K      M     N     O    sign   other
+//   256    4096  1000  4    358    224           256    1000  1000  16   150    189
+//   320    4096  1000  4    405    278           1024   1000  1000  4    225    253
+//   256    4096  128   4    53     37            1024   1000  64    32   72     62
+//   512    250   500   64   120    107           8192   1000  1000  16   2477   5565
+//   30000  4096  256   2    5490   4450          30000  4096  256   4    5490   6230
+//   30000  4096  256   32   11900  22000         8192   1000  64    4    221    129
+//   8192   1000  1000  4    2547   1726 (b and c in rows that are not 16-byte aligned; 1535 where they are)
+// Its split of k stays within the one that callers were told of (see kermac_b200_cdist_grad_scratch_bytes).
+void consider_sign(const KmGradArgs* a, GradPlan* plan) {
+    if (a->norm_type != KM_NORM_L1 || a->contraction == KM_CONTRACT_FP32 || plan->partial_elems == 0) return;
+    const bool named = a->contraction == KM_CONTRACT_TENSOR;
+    // below 256 k the automatic choice has always been the FP32 kernel
+    if (a->k < (named ? 1 : 8 * G_BK) || a->n < (named ? 96 : 64)) return;
+    GradPlan sign = *plan;
+    GradParams& p = sign.p;
+    sign.sign = sign.tensor = true;
+    sign.ot                 = gs_ot_for(a->o);
+    // (its tiles and channel chunks are smaller than those of the plan: calls that would need too many keep theirs)
+    const long long tiles_m = ceil_div_ll(p.M, gs_mt_for(sign.ot)), tiles_n = ceil_div_ll(p.N, GS_TN);
+    const long long chunks = ceil_div_ll(p.O, sign.ot), slabs = ceil_div_ll(p.K, G_BK), sms = sm_count();
+    if (tiles_m * tiles_n > (1LL << 26) || chunks > 65535) return;
+    p.tiles_m = (int)tiles_m; p.tiles_n = (int)tiles_n; p.o_chunks = (int)chunks;
+    // for 16 blocks per SM and more a further split gains nothing
+    const long long last = std::min<long long>(plan->splits_told, 16 * sms / (tiles_m * tiles_n * chunks * p.L));
+    sign.splits = cheapest_split(slabs, last, [&](long long s, long long per) { return estimated_us(sign, a, sms, s, per); });
+    auto us     = [&](const GradPlan& q) {
+        const long long per = ceil_div_ll(slabs, a->split_k > 0 ? a->split_k : q.splits);
+        return estimated_us(q, a, sms, ceil_div_ll(slabs, per), per);
+    };
+    // Callers who name the tensor cores get this kernel from 96 rows on unless the other one is estimated to be a tenth
+    // and 8 us faster, so that near ties do not follow the operands' alignment.  The automatic choice wants 3 % for the
+    // estimate's error.
+    const double with = us(sign), without = us(*plan);
+    if (named ? with <= std::max(1.1 * without, without + 8.0) : 1.03 * with < without) *plan = sign;
 }
 
 int make_grad_plan(const KmGradArgs* a, GradPlan* plan) {
@@ -525,18 +587,7 @@ int make_grad_plan(const KmGradArgs* a, GradPlan* plan) {
 
     plan->splits = plan->splits_told = preferred_split(*plan, a->norm_type, !a->p.ptr && a->p.value == 1.5f);
     plan->partial_elems = (long long)p.L * p.O * p.N * p.M;
-    // (its tiles and channel chunks are smaller than the ones checked above: calls that would need too many keep theirs)
-    if (sign_preferred(a) && ceil_div_ll(p.M, 4) * ceil_div_ll(p.N, GS_TN) <= (1LL << 26) &&
-        ceil_div_ll(p.O, gs_ot_for(a->o)) <= 65535) {
-        // its split stays within the one above, and so within the scratch that callers were told of: its blocks are no
-        // larger than the other kernels' (512 results per channel against 512 to 4096), it rarely wants more
-        plan->sign = plan->tensor = true;
-        plan->ot   = gs_ot_for(a->o);
-        p.tiles_m  = (int)ceil_div_ll(p.M, gs_mt_for(plan->ot));
-        p.tiles_n  = (int)ceil_div_ll(p.N, GS_TN);
-        p.o_chunks = (int)ceil_div_ll(p.O, plan->ot);
-        plan->splits = std::min(plan->splits_told, preferred_split(*plan, a->norm_type, false));
-    }
+    consider_sign(a, plan);
     return 0;
 }
 
