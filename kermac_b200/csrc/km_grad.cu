@@ -525,8 +525,10 @@ void consider_sign(const KmGradArgs* a, GradPlan* plan) {
     // for 16 blocks per SM and more a further split gains nothing
     const long long last = std::min<long long>(plan->splits_told, 16 * sms / (tiles_m * tiles_n * chunks * p.L));
     sign.splits = cheapest_split(slabs, last, [&](long long s, long long per) { return estimated_us(sign, a, sms, s, per); });
-    auto us     = [&](const GradPlan& q) {
-        const long long per = ceil_div_ll(slabs, a->split_k > 0 ? a->split_k : q.splits);
+    // compared with the automatic splits, also where the caller asks for others: a call that has no room for partial sums
+    // then takes the kernel of the same call with split_k = 1
+    auto us = [&](const GradPlan& q) {
+        const long long per = ceil_div_ll(slabs, q.splits);
         return estimated_us(q, a, sms, ceil_div_ll(slabs, per), per);
     };
     // Callers who name the tensor cores get this kernel from 96 rows on unless the other one is estimated to be a tenth

@@ -93,4 +93,7 @@ def test_splits_stay_within_the_scratch_that_callers_are_asked_for():
         told = max(1, _native.lib().kermac_b200_cdist_grad_scratch_bytes(g) // (4 * M * N * O))
         assert 1 <= int(plan["splits"]) <= told and (plan["kernel"] == "sign" or int(plan["splits"]) == told)
         seen.add(plan["kernel"])
+        for split_k in (1, 3):                                       # the kernel does not follow the split that is asked for
+            g.split_k = split_k
+            assert described(g) == dict(plan, splits=str(split_k))
     assert seen == {"fp32", "weights", "sign"}
