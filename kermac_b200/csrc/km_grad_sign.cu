@@ -6,7 +6,7 @@
 // For a fixed m the sum is a matrix product over k of S_m[n, k] = sign(d[n, m] - b[n, k]) and the
 // products P_m[o, k] = c[o, k] * a[k, m].  The signs are exact in bf16, so only P has to be split to
 // keep fp32 accuracy: each fp32 product becomes three bf16 pieces by truncation (8 + 8 + 8 significant
-// bits, nothing is lost), and one tcgen05.mma kind::f16 of 128 rows (n) x 3 OT columns (piece, channel)
+// bits; the second and third scaled by powers of two, so that no bit of a normal product is lost), and one tcgen05.mma kind::f16 of 128 rows (n) x 3 OT columns (piece, channel)
 // x 16 k takes all three.  The general tensor-core kernel (km_grad_tensor.cu) has the weights
 // a * g(d - b) in the A operand, split per (n, m, k); here the A operand costs a subtract, a byte
 // permute and one logic operation per two k, and the split is done once per (o, k, m), shared by the
@@ -29,8 +29,8 @@
 // The product warps have no global loads of their own: their fence to the asynchronous units waits for
 // every memory operation of the thread, and behind loads in flight it made each slab as long as a load.
 // What bounds it (B200, K = 30000, M = 4096, N = 256; ms, in brackets the kernel that took these calls before):
-// 4 channels 5.5 (6.2), 8: 6.0 (10.6), 16: 8.9 (20.3), 32: 11.9 (22.0), 64: 23.8 (29.5).  The MMAs alone would
-// take 2.5 ms at 32 channels (an MMA of 128 rows x N columns holds the tensor pipe N / 2 cycles, also with the
+// 4 channels 5.5 (6.2), 8: 6.0 (10.6), 16: 8.9 (20.3), 32: 12.1 (22.0), 64: 23.8 (29.5); scaling the pieces is
+// 0.15 of the 12.1.  The MMAs alone would take 2.5 ms at 32 channels (an MMA of 128 rows x N columns holds the tensor pipe N / 2 cycles, also with the
 // stores to tensor memory beside it), the ALU pipe (permutes and logic, half rate) about 3.5.  At 32 channels a slab of
 // 4 m takes some 1600 cycles: the product warps compute for 920 of them (their instructions issue once in four to
 // five cycles beside the generating warps) and a wait for a phase that is long complete costs 100 to 250.  On the way
@@ -258,8 +258,8 @@ grad_sign_kernel(const __grid_constant__ GradTensorParams p, const __grid_consta
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const u64 v  = mul2(c2[e], a2[e]);
-                    const u64 r  = bf16_remainder2(v);
-                    const u64 r2 = bf16_remainder2(r);
+                    const u64 r  = bf16_remainder2(v, BF16_STEP_2);
+                    const u64 r2 = bf16_remainder2(r, BF16_STEP_3);
                     p1[e]        = upper_halves(v);
                     p2[e]        = upper_halves(r);
                     p3[e]        = upper_halves(r2);
@@ -304,13 +304,13 @@ grad_sign_kernel(const __grid_constant__ GradTensorParams p, const __grid_consta
                 uint32_t r[16];
                 tc::ld_32x32b_x16(t_row + m * S::COLS, r);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) v[i] = __uint_as_float(r[i]) + (__uint_as_float(r[4 + i]) + __uint_as_float(r[8 + i]));
+                for (int i = 0; i < 4; ++i) v[i] = bf16_joined(__uint_as_float(r[i]), __uint_as_float(r[4 + i]), __uint_as_float(r[8 + i]));
             } else if constexpr (OT == 8) {
                 uint32_t r1[16], r3[8];
                 tc::ld_32x32b_x16(t_row + m * S::COLS, r1);
                 tc::ld_32x32b_x8(t_row + m * S::COLS + 16, r3);
 #pragma unroll
-                for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r1[i]) + (__uint_as_float(r1[8 + i]) + __uint_as_float(r3[i]));
+                for (int i = 0; i < 8; ++i) v[i] = bf16_joined(__uint_as_float(r1[i]), __uint_as_float(r1[8 + i]), __uint_as_float(r3[i]));
             } else {
 #pragma unroll
                 for (int o = 0; o < OT; o += 16) {
@@ -318,7 +318,7 @@ grad_sign_kernel(const __grid_constant__ GradTensorParams p, const __grid_consta
                     const uint32_t t = t_row + m * S::COLS + o;
                     tc::ld3_32x32b_x16(t, t + OT, t + 2 * OT, r1, r2, r3);
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) v[o + i] = __uint_as_float(r1[i]) + (__uint_as_float(r2[i]) + __uint_as_float(r3[i]));
+                    for (int i = 0; i < 16; ++i) v[o + i] = bf16_joined(__uint_as_float(r1[i]), __uint_as_float(r2[i]), __uint_as_float(r3[i]));
                 }
             }
             tc::fence_before_sync();

@@ -105,3 +105,18 @@ def test_the_automatic_choice_agrees_with_the_fp32_kernel(shape):
     # K terms rounded in another order
     assert float((got - want).abs().max()) <= 2.0 ** -23 * shape[0] ** 0.5 * float(want.abs().max())
     assert _native.device_error_flag() == 0
+
+
+@pytest.mark.parametrize("O", [4, 8, 16, 32])
+@pytest.mark.parametrize("shift", [0, 60, 110, 118])
+def test_small_products_keep_their_bits(O, shift):
+    # kernel values of distant points as weights: the products c * a are normal numbers down to 2^-120 here.  bf16 ends
+    # at 2^-133, so pieces that were not scaled up would be 2^-15 of such a product off.  Terms of random sign: a
+    # rounded product each and 32 truncating additions per chain stay below 2^-22 of the largest entry.
+    K, M, N = 600, 24, 128
+    a, b, c, d = inputs(K, M, N, O)
+    a, c = (a + 0.5), torch.copysign(c.abs().clamp(0.5, 2.0), c)
+    got = kermac.cdist_grad((a * 2.0 ** -shift).cuda(), b.cuda(), c.cuda(), d.cuda(), p=1.0, contraction="tensor")
+    ref = ko.cdist_grad_ref(a, b, c, d, p=1.0)
+    assert float((got.cpu().double() * 2.0 ** shift - ref).abs().max()) < 2.0 ** -22 * float(ref.abs().max())
+    assert _native.device_error_flag() == 0
