@@ -1,11 +1,15 @@
 """GPU parity of the p = 1 tensor-core form of cdist_grad (signs as a matrix operand) against the float64 CPU
-oracle.  Reached with contraction="tensor" from 96 rows n on.  Tolerance: max |x - ref| / max |ref| <= 5e-5 as for
-the other gradient kernels; where the test is about accuracy it is tighter and says why."""
+oracle.  Reached with contraction="tensor" from 96 rows n on (unless the other kernel is much faster; every call here
+checks which kernel it gets).  Tolerance: max |x - ref| / max |ref| <= 5e-5 as for the other gradient kernels; where the
+test is about accuracy it is tighter and says why."""
+import ctypes
+
 import pytest
 import torch
 
 import kermac_b200 as kermac
 from kermac_b200 import _native
+from kermac_b200.cdist_grad import _marshal_grad
 from oracle import kermac_oracle as ko
 
 pytestmark = pytest.mark.gpu
@@ -21,11 +25,43 @@ def inputs(K, M, N, O, seed=3):
     return gen((K, M), seed, "rand"), gen((N, K), seed + 1), gen((O, K), seed + 2), gen((N, M), seed + 3)
 
 
+def arguments(a, b, c, d, out, contraction="tensor", split_k=0):
+    """The C-ABI arguments of a call on 2-D or batched operands."""
+    g, _ = _marshal_grad(a, b, c, d, out, 1.0, contraction)
+    g.split_k = split_k
+    return g
+
+
+def takes_sign(g):
+    return "kernel=sign" in _native.describe_grad(g)
+
+
 def check(a, b, c, d, tol=TOL):
     got = kermac.cdist_grad(a.cuda(), b.cuda(), c.cuda(), d.cuda(), p=1.0, contraction="tensor")
+    assert takes_sign(arguments(a.cuda(), b.cuda(), c.cuda(), d.cuda(), got))
     assert ko.rel_err_signed(got, ko.cdist_grad_ref(a, b, c, d, p=1.0)) < tol
     assert _native.device_error_flag() == 0
     return got
+
+
+def with_split(a, b, c, d, split_k):
+    """The sums in `split_k` pieces of k (operands on the device)."""
+    out = torch.full((c.shape[0], b.shape[0], a.shape[1]), float("nan"), device="cuda")
+    g = arguments(a, b, c, d, out, split_k=split_k)
+    assert takes_sign(g)
+    need = _native.lib().kermac_b200_cdist_grad_scratch_bytes(ctypes.byref(g))
+    scratch = torch.full((max(1, need // 4),), float("nan"), device="cuda")
+    g.scratch, g.scratch_bytes = scratch.data_ptr(), need
+    _native.launch_grad(g, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    return out
+
+
+def unaligned(t):
+    """The same numbers in rows that are not 16-byte aligned."""
+    view = torch.zeros(t.shape[0], t.shape[1] + (3 - t.shape[1]) % 4, device="cuda")[:, :t.shape[1]]
+    view.copy_(t)
+    return view
 
 
 @pytest.mark.parametrize("O", [1, 4, 5, 8, 9, 16, 17, 32, 33, 64])
@@ -42,9 +78,25 @@ def test_columns_around_the_tiles(M, O):
 
 @pytest.mark.parametrize("K", [1, 15, 16, 17, 31, 32, 33, 127, 128, 129, 511, 512, 513, 1600])
 @pytest.mark.parametrize("O", [4, 8, 16, 32])
-def test_k_extents_around_slabs_and_chains(K, O):
-    # 32 k per slab, 512 per accumulation chain, cut at staggered slabs for the columns m of a block
+def test_k_extents_around_slabs(K, O):
+    # 32 k per slab; the automatic split leaves a block one slab to a few
     check(*inputs(K, 9, 100, O))
+
+
+@pytest.mark.parametrize("K", [511, 512, 513, 544, 1024, 1600, 5001])
+@pytest.mark.parametrize("O", [4, 8, 16, 32])
+def test_k_extents_around_chains_and_rings(K, O):
+    # a single pass: 512 k per accumulation chain, cut at staggered slabs for the columns m of a block, and every ring of
+    # barriers (4 slabs at most) goes round many times; then three pieces with a short last one
+    a, b, c, d = inputs(K, 9, 100, O)
+    ref = ko.cdist_grad_ref(a, b, c, d, p=1.0)[0]
+    a, b, c, d = a.cuda(), b.cuda(), c.cuda(), d.cuda()
+    views = unaligned(b), unaligned(c)
+    for split_k in (1, 3):
+        got = with_split(a, b, c, d, split_k)
+        assert ko.rel_err_signed(got, ref) < TOL
+        assert torch.equal(got, with_split(a, *views, d, split_k))      # staged by copies of 4 bytes
+    assert _native.device_error_flag() == 0
 
 
 @pytest.mark.parametrize("K", [36, 260, 3000])
@@ -69,6 +121,9 @@ def test_same_sign_sums_stay_at_fp32_accuracy(O):
     a, c = gen((K, M), 24, "rand"), gen((O, K), 25, "rand")
     b, d = gen((N, K), 26, "rand"), gen((N, M), 27, "rand") + 2.0
     check(a, b, c, d, 2e-6)
+    # in one pass 40 chains: their sum rounds by 2^-25 of a partial sum, half of the result on average, each time
+    got = with_split(a.cuda(), b.cuda(), c.cuda(), d.cuda(), 1)
+    assert ko.rel_err_signed(got, ko.cdist_grad_ref(a, b, c, d, p=1.0)[0]) < 2e-6 + 40 * 2.0 ** -26
 
 
 def test_batches_broadcasting_and_unaligned_output():
@@ -98,10 +153,14 @@ def test_ties_infinities_and_nan_as_in_the_fp32_kernel():
     assert float((got - want)[finite].abs().max()) < TOL * float(want[finite].abs().max())
 
 
-@pytest.mark.parametrize("shape", [(300, 33, 64, 9), (257, 500, 130, 24), (400, 64, 70, 40), (256, 31, 200, 4)])
-def test_the_automatic_choice_agrees_with_the_fp32_kernel(shape):
+@pytest.mark.parametrize("shape, sign", [
+    ((300, 33, 64, 9), False), ((257, 500, 130, 24), False), ((400, 64, 70, 40), False), ((256, 31, 200, 4), True),
+    ((1000, 1000, 128, 3), True), ((1024, 130, 100, 16), True), ((4096, 250, 128, 24), True), ((2048, 250, 128, 32), True),
+    ((1024, 130, 256, 64), True)])
+def test_the_automatic_choice_agrees_with_the_fp32_kernel(shape, sign):
     a, b, c, d = (t.cuda() for t in inputs(*shape))
     got, want = (kermac.cdist_grad(a, b, c, d, p=1.0, contraction=k) for k in ("auto", "fp32"))
+    assert takes_sign(arguments(a, b, c, d, got, "auto")) == sign
     # K terms rounded in another order
     assert float((got - want).abs().max()) <= 2.0 ** -23 * shape[0] ** 0.5 * float(want.abs().max())
     assert _native.device_error_flag() == 0
