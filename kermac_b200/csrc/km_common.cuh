@@ -91,25 +91,12 @@ __device__ __forceinline__ uint32_t upper_halves(u64 v) {
 __device__ __forceinline__ u64 bf16_remainder2(u64 v, float step) {
     return mul2(sub2(v, v & 0xFFFF0000FFFF0000ull), pack2(step, step));
 }
-// The value (or a sum of values) from its pieces (or their sums).
+// A sum of values from the sums of their pieces.  An infinite value or a NaN among them leaves NaN in the second and third
+// piece and itself in the first (as long as the NaN is the one that arithmetic makes, whose upper half is a NaN too), so
+// the first sum alone is the result where it is not finite.
 __device__ __forceinline__ float bf16_joined(float x1, float x2, float x3) {
-    return fmaf(fmaf(x3, 1.0f / BF16_STEP_3, x2), 1.0f / BF16_STEP_2, x1);
-}
-// The pieces where that goes wrong (the remainders are NaN then): an infinite value has no remainder, and every NaN
-// has to stay one.
-__device__ __forceinline__ void bf16_pieces_special(u64 v, uint32_t& w1, uint32_t& w2, uint32_t& w3) {
-    float x[2], r[2];
-    unpack2(v, x[0], x[1]);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        x[i] = x[i] == x[i] ? x[i] : __int_as_float(0x7FFFFFFF);
-        r[i] = fabsf(x[i]) == __int_as_float(0x7F800000)
-                   ? 0.0f
-                   : (x[i] - __uint_as_float(__float_as_uint(x[i]) & 0xFFFF0000u)) * BF16_STEP_2;
-    }
-    w1 = upper_halves(pack2(x[0], x[1]));
-    w2 = upper_halves(pack2(r[0], r[1]));
-    w3 = upper_halves(bf16_remainder2(pack2(r[0], r[1]), BF16_STEP_3));
+    const float sum = fmaf(fmaf(x3, 1.0f / BF16_STEP_3, x2), 1.0f / BF16_STEP_2, x1);
+    return x1 - x1 == 0.0f ? sum : x1;
 }
 
 // ---------------------------------------------------------------- exp2 on the FP32 pipe

@@ -457,10 +457,10 @@ struct P1Cost {
 P1Cost p1_cost(const GradPlan& plan) {
     if (plan.sign) {
         switch (plan.ot) {
-            case 4: return {0.84, 5.3, 0.5, 0.59};
-            case 8: return {0.91, 6.7, 1.6, 0.51};
-            case 16: return {0.68, 5.1, 1.8, 0.62};
-            default: return {0.90, 7.8, 3.3, 0.63};
+            case 4: return {0.80, 5.3, 0.5, 0.63};
+            case 8: return {0.89, 6.7, 1.6, 0.53};
+            case 16: return {0.66, 5.1, 1.8, 0.64};
+            default: return {0.87, 7.8, 3.3, 0.66};
         }
     }
     if (plan.tensor) return plan.ot == 16 ? P1Cost{1.50, 3.1, 0.3, 0.0} : plan.ot == 32 ? P1Cost{1.67, 5.9, 0.3, 0.0} : P1Cost{1.17, 5.9, 0.3, 0.0};
@@ -573,7 +573,8 @@ int make_grad_plan(const KmGradArgs* a, GradPlan* plan) {
     // products to the MMA.  Up to 16 channels the FP32 kernel is level or faster (K = 30000, M = 4096,
     // N = 256: 20.4 against 19.1 ms at 16, 20.3 when the operands cannot be staged by TMA); from 17 on
     // it needs a second pass and the tensor cores win (40.4 against 22.0 ms at 32, 80.7 against 29.6 at
-    // 64).  The tensor kernel needs at least one slab of k.
+    // 64).  The tensor kernel needs at least one slab of k.  For p = 1 consider_sign() may put a third kernel in
+    // place of the one chosen here.
     plan->tensor = a->k > 0 && (a->contraction == KM_CONTRACT_TENSOR ||
                                 (a->contraction == KM_CONTRACT_AUTO && a->o >= KM_GRAD_TENSOR_MIN_O && a->k >= 8 * G_BK));
     plan->sign = false;

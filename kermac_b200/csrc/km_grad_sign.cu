@@ -29,15 +29,16 @@
 // The product warps have no global loads of their own: their fence to the asynchronous units waits for
 // every memory operation of the thread, and behind loads in flight it made each slab as long as a load.
 // What bounds it (B200, K = 30000, M = 4096, N = 256; ms, in brackets the kernel that took these calls before):
-// 4 channels 5.5 (6.2), 8: 6.0 (10.6), 16: 8.9 (20.3), 32: 12.1 (22.0), 64: 23.8 (29.5); scaling the pieces is
-// 0.15 of the 12.1.  The MMAs alone would take 2.5 ms at 32 channels (an MMA of 128 rows x N columns holds the tensor pipe N / 2 cycles, also with the
+// 4 channels 5.25 (6.2), 8: 5.8 (10.6), 16: 8.6 (20.3), 32: 11.3 (22.0), 64: 22.6 (29.5).
+// The MMAs alone would take 2.5 ms at 32 channels (an MMA of 128 rows x N columns holds the tensor pipe N / 2 cycles, also with the
 // stores to tensor memory beside it), the ALU pipe (permutes and logic, half rate) about 3.5.  At 32 channels a slab of
 // 4 m takes some 1600 cycles: the product warps compute for 920 of them (their instructions issue once in four to
 // five cycles beside the generating warps) and a wait for a phase that is long complete costs 100 to 250.  On the way
 // here (ms at 4 / 32 channels): one thread issuing all MMAs 18.5 / -; every role handing over per 16 k by its own
 // barrier, four issuing warps 6.7 / 14.5; global loads taken from the product warps 7.0 / 14.2; eight product warps
 // and carried copy addresses 7.5 / 12.4; all MMAs of a slab in one elected block 6.2 / 11.9; 16 k of all eight m
-// per group and slab instead of four 5.5 / 11.9.
+// per group and slab instead of four 5.5 / 11.9; pieces scaled 5.5 / 12.1; infinite and NaN products left to the sums
+// (bf16_joined) instead of being looked for in each product 5.25 / 11.3.
 // Hand-over is by mbarriers, one round per slab; every wait is bounded, and a wait that runs out sets a
 // flag (kermac_b200_device_error_flag) and lets the block run to its end without its results.
 #include <cstring>
@@ -235,6 +236,7 @@ grad_sign_kernel(const __grid_constant__ GradTensorParams p, const __grid_consta
         const int kc  = lane & 3;                                   // eight k of the slab
         const int mi0 = (pw / S::OCTS) * S::MSUB + (OT >= 8 ? 0 : (lane >> 2) / OT);
         constexpr int MSTEP = (S::PROD / S::OCTS) * S::MSUB;
+        static_assert(MT % MSTEP == 0, "every product warp takes the same number of m");
         for (int s = 0; s < nslabs; ++s) {
             const int ac = s % GS_AC_SLOTS;
             wait(acfull(ac), (s / GS_AC_SLOTS) & 1);
@@ -247,14 +249,12 @@ grad_sign_kernel(const __grid_constant__ GradTensorParams p, const __grid_consta
             const ulonglong2 c1 = *reinterpret_cast<const ulonglong2*>(cs + 4);
             const u64 c2[4] = {c0.x, c0.y, c1.x, c1.y};
 #pragma unroll
-            for (int it = 0; it < (MT + MSTEP - 1) / MSTEP; ++it) {
+            for (int it = 0; it < MT / MSTEP; ++it) {
                 const int mi = mi0 + it * MSTEP;
-                if (MSTEP > MT && mi >= MT) break;
                 const ulonglong2 a0 = *reinterpret_cast<const ulonglong2*>(as + mi * GS_BK);
                 const ulonglong2 a1 = *reinterpret_cast<const ulonglong2*>(as + mi * GS_BK + 4);
                 const u64 a2[4] = {a0.x, a0.y, a1.x, a1.y};
                 uint32_t p1[4], p2[4], p3[4];
-                u64 check = 0ull;
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
                     const u64 v  = mul2(c2[e], a2[e]);
@@ -263,14 +263,6 @@ grad_sign_kernel(const __grid_constant__ GradTensorParams p, const __grid_consta
                     p1[e]        = upper_halves(v);
                     p2[e]        = upper_halves(r);
                     p3[e]        = upper_halves(r2);
-                    check        = e ? add2(check, r2) : r2;
-                }
-                float x0, x1;
-                unpack2(check, x0, x1);
-                if (!(x0 + x1 == x0 + x1)) {
-                    // an infinite or NaN product among them
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) bf16_pieces_special(mul2(c2[e], a2[e]), p1[e], p2[e], p3[e]);
                 }
                 unsigned char* dst = tiles + S::OFF_P + (slot * MT + mi) * S::P_BYTES;
 #pragma unroll

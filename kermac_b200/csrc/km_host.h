@@ -47,7 +47,7 @@ struct GradTensorParams {
     const float* D; long long ldd, d_sl;
     float*       E; long long e_sn, e_so, e_sl;   // destination (out, or scratch when split)
     KmHyper p;
-    int ot;                                         // channels per thread block: 16, 32 or 64
+    int ot;                                         // channels per thread block: 16, 32 or 64 (sign kernel: 4 to 32)
     int rg;                                         // row groups per thread block
     int tiles_m, tiles_n, o_chunks, splits;
     int k_per_split;

@@ -153,6 +153,26 @@ def test_ties_infinities_and_nan_as_in_the_fp32_kernel():
     assert float((got - want)[finite].abs().max()) < TOL * float(want[finite].abs().max())
 
 
+@pytest.mark.parametrize("O", [4, 8, 16, 32])
+def test_values_that_are_not_finite_stay_in_their_sums(O):
+    # over several chains of 512 k: infinities of one and of both signs, products that overflow, and a NaN whose payload
+    # is lost when it is cut to bf16
+    a, b, c, d = inputs(1600, 9, 100, O)
+    a[7, 2] = float("inf")
+    a[40, 3], a[900, 3] = float("inf"), float("-inf")
+    a[1100, 5], c[1, 1100] = 1e30, 1e30
+    a.view(torch.int32)[1300, 6] = 0x7F800001
+    c[O - 1, 60] = float("nan")
+    a, b, c, d = (t.cuda() for t in (a, b, c, d))
+    got = with_split(a, b, c, d, 1)
+    want = kermac.cdist_grad(a, b, c, d, p=1.0, contraction="fp32")[0]
+    finite = torch.isfinite(want)
+    assert torch.equal(torch.isfinite(got), finite) and torch.equal(torch.isnan(got), torch.isnan(want))
+    assert torch.equal(got[torch.isinf(want)], want[torch.isinf(want)])
+    assert 0 < int(finite.sum()) and float((got - want)[finite].abs().max()) < TOL * float(want[finite].abs().max())
+    assert _native.device_error_flag() == 0
+
+
 @pytest.mark.parametrize("shape, sign", [
     ((300, 33, 64, 9), False), ((257, 500, 130, 24), False), ((400, 64, 70, 40), False), ((256, 31, 200, 4), True),
     ((1000, 1000, 128, 3), True), ((1024, 130, 100, 16), True), ((4096, 250, 128, 24), True), ((2048, 250, 128, 32), True),
