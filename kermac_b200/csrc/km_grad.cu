@@ -532,10 +532,10 @@ void consider_sign(const KmGradArgs* a, GradPlan* plan) {
         return estimated_us(q, a, sms, ceil_div_ll(slabs, per), per);
     };
     // Callers who name the tensor cores get this kernel from 96 rows on unless the other one is estimated to be a tenth
-    // and 8 us faster, so that near ties do not follow the operands' alignment.  The automatic choice wants 3 % for the
+    // and 5 us faster, so that near ties do not follow the operands' alignment.  The automatic choice wants 3 % for the
     // estimate's error.
     const double with = us(sign), without = us(*plan);
-    if (named ? with <= std::max(1.1 * without, without + 8.0) : 1.03 * with < without) *plan = sign;
+    if (named ? with <= std::max(1.1 * without, without + 5.0) : 1.03 * with < without) *plan = sign;
 }
 
 int make_grad_plan(const KmGradArgs* a, GradPlan* plan) {
