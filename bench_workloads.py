@@ -269,7 +269,7 @@ def grad(args, ctx):
         "data": "synthetic",
         "config": {"workload": "cdist_grad fp32 a(K=30000,M=4096) U(0,1), b(N=256,K) c(O=4,K) d(N,M) N(0,1) seed 3",
                    "l2": "a 256 MB write between steps flushes the L2; its time is subtracted"},
-        "clocks": clocks.summary(), "gpu_launches": 2 * args.steps,
+        "clocks": clocks.summary(), "gpu_launches": args.steps,      # p = 1: one pass over k, nothing to reduce
         "p=1.5": {"ms_per_step": ms15, "value": ops / (ms15 * 1e-3),
                   "roofline": {"bound": "mufu", "achieved": triples / (ms15 * 1e-3) / 1e12, "peak": pipes.mufu / 1e12,
                                "unit": "T MUFU-op/s", "frac": triples / (ms15 * 1e-3) / pipes.mufu,
@@ -281,20 +281,29 @@ def grad(args, ctx):
                                "unit": "T MUFU-op/s", "frac": 1.75 * triples / (ms17 * 1e-3) / pipes.mufu,
                                "note": "general p: lg2 and ex2 per (m, n, k); one pair in four takes its ex2 on the FP32 "
                                        "pipe, so 1.75 MUFU operations per (m, n, k)", "traffic": None}},
-        # sub + O fma lane-operations per (m, n, k); the sign flip is a bit operation on the ALU pipe
-        "roofline": _fp32_roofline((1.0 + O) * triples, ms1 * 1e-3, pipes, "1 + O lane-operations per (m, n, k) for p = 1"),
+        # The automatic choice here is the kernel with the signs as a matrix operand.  Its ALU work: a byte permute and a
+        # logic operation per two signs, and per two products c * a, which 128 rows share, four and three to split them.
+        "roofline": {"bound": "alu", "achieved": (1.0 + 3.5 * O / 128.0) * triples / (ms1 * 1e-3) / 1e12,
+                     "peak": pipes.lane / 2.0 / 1e12, "unit": "T ALU lane-op/s",
+                     "frac": (1.0 + 3.5 * O / 128.0) * triples / (ms1 * 1e-3) / (pipes.lane / 2.0), "traffic": None,
+                     "peak_source": "half the FP32 lane rate measured on this device (fma.rn.f32x2 chains)",
+                     "note": "p = 1: signs of d - b in bf16, products c * a in three bf16 pieces, tcgen05 kind::f16"},
     }
-    # what the k step's instruction mix sustains from registers alone (no loads, staging or barriers):
-    # its packed FMAs read three different register pairs and do not issue at the packed rate
+    # The FP32 kernel on the same problem: sub + O fma lane-operations per (m, n, k); the sign flip is a bit operation
+    # on the ALU pipe.  Beside it what its k step sustains from registers alone (no loads, staging or barriers): its
+    # packed FMAs read three different register pairs and do not issue at the packed rate.
+    few = max(2, args.steps // 3)
+    ms_fp32 = _timed(run(lambda: kermac.cdist_grad(ad, bd, cd, dd, out=out, p=1.0, contraction="fp32")), few, 1,
+                     ctx.barrier) - t_flush
     step_packed = _native.measure_pipe(6, 2048)[0]
     step_scalar = _native.measure_pipe(7, 2048)[0]
-    line["roofline"]["inner_step_ceiling_lane_ops"] = step_packed
-    line["roofline"]["frac_of_inner_step_ceiling"] = (1.0 + O) * triples / (ms1 * 1e-3) / step_packed
-    line["roofline"]["inner_step_ceiling_scalar_fma_lane_ops"] = step_scalar
-    # (these two are ceilings of the FP32 kernel; the automatic choice for p = 1 and many rows is the sign kernel)
+    fp32 = _fp32_roofline((1.0 + O) * triples, ms_fp32 * 1e-3, pipes, "1 + O lane-operations per (m, n, k) for p = 1")
+    fp32["inner_step_ceiling_lane_ops"] = step_packed
+    fp32["frac_of_inner_step_ceiling"] = (1.0 + O) * triples / (ms_fp32 * 1e-3) / step_packed
+    fp32["inner_step_ceiling_scalar_fma_lane_ops"] = step_scalar
+    line["fp32_kernel"] = {"ms_per_step": ms_fp32, "roofline": fp32}
     # 32 and 64 channels: the tensor-core form for p = 1 (the signs as the matrix operand) next to the FP32 kernel.
     # Its tensor-pipe bound: one bf16 MMA of 128 rows x 96 columns (three pieces of 32 channels) x 16 k per 128 n and m.
-    few = max(2, args.steps // 3)
     mma_rates = [_native.measure_pipe(kind, 4096)[0] for kind in (8, 9, 10, 11)]   # 128 x {32, 64, 128, 256} x 8
     for O2 in (32, 64):
         c2 = torch.randn(O2, K, generator=g).cuda()

@@ -161,12 +161,15 @@ int64_t kermac_b200_build_tile_count(const KmBuildArgs* args);
  * products with c run: KM_CONTRACT_FP32 as packed FP32 FMAs; KM_CONTRACT_TENSOR on the tcgen05
  * tensor cores, up to 64 channels at a time, as three tf32 products per term (weights and
  * coefficients split into a tf32 head and an fp32 remainder, accumulation chains of 128 k added up
- * in fp32: fp32-level accuracy, not the FP32 kernel's bits).  For KM_NORM_L1 and 96 or more rows n the
- * signs themselves are the matrix operand and the products c * a are split, into three bf16 pieces that lose
- * nothing.  KM_CONTRACT_AUTO takes the tensor cores from 17 channels and 256 k on, and for KM_NORM_L1 from 64
- * rows and 256 k on wherever that is estimated to be the faster form (3 channels on, for many rows).  The weights
- * a * g(d - b) are computed in FP32 either way.  A bounded wait inside a tensor-core kernel that runs out raises
- * kermac_b200_device_error_flag().
+ * in fp32: fp32-level accuracy, not the FP32 kernel's bits); the weights a * g(d - b) are computed in FP32 there
+ * and in the FP32 kernel.  For KM_NORM_L1 and 96 or more rows n KM_CONTRACT_TENSOR takes a third kernel unless that is
+ * estimated to be a tenth and 5 us slower: the signs themselves are the matrix operand, no weights are formed, and the
+ * fp32 products c * a are split into three scaled bf16 pieces, which keeps every bit of a product that is a normal
+ * number.  KM_CONTRACT_AUTO takes the tensor cores from 17 channels and 256 k on, and for KM_NORM_L1, 64 or more rows
+ * and 256 or more k the third kernel wherever that is estimated to be the fastest one (long sums over many rows, from 3
+ * channels on).  For KM_NORM_L1 the kernel, and with it the last bits of the result, therefore depends on all extents
+ * and on whether b, c and out lie in 16-byte aligned rows, not on split_k or scratch.  A bounded wait inside a
+ * tensor-core kernel that runs out raises kermac_b200_device_error_flag().
  */
 typedef struct KmGradArgs {
     int32_t m, n, o, k, l;

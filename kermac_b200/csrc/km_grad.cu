@@ -500,13 +500,13 @@ double estimated_us(const GradPlan& plan, const KmGradArgs* a, long long sms, lo
 // and is alone on its SM, so short sums lose what many k win.  Measured on B200, us, sign kernel against the other one
 // (FP32 up to 16 channels, weights from 17 on):
 //   K      M     N     O    sign   other         K      M     N     O    sign   other
-//   256    4096  1000  4    358    224           256    1000  1000  16   150    189
-//   320    4096  1000  4    405    278           1024   1000  1000  4    225    253
-//   256    4096  128   4    53     37            1024   1000  64    32   72     62
-//   512    250   500   64   120    107           8192   1000  1000  16   2477   5565
-//   30000  4096  256   2    5490   4450          30000  4096  256   4    5490   6230
-//   30000  4096  256   32   11900  22000         8192   1000  64    4    221    129
-//   8192   1000  1000  4    2547   1726 (b and c in rows that are not 16-byte aligned; 1535 where they are)
+//   256    4096  1000  4    353    224           256    1000  1000  16   150    189
+//   320    4096  1000  4    396    277           1024   1000  1000  4    216    253
+//   256    4096  128   4    52     37            1024   1000  64    32   72     62
+//   512    250   500   64   117    108           8192   1000  1000  16   2377   5577
+//   30000  4096  256   2    5250   4460          30000  4096  256   4    5250   6240
+//   30000  4096  256   32   11310  22000         8192   1000  64    4    212    129
+//   8192   1000  1000  4    2506   1727 (b and c in rows that are not 16-byte aligned; 1457 where they are)
 // Its split of k stays within the one that callers were told of (see kermac_b200_cdist_grad_scratch_bytes).
 void consider_sign(const KmGradArgs* a, GradPlan* plan) {
     if (a->norm_type != KM_NORM_L1 || a->contraction == KM_CONTRACT_FP32 || plan->partial_elems == 0) return;

@@ -30,8 +30,8 @@
 // every memory operation of the thread, and behind loads in flight it made each slab as long as a load.
 // What bounds it (B200, K = 30000, M = 4096, N = 256; ms, in brackets the kernel that took these calls before):
 // 4 channels 5.25 (6.2), 8: 5.8 (10.6), 16: 8.6 (20.3), 32: 11.3 (22.0), 64: 22.6 (29.5).
-// The MMAs alone would take 2.5 ms at 32 channels (an MMA of 128 rows x N columns holds the tensor pipe N / 2 cycles, also with the
-// stores to tensor memory beside it), the ALU pipe (permutes and logic, half rate) about 3.5.  At 32 channels a slab of
+// The MMAs alone would take 2.5 ms at 32 channels (an MMA of 128 rows x N columns holds the tensor pipe N / 2 cycles,
+// also with the stores to tensor memory beside it), the ALU pipe (permutes and logic, half rate) about 3.5.  At 32 channels a slab of
 // 4 m takes some 1600 cycles: the product warps compute for 920 of them (their instructions issue once in four to
 // five cycles beside the generating warps) and a wait for a phase that is long complete costs 100 to 250.  On the way
 // here (ms at 4 / 32 channels): one thread issuing all MMAs 18.5 / -; every role handing over per 16 k by its own

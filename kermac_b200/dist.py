@@ -391,9 +391,11 @@ def cdist_grad_sharded(a: torch.Tensor, b: torch.Tensor, c: torch.Tensor, d: tor
     else this rank's (O, rows_r, M) slab.  `compute(a, b_rows, c, d_rows, out=...)` defaults to
     `kermac_b200.cdist_grad`.
 
-    Bit-identical to the single-GPU result while the launcher keeps the whole k range in one thread
-    block; once it splits k (few output tiles, long K) the split follows the number of thread
-    blocks, which sharding changes, and the results agree to rounding only.
+    Bit-identical to the single-GPU result while the launcher takes the same kernel for a shard as for
+    the whole and keeps the whole k range in one thread block.  Once it splits k (few output tiles,
+    long K) the split follows the number of thread blocks, and for p = 1 with 256 or more k the fastest
+    kernel depends on the rows that a call has (a kernel for 128 rows at a time is no gain for a shard
+    of 32): sharding changes both, and the results then agree to rounding only.
     """
     if a.dim() != 2 or b.dim() != 2 or c.dim() != 2 or d.dim() != 2:
         raise ValueError("cdist_grad_sharded takes 2-D a, b, c and d")

@@ -153,7 +153,8 @@ def test_split_k_through_the_c_abi(O):
 
 
 def test_automatic_choice_and_run_to_run_identity():
-    # more than 16 channels and 256 k or more: the tensor cores; otherwise the FP32 kernel
+    # more than 16 channels and 256 k or more: the tensor cores; otherwise the FP32 kernel (fewer than 64 rows: for
+    # more of them p = 1 has a third kernel, tests/test_grad_sign_gpu.py)
     K, M, N = 600, 100, 50
     a, b, d = gen((K, M), 32, "rand").cuda(), gen((N, K), 33).cuda(), gen((N, M), 34).cuda()
     for O, expect in ((16, "fp32"), (17, "tensor"), (40, "tensor")):
