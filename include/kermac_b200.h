@@ -168,7 +168,7 @@ int64_t kermac_b200_build_tile_count(const KmBuildArgs* args);
  * number.  KM_CONTRACT_AUTO takes the tensor cores from 17 channels and 256 k on, and for KM_NORM_L1, 64 or more rows
  * and 256 or more k the third kernel wherever that is estimated to be the fastest one (long sums over many rows, from 3
  * channels on).  For KM_NORM_L1 the kernel, and with it the last bits of the result, therefore depends on all extents
- * and on whether b, c and out lie in 16-byte aligned rows, not on split_k or scratch.  A bounded wait inside a
+ * and on whether b and c lie in 16-byte aligned rows, not on out, split_k or scratch.  A bounded wait inside a
  * tensor-core kernel that runs out raises kermac_b200_device_error_flag().
  */
 typedef struct KmGradArgs {

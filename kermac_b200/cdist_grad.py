@@ -144,7 +144,7 @@ def cdist_grad(
     packed FP32 FMAs, "tensor" on the tcgen05 tensor cores (every factor split so that
     fp32-level accuracy is kept), "auto" the tensor cores from 17 channels and 256 k on, and for p = 1
     wherever they are estimated to be faster (long sums over many rows n from 3 channels on).  For p = 1
-    the kernel, and so the last bits, depends on the sizes and on whether rows are 16-byte aligned.  The
+    the kernel, and so the last bits, depends on the sizes and on whether rows of b and c are 16-byte aligned.  The
     tensor-core kernels bound their waits; one that runs out is reported by
     `kermac_b200._native.device_error_flag()`.
 

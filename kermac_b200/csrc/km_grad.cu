@@ -485,9 +485,8 @@ double estimated_us(const GradPlan& plan, const KmGradArgs* a, long long sms, lo
     } else if (!plan.tensor) {
         work = 0.9 * share + ((share & 1) ? 0.1 : 0.0);
     }
-    const bool stores_vec = s > 1 ? p.M % 4 == 0
-                                  : aligned16(a->out) && a->out_stride_n % 4 == 0 && a->out_stride_o % 4 == 0 &&
-                                        (p.L == 1 || a->out_stride_l % 4 == 0);
+    // (dense rows assumed: which memory the result goes to has no say in how it is computed)
+    const bool stores_vec = p.M % 4 == 0;
     const double mbytes = 4e-6 * p.L * p.O * p.N * p.M;
     // the sign kernel writes rows 16 bytes at a time, which costs more where the result does not fit L2
     const double stores = plan.sign ? 0.2 * std::max(0.0, mbytes - 128.0) : 0.0;

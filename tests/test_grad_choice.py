@@ -96,4 +96,6 @@ def test_splits_stay_within_the_scratch_that_callers_are_asked_for():
         for split_k in (1, 3):                                       # the kernel does not follow the split that is asked for
             g.split_k = split_k
             assert described(g) == dict(plan, splits=str(split_k))
+        g.split_k, g.out, g.out_stride_n, g.out_stride_o = 0, 0x1004, M + 1, N * (M + 1)     # nor where the result goes
+        assert described(g) == plan
     assert seen == {"fp32", "weights", "sign"}
