@@ -537,7 +537,8 @@ void consider_sign(const KmGradArgs* a, GradPlan* plan) {
     if (named ? with <= std::max(1.1 * without, without + 5.0) : 1.03 * with < without) *plan = sign;
 }
 
-int make_grad_plan(const KmGradArgs* a, GradPlan* plan) {
+// (splits_told does not depend on the sign kernel: without `any_kernel` the plan is done before that is looked at)
+int make_grad_plan(const KmGradArgs* a, GradPlan* plan, bool any_kernel = true) {
     if (!a) return fail(KM_ERR_NULL_POINTER, "args is NULL");
     if (a->m < 0 || a->n < 0 || a->o < 0 || a->k < 0 || a->l < 1)
         return fail(KM_ERR_BAD_SHAPE, "bad extents m=%d n=%d o=%d k=%d l=%d", a->m, a->n, a->o, a->k, a->l);
@@ -589,7 +590,7 @@ int make_grad_plan(const KmGradArgs* a, GradPlan* plan) {
 
     plan->splits = plan->splits_told = preferred_split(*plan, a->norm_type, !a->p.ptr && a->p.value == 1.5f);
     plan->partial_elems = (long long)p.L * p.O * p.N * p.M;
-    consider_sign(a, plan);
+    if (any_kernel) consider_sign(a, plan);
     return 0;
 }
 
@@ -599,7 +600,7 @@ int make_grad_plan(const KmGradArgs* a, GradPlan* plan) {
 extern "C" int64_t kermac_b200_cdist_grad_scratch_bytes(const KmGradArgs* args) {
     using namespace km;
     GradPlan plan;
-    if (make_grad_plan(args, &plan)) return 0;
+    if (make_grad_plan(args, &plan, false)) return 0;
     int splits = args->split_k > 0 ? args->split_k : plan.splits_told;
     if (splits <= 1) return 0;
     return (int64_t)splits * plan.partial_elems * 4;
