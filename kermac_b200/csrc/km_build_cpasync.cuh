@@ -172,7 +172,8 @@ __global__ void __launch_bounds__(CPA_THREADS, 2) build_cpasync_kernel(const __g
     const int K     = p.K;
     const int ktiles = (K + CPA_BK - 1) / CPA_BK;
 
-    const float p_inner = (INNER == IN_DIFF_POW || INNER == IN_DOT_POW) ? read_hyper(p.p_inner, l) : 0.0f;
+    constexpr bool POW  = INNER == IN_DIFF_POW || INNER == IN_DOT_POW || INNER == IN_DIFF_POW_TABLE;
+    const float p_inner = POW ? read_hyper(p.p_inner, l) : 0.0f;
 
     // thread -> sub-block of the tile
     const int lm = lane & 7, ln = lane >> 3;
@@ -196,6 +197,16 @@ __global__ void __launch_bounds__(CPA_THREADS, 2) build_cpasync_kernel(const __g
         cp_async_commit();
     }
 
+    PowTable table;
+    if constexpr (INNER == IN_DIFF_POW_TABLE) {
+        // (the first barrier of the k loop publishes it)
+        __shared__ float s_pow[POW_ENTRIES];
+        fill_pow_table(s_pow, p.pow, p_inner, tid, CPA_THREADS);
+        table.base = smem_u32(s_pow);
+#pragma unroll
+        for (int i = 0; i <= POW_DEGREE; ++i) table.c[i] = pack2(p.pow.c[i], p.pow.c[i]);
+    }
+
     for (int kt = 0; kt < ktiles; ++kt) {
         cp_async_wait<CPA_STAGES - 2>();
         __syncthreads();
@@ -210,7 +221,7 @@ __global__ void __launch_bounds__(CPA_THREADS, 2) build_cpasync_kernel(const __g
         }
         const float* sa = smem + (kt % CPA_STAGES) * CPA_STAGE_FLOATS + tm_off;
         const float* sb = smem + (kt % CPA_STAGES) * CPA_STAGE_FLOATS + CPA_BK * CPA_PITCH + tn_off;
-        consume_slab<INNER, CPA_BK, CPA_PITCH>(acc, sa, sb, K - kt * CPA_BK, p_inner, p.sgn);
+        consume_slab<INNER, CPA_BK, CPA_PITCH>(acc, sa, sb, K - kt * CPA_BK, p_inner, p.sgn, table);
     }
     cp_async_wait<0>();
 

@@ -22,6 +22,8 @@ BuildKernelFn cpasync_kernel_diff(int inner, bool avec, bool bvec, bool symmetri
         case IN_DIFF_ABS: return symmetric ? pick_symmetric<IN_DIFF_ABS>(avec && bvec) : pick<IN_DIFF_ABS>(avec, bvec);
         case IN_DIFF_SQUARE: return symmetric ? pick_symmetric<IN_DIFF_SQUARE>(avec && bvec) : pick<IN_DIFF_SQUARE>(avec, bvec);
         case IN_DIFF_POW: return symmetric ? pick_symmetric<IN_DIFF_POW>(avec && bvec) : pick<IN_DIFF_POW>(avec, bvec);
+        case IN_DIFF_POW_TABLE:
+            return symmetric ? pick_symmetric<IN_DIFF_POW_TABLE>(avec && bvec) : pick<IN_DIFF_POW_TABLE>(avec, bvec);
         case IN_DIFF_NOOP: return symmetric ? nullptr : pick<IN_DIFF_NOOP>(avec, bvec);
         case IN_DIFF_SQRT: return symmetric ? nullptr : pick<IN_DIFF_SQRT>(avec, bvec);
     }

@@ -2,6 +2,7 @@
 // variant choice and launch.  Host-side counterpart of the second half of the
 // reference's run_kernel (src/kermac/build_a_kernel.py:237-392).
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 
 #include "km_build_cpasync_table.cuh"
@@ -26,6 +27,52 @@ bool layout_ok(long long rows, long long cols, long long s_row, long long s_col)
     if (s_col == 1 && s_row >= cols) return true;
     if (s_row == 1 && s_col >= rows) return true;
     return false;
+}
+
+// What takes the values of a function of f at the N Chebyshev nodes of [-0.5, 0.5] to the coefficients of the polynomial
+// through them.
+struct Interpolation {
+    static constexpr int N = POW_DEGREE + 1;
+    double node[N], coef[N][N];
+    Interpolation() {
+        std::memset(coef, 0, sizeof(coef));
+        for (int j = 0; j < N; ++j) node[j] = 0.5 * std::cos(M_PI * (j + 0.5) / N);
+        double t_prev[N] = {1.0}, t_now[N] = {0.0, 1.0};                         // T_0 and T_1 by powers of 2 f
+        for (int k = 0; k < N; ++k) {
+            const double* t = k ? t_now : t_prev;
+            for (int i = 0; i < N; ++i)
+                for (int j = 0; j < N; ++j)
+                    coef[i][j] += std::ldexp(t[i], i) * (k ? 2.0 : 1.0) / N * std::cos(M_PI * k * (j + 0.5) / N);
+            if (k == 0) continue;
+            for (int i = N - 1; i >= 0; --i) {                                   // T_{k+1} = 2 x T_k - T_{k-1}
+                const double next = (i ? 2.0 * t_now[i - 1] : 0.0) - t_prev[i];
+                t_prev[i] = t_now[i];
+                t_now[i]  = next;
+            }
+        }
+    }
+};
+
+// The table route's coefficients for |x|^exponent: m^exponent on [1, 2) through the Chebyshev nodes.  Exponents outside
+// the range, or whose polynomial has no sign where the topmost exponent bits need one, keep the MUFU route.
+PowCoefs pow_coefs(float exponent) {
+    static const Interpolation through;
+    PowCoefs pc;
+    std::memset(&pc, 0, sizeof(pc));
+    if (!(exponent >= POW_MIN && exponent <= POW_MAX)) return pc;
+    double value[Interpolation::N];
+    for (int j = 0; j < Interpolation::N; ++j) value[j] = std::pow(1.5 + through.node[j], (double)exponent);
+    for (int i = 0; i < Interpolation::N; ++i) {
+        double sum = 0.0;
+        for (int j = 0; j < Interpolation::N; ++j) sum += through.coef[i][j] * value[j];
+        pc.c[i] = (float)sum;
+    }
+    float at_zero = pc.c[POW_DEGREE];                                            // f = -1.5, as the kernel computes it
+    for (int i = POW_DEGREE - 1; i >= 0; --i) at_zero = std::fmaf(at_zero, -1.5f, pc.c[i]);
+    pc.use  = at_zero != 0.0f && pc.c[POW_DEGREE] != 0.0f;
+    pc.t254 = std::copysign(INFINITY, at_zero);
+    pc.t255 = std::copysign(1.0f, pc.c[POW_DEGREE]);
+    return pc;
 }
 
 struct BuildPlan {
@@ -165,6 +212,7 @@ int make_plan(const KmBuildArgs* a, BuildPlan* plan) {
     p.outer_power    = a->outer_power;
     p.kernel_type    = a->kernel_type;
     p.p_inner        = a->p_inner;
+    if (p.inner_id == IN_DIFF_POW && !p.p_inner.ptr) p.pow = pow_coefs(p.p_inner.value);
     p.p_outer        = a->p_outer;
     p.bandwidth      = a->bandwidth;
     p.regularization = a->regularization;
@@ -272,7 +320,7 @@ KmBuildArgs packed_arguments(const KmBuildArgs& args, const BuildPlan& plan, Pac
     return packed;
 }
 
-const char* const kInnerNames[IN_COUNT] = {"diff_abs", "diff_square", "diff_pow", "diff_noop", "diff_sqrt",
+const char* const kInnerNames[IN_COUNT] = {"diff_abs", "diff_square", "diff_pow", "diff_noop", "diff_sqrt", "diff_pow",
                                            "dot_noop", "dot_abs",     "dot_square", "dot_sqrt", "dot_pow"};
 
 }  // namespace
@@ -286,7 +334,7 @@ int launch_plan(const BuildPlan& plan, cudaStream_t st) {
     if (plan.small) return launch_build_small(p, plan.variant == KM_VARIANT_TMA, st);
     if (plan.variant == KM_VARIANT_TMA) return launch_build_tma(p, st);
 
-    BuildKernelFn fn = cpasync_kernel(p.inner_id, plan.avec, plan.bvec, p.symmetric != 0);
+    BuildKernelFn fn = cpasync_kernel(kernel_inner(p), plan.avec, plan.bvec, p.symmetric != 0);
     if (!fn) return fail(KM_ERR_INTERNAL, "no kernel for inner id %d", p.inner_id);
     if (int rc = cuda_status(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, BUILD_CPA_SMEM_BYTES),
                              "cudaFuncSetAttribute(build_cpasync_kernel)"))
@@ -367,10 +415,11 @@ extern "C" int kermac_b200_describe_variant(const KmBuildArgs* args, char* buf, 
     auto name  = [](const BuildPlan& q) { return q.variant == KM_VARIANT_TMA ? "tma" : "cpasync"; };
     int length = snprintf(buf, (size_t)buf_len,
              "build_kernel variant=%s inner=%s outer_power=%d kernel_type=%d exchanged=%d a_vec16=%d b_vec16=%d "
-             "out_vec16=%d tiles=%dx%d batches=%d symmetric=%d tile_range=%d+%d kernel_tile=%d",
+             "out_vec16=%d tiles=%dx%d batches=%d symmetric=%d tile_range=%d+%d kernel_tile=%d%s",
              name(plan), kInnerNames[p.inner_id], p.outer_power, p.kernel_type,
              plan.swapped ? 1 : 0, plan.avec ? 1 : 0, plan.bvec ? 1 : 0, p.c_vec4, p.tiles_m, p.tiles_n, p.L, p.symmetric,
-             p.tile_first, p.tile_count, plan.small ? 64 : BUILD_TILE);
+             p.tile_first, p.tile_count, plan.small ? 64 : BUILD_TILE,
+             plan.variant != KM_VARIANT_TMA && kernel_inner(p) == IN_DIFF_POW_TABLE ? " pow=table" : "");
     // what kermac_b200_build_kernel_scratch does with as much scratch as it asks for (any aligned address stands for it)
     PackPlan pack;
     plan_pack_operands(plan, &pack);

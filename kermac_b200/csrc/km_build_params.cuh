@@ -26,6 +26,7 @@ struct BuildParams {
     float*       C; long long c_ld, c_sl;   // C[l][n][m] = C[l * c_sl + n * c_ld + m]
     int inner_id, outer_power, kernel_type;
     KmHyper p_inner, p_outer, bandwidth, regularization;
+    PowCoefs pow;                   // |.|^p steps with p by value
     int   reg_off_m, reg_off_n;     // diagonal rule in kernel coordinates: reg_off_m + m == reg_off_n + n
     float epsilon;
     float sgn;                      // -1 when A and B were exchanged, else +1
@@ -38,6 +39,11 @@ struct BuildParams {
     int   symmetric;                // A and B are the same matrix and the chain is symmetric in (m, n):
                                     // tiles with tile_n < tile_m are skipped, the others also write their mirror image
 };
+
+// The inner step of the kernel that runs.
+inline int kernel_inner(const BuildParams& p) {
+    return p.inner_id == IN_DIFF_POW && p.pow.use ? IN_DIFF_POW_TABLE : p.inner_id;
+}
 
 // Maps a linear tile index to (tile_m, tile_n) so that thread blocks that run at
 // the same time cover a compact patch of the output and share A and B tiles in L2.

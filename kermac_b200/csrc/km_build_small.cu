@@ -43,7 +43,9 @@ constexpr int SB_PITCH   = SB_TILE + 4;     // floats per staged k row without T
 // Resident blocks per SM the inner steps are compiled for.  Measured with 4 / 5 / 6 / 7 blocks (128 / 102 /
 // 85 / 73 registers): |.| 4000 x 4000 x 512 569 / 572 / 623 / 626 us and |.|^1.3 2048 x 2048 x 64 107 / 109 /
 // 115 / 116 us want the registers; the square is level (16384 x 16384 x 512 8247 / 8246 / 8178 / 8227 us).
-constexpr int small_min_blocks(int inner) { return (inner == IN_DIFF_ABS || inner == IN_DIFF_POW) ? 4 : 6; }
+constexpr int small_min_blocks(int inner) {
+    return (inner == IN_DIFF_ABS || inner == IN_DIFF_POW || inner == IN_DIFF_POW_TABLE) ? 4 : 6;
+}
 
 __device__ int g_small_wait_expired = 0;
 
@@ -266,7 +268,7 @@ build_small_kernel(const __grid_constant__ SmallParams sp, const __grid_constant
     if (m0 >= p.M || n0 >= p.N) return;
     const int K  = p.K;
     const int ktiles = (K + SB_BK - 1) / SB_BK;
-    const float p_inner = (INNER == IN_DIFF_POW) ? read_hyper(p.p_inner, l) : 0.0f;
+    const float p_inner = (INNER == IN_DIFF_POW || INNER == IN_DIFF_POW_TABLE) ? read_hyper(p.p_inner, l) : 0.0f;
 
     const int tm_off = (warp & 1) * 32 + (lane & 7) * 4;
     const int tn_off = (warp >> 1) * 32 + (lane >> 3) * 4;   // + {0, 16}
@@ -338,6 +340,15 @@ build_small_kernel(const __grid_constant__ SmallParams sp, const __grid_constant
         la.start(smem, 0);
         lb.start(smem + SB_BK * PITCH, 0);
         cp_async_commit();
+        PowTable table;
+        if constexpr (INNER == IN_DIFF_POW_TABLE) {
+            // (the first barrier of the k loop publishes it)
+            __shared__ float s_pow[POW_ENTRIES];
+            fill_pow_table(s_pow, p.pow, p_inner, tid, SB_THREADS);
+            table.base = smem_u32(s_pow);
+#pragma unroll
+            for (int i = 0; i <= POW_DEGREE; ++i) table.c[i] = pack2(p.pow.c[i], p.pow.c[i]);
+        }
         la.finish(smem);
         lb.finish(smem + SB_BK * PITCH);
         for (int kt = 0; kt < ktiles; ++kt) {
@@ -351,7 +362,7 @@ build_small_kernel(const __grid_constant__ SmallParams sp, const __grid_constant
                 lb.start(next + SB_BK * PITCH, kt + 1);
             }
             cp_async_commit();
-            consume_slab<INNER, SB_BK, PITCH>(acc, cur + tm_off, cur + SB_BK * PITCH + tn_off, K - kt * SB_BK, p_inner, 1.0f);
+            consume_slab<INNER, SB_BK, PITCH>(acc, cur + tm_off, cur + SB_BK * PITCH + tn_off, K - kt * SB_BK, p_inner, 1.0f, table);
             if (more) {
                 la.finish(next);
                 lb.finish(next + SB_BK * PITCH);
@@ -378,6 +389,7 @@ SmallKernelFn small_kernel(int inner, bool tma, bool symmetric) {
         case IN_DIFF_ABS: return pick<IN_DIFF_ABS>(tma, symmetric);
         case IN_DIFF_SQUARE: return pick<IN_DIFF_SQUARE>(tma, symmetric);
         case IN_DIFF_POW: return pick<IN_DIFF_POW>(tma, symmetric);
+        case IN_DIFF_POW_TABLE: return pick<IN_DIFF_POW_TABLE>(tma, symmetric);
         case IN_DOT_NOOP: return pick<IN_DOT_NOOP>(tma, symmetric);
     }
     return nullptr;
@@ -410,7 +422,7 @@ bool small_supported(const BuildParams& p) {
 }
 
 int launch_build_small(const BuildParams& p, bool tma, cudaStream_t stream) {
-    SmallKernelFn fn = small_kernel(p.inner_id, tma, p.symmetric != 0);
+    SmallKernelFn fn = small_kernel(kernel_inner(p), tma, p.symmetric != 0);
     if (!fn) return fail(KM_ERR_INTERNAL, "no 64 x 64 kernel for inner id %d", p.inner_id);
     SmallParams sp;
     sp.b       = p;

@@ -145,6 +145,51 @@ __device__ __forceinline__ void ex2_poly2(float x0, float x1, u64& r, u64& scale
     scale = pack2(__int_as_float(__float_as_int(t0) << 23), __int_as_float(__float_as_int(t1) << 23));
 }
 
+// ---------------------------------------------------------------- |x|^p without MUFU
+// With x = +-2^(e - 127) m, m in [1, 2), |x|^p is 2^((e - 127) p), looked up in shared memory by the sign and exponent
+// bits of x (a thread's lanes mostly share a few exponents, so the loads hardly collide), times m^p, a polynomial of
+// degree POW_DEGREE in f = m - 1.5 whose coefficients the launcher computes for the call's p.  m itself is x times
+// +-2^(127 - e), an integer subtraction from the bits of the exponent, which carries the sign and what is not finite:
+//   e = 0     T is 0: zeros and (like lg2.approx.ftz) denormals add nothing
+//   e = 254   the factor 2^-127 comes out as 0, so f = -1.5; with p >= POW_MIN the power overflows anyway, and T is an
+//             infinity of the sign that the polynomial has there
+//   e = 255   an infinity times an infinity of its own sign, negated: f = -inf, T has the sign of the polynomial; a NaN
+//             stays one
+// The polynomial is within 3e-7 of m^p for exponents in [POW_MIN, POW_MAX], and within 1.5e-7 up to 3.5.
+constexpr int   POW_DEGREE = 6;
+constexpr int   POW_ENTRIES = 512;
+constexpr float POW_MIN = 1.01f, POW_MAX = 4.0f;
+struct PowCoefs {
+    float c[POW_DEGREE + 1];    // of f^0 .. f^POW_DEGREE
+    float t254, t255;           // table entries of the two topmost exponents
+    int   use;                  // the call's exponent is taken this way
+};
+struct PowTable {
+    u64      c[POW_DEGREE + 1];
+    uint32_t base;              // shared-memory address of the table
+};
+// 2^(i p) to about one unit in the last place: the exponent is split exactly, 2^f comes from its series.
+__device__ __forceinline__ float exp2_multiple(int i, float p) {
+    const float x  = static_cast<float>(i);
+    const float hi = __fmul_rn(x, p), lo = fmaf(x, p, -hi);
+    const float n  = fminf(fmaxf(rintf(hi), -200.0f), 200.0f);
+    const float f  = (hi - n) + lo;
+    float q = 1.5252734e-5f;                 // ln(2)^k / k!, k = 7 .. 1
+    q = fmaf(q, f, 1.5403530e-4f);
+    q = fmaf(q, f, 1.3333558e-3f);
+    q = fmaf(q, f, 9.6181291e-3f);
+    q = fmaf(q, f, 5.5504109e-2f);
+    q = fmaf(q, f, 2.4022651e-1f);
+    q = fmaf(q, f, 6.9314718e-1f);
+    return ldexpf(fmaf(q, f, 1.0f), static_cast<int>(n));
+}
+__device__ __forceinline__ void fill_pow_table(float* table, const PowCoefs& pc, float p, int tid, int threads) {
+    for (int i = tid; i < POW_ENTRIES; i += threads) {
+        const int e = i & 255;
+        table[i] = e == 0 ? 0.0f : e == 254 ? pc.t254 : e == 255 ? pc.t255 : exp2_multiple(e - 127, p);
+    }
+}
+
 // ---------------------------------------------------------------- result stores
 // Ordinary stores, or multimem.st to an NVSwitch multicast address: one store that the
 // switch delivers to the same offset of every GPU bound to the multicast object.
@@ -290,6 +335,7 @@ enum InnerId {
     IN_DIFF_POW,
     IN_DIFF_NOOP,
     IN_DIFF_SQRT,
+    IN_DIFF_POW_TABLE,     // IN_DIFF_POW for an exponent that PowTable takes; chosen by the launcher
     IN_DOT_NOOP,
     IN_DOT_ABS,
     IN_DOT_SQUARE,
@@ -390,13 +436,70 @@ __device__ __forceinline__ void inner_block(u64 (&acc)[8][MP], const u64 (&ap)[M
     }
 }
 
+// The pairs of 16 (of a register block, row by row) that take |x|^p as lg2 and ex2 on MUFU; the others take the table.
+// A pair costs 32 MUFU cycles of a scheduler one way; the other way about 25 cycles of the FP32 pipe (nine packed
+// instructions, most with three different sources), 12 of the ALU and 16 issue slots.  Rows alternate, so both pipes
+// have work at any time.  Measured with 6 / 7 / 8 / 9 of 16 on MUFU: 2 x 16384^2 x 512, p = 1.3, 78.1 / 76.3 / 75.2 /
+// 82 ms (all of them lg2 on MUFU and six of eight ex2_poly2: 98.5); in the 64 x 64 kernel, unrolled by 4, 7 / 8:
+// 8000^2 x 96 rows 1730 / 1885 us (2260), 4000^2 x 512 rows 2301 / 2532 (3040).
+__host__ __device__ constexpr int pow_mufu_sixteenths(int mp_count) { return mp_count == 4 ? 8 : 7; }
+template <int MP>
+__device__ __forceinline__ constexpr bool pow_pair_uses_mufu(int n, int mp) {
+    constexpr int ROWS = 16 / MP;                              // rows of 16 pairs: even ones first
+    const int r    = n % ROWS;
+    const int rank = (r & 1) ? ROWS / 2 + (r >> 1) : (r >> 1);
+    return rank * MP + mp < pow_mufu_sixteenths(MP);
+}
+
+// One k step of |b - a|^p, with the arguments of inner_block.
+template <int MP>
+__device__ __forceinline__ void pow_block(u64 (&acc)[8][MP], const u64 (&ap)[MP], const float (&bv)[8], float p_inner,
+                                          const PowTable& table) {
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+        const u64 bd = pack2(bv[n], bv[n]);
+        u64 f[MP], t[MP], q[MP];
+#pragma unroll
+        for (int mp = 0; mp < MP; ++mp) {
+            const u64 d = sub2(bd, ap[mp]);
+            float d0, d1;
+            unpack2(d, d0, d1);
+            if (pow_pair_uses_mufu<MP>(n, mp)) {
+                float x0, x1;
+                unpack2(mul2(pack2(lg2_approx(fabsf(d0)), lg2_approx(fabsf(d1))), pack2(p_inner, p_inner)), x0, x1);
+                acc[n][mp] = add2(acc[n][mp], pack2(ex2_approx(x0), ex2_approx(x1)));
+            } else {
+                const uint32_t h0 = __float_as_uint(d0) & 0xFF800000u, h1 = __float_as_uint(d1) & 0xFF800000u;
+                // (as an array in shared memory: 2 % slower with 32 pairs, 4 % with 16)
+                float t0, t1;
+                asm("ld.shared.f32 %0, [%1];" : "=f"(t0) : "r"(table.base + (h0 >> 21)));
+                asm("ld.shared.f32 %0, [%1];" : "=f"(t1) : "r"(table.base + (h1 >> 21)));
+                t[mp] = pack2(t0, t1);
+                f[mp] = fma2(d, pack2(__uint_as_float(0x7F000000u - h0), __uint_as_float(0x7F000000u - h1)),
+                             pack2(-1.5f, -1.5f));
+            }
+        }
+        // the polynomials of a row side by side
+#pragma unroll
+        for (int k = POW_DEGREE; k >= 0; --k)
+#pragma unroll
+            for (int mp = 0; mp < MP; ++mp) {
+                if (pow_pair_uses_mufu<MP>(n, mp)) continue;
+                q[mp] = k == POW_DEGREE ? table.c[k] : fma2(q[mp], f[mp], table.c[k]);
+            }
+#pragma unroll
+        for (int mp = 0; mp < MP; ++mp)
+            if (!pow_pair_uses_mufu<MP>(n, mp)) acc[n][mp] = fma2(q[mp], t[mp], acc[n][mp]);
+    }
+}
+
 // Consumes one staged k slab ([BK][PITCH] floats per operand, tile dimension
 // contiguous) for a thread whose 8 x 2 MP block reads the m-side at sa + {0, 32} (MP = 4) or
 // sa (MP = 2) and the n-side at sb + {0, 16}.  Only the first `kvalid` k rows are used, so a partial
 // last slab contributes exactly the rows that exist.
 template <int INNER, int BK, int PITCH, int MP>
 __device__ __forceinline__ void consume_slab(u64 (&acc)[8][MP], const float* sa, const float* sb, int kvalid,
-                                             float p_inner, float sgn) {
+                                             float p_inner, float sgn, const PowTable& table = PowTable()) {
     auto step = [&](int kk) {
         u64 ap[MP];
 #pragma unroll
@@ -418,12 +521,15 @@ __device__ __forceinline__ void consume_slab(u64 (&acc)[8][MP], const float* sa,
             bv[0] = b0.x; bv[1] = b0.y; bv[2] = b0.z; bv[3] = b0.w;
             bv[4] = b1.x; bv[5] = b1.y; bv[6] = b1.z; bv[7] = b1.w;
         }
-        inner_block<INNER>(acc, ap, bv, p_inner, sgn);
+        if constexpr (INNER == IN_DIFF_POW_TABLE) pow_block(acc, ap, bv, p_inner, table);
+        else inner_block<INNER>(acc, ap, bv, p_inner, sgn);
     };
     // The whole slab is unrolled, so operand loads are scheduled ahead of the math across all
     // of its rows.  The fractional-power step is ~30 instructions per element; unrolling it
-    // that far would not fit the instruction cache, so it is unrolled by 2 only.
-    constexpr int UNROLL = (INNER == IN_DIFF_POW || INNER == IN_DOT_POW) ? 2 : BK;
+    // that far would not fit the instruction cache, so it is unrolled by 2 only.  The one with the table is some 450
+    // instructions a row of 32 pairs and is not unrolled at all there (2 x 16384^2 x 512, p = 1.3: 76.3 ms, by 2 85.6,
+    // by 4 84.4); in the 64 x 64 kernel, with half the pairs, by 4 (8000^2 x 96 rows: 1853, by 2 1816, by 4 1730 us).
+    constexpr int UNROLL = INNER == IN_DIFF_POW_TABLE ? (MP == 4 ? 1 : 4) : (INNER == IN_DIFF_POW || INNER == IN_DOT_POW) ? 2 : BK;
     if (kvalid >= BK) {
 #pragma unroll UNROLL
         for (int kk = 0; kk < BK; ++kk) step(kk);
