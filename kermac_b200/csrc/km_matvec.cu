@@ -223,8 +223,10 @@ __global__ void __launch_bounds__(MV_THREADS, 2) matvec_kernel(const __grid_cons
 //
 // fp32 accuracy is kept by splitting every operand value x into hi = x with the 13
 // low mantissa bits cleared (exactly representable in tf32) and lo = x - hi, and
-// issuing three products per k-block: hi*c_hi + lo*c_hi + hi*c_lo (the dropped
-// lo*c_lo term is below 2^-22 of the product).
+// adding three products per k-block: hi*c_hi + lo*c_hi + hi*c_lo (the dropped
+// lo*c_lo term is below 2^-22 of the product).  hi * [c_hi | c_lo] is one MMA of 32
+// columns, lo * c_hi one of 16 that adds to the right half of its result: an MMA
+// holds the tensor pipe as long with 16 columns as with 32.
 //
 // A tile is contracted in two rounds of 64 m-columns (the columns a thread holds in
 // its accumulator halves h = 0, 1), so that hi and lo of a round fit in 64 KiB.
@@ -233,24 +235,25 @@ __global__ void __launch_bounds__(MV_THREADS, 2) matvec_kernel(const __grid_cons
 //
 // The tensor core truncates when it adds into its fp32 accumulator, so a long chain
 // of MMAs drifts low (measured: 5e-6 relative after 48 steps on same-sign data).
-// Chains are therefore kept short: per tile, each round's hi*c_hi products (8 MMAs)
-// have their own 16-column accumulator and the two correction products share a third,
-// whose truncation is relative to sums 2^-11 smaller.  The three partial sums are
-// added, rounding to nearest, to the thread's fp32 running sums one tile later, when
-// the tile's MMAs are known to be complete (two sets of accumulators alternate).
+// Chains are therefore kept short: each round's hi*c_hi products (8 MMAs) have their
+// own 16-column accumulator and the two correction products share another, whose
+// truncation is relative to sums 2^-11 smaller.  A tile's four partial sums are added,
+// rounding to nearest, to the thread's fp32 running sums one tile later, when the
+// tile's MMAs are known to be complete (two sets of accumulators alternate).
+// A round's MMAs are issued by one elected lane in warp-uniform code: issued behind a
+// test of the thread index they took 80 cycles each, 3700 of the 15200 cycles of a tile
+// of 27 features, during which the issuing warp held back everybody's next slab.
 // One mbarrier tracks MMA completion (tcgen05.commit); every wait on it is bounded.
 constexpr int MT_OT         = 16;
 constexpr int MT_SLAB_A     = 128 * 128;              // bytes: 128 rows (n) of 32 floats
-constexpr int MT_SLAB_B     = MT_OT * 128;            // bytes: 16 rows (o) of 32 floats
+constexpr int MT_SLAB_B     = 2 * MT_OT * 128;        // bytes: 16 rows c_hi[o] and 16 rows c_lo[o] of 32 floats
 constexpr int MT_A_BYTES    = 2 * MT_SLAB_A;          // one round: 64 m-columns
-constexpr int MT_B_BYTES    = 2 * MT_SLAB_B;
 constexpr int MT_OFF_A_HI   = 0;
 constexpr int MT_OFF_A_LO   = MT_A_BYTES;
-constexpr int MT_OFF_B_HI   = 2 * MT_A_BYTES;
-constexpr int MT_OFF_B_LO   = 2 * MT_A_BYTES + MT_B_BYTES;
-constexpr int MT_TILE_BYTES = 2 * MT_A_BYTES + 2 * MT_B_BYTES;
+constexpr int MT_OFF_B      = 2 * MT_A_BYTES;
+constexpr int MT_TILE_BYTES = 2 * MT_A_BYTES + 2 * MT_SLAB_B;
 constexpr int MT_SMEM_BYTES = 1024 + MT_TILE_BYTES + MV_STAGES * MV_STAGE_FLOATS * 4;
-constexpr int MT_TMEM_SET   = 64;                     // columns per tile: main h=0, main h=1, corrections, (unused)
+constexpr int MT_TMEM_SET   = 64;                     // columns per tile: per round, hi * c_hi and the corrections
 constexpr int MT_TMEM_COLS  = 2 * MT_TMEM_SET;
 static_assert(MT_TILE_BYTES % 1024 == 0 && MT_SLAB_B % 1024 == 0, "operand slabs must stay 1024-byte aligned");
 
@@ -323,7 +326,8 @@ matvec_tensor_kernel(const __grid_constant__ MatvecParams p, const __grid_consta
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    const uint32_t tmem = s_tmem;
+    const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, s_tmem, 0);
+    const int warp_u    = __shfl_sync(0xFFFFFFFFu, warp, 0);     // warp-uniform, and known to be
 
     const int lm = lane & 7, ln = lane >> 3;
     const int wm = warp & 1, wn = warp >> 1;
@@ -348,25 +352,21 @@ matvec_tensor_kernel(const __grid_constant__ MatvecParams p, const __grid_consta
 #pragma unroll
         for (int i = 0; i < 4; ++i) acc[j][i] = 0ull;
 
-    bool pending = false;   // a commit has been issued that nobody has waited for yet
-    int  parity  = 0;
     bool expired = false;
-    auto wait_mma = [&]() {
-        if (pending) {
-            // once a wait has run out this thread stops waiting, so a stuck barrier costs one limit, not one per tile
-            if (!expired && !mbar_wait_bounded(bar, parity)) expired = true;
-            parity ^= 1;
-            pending = false;
-        }
+    // Waits for a round's MMAs: round h of any chunk completes a phase of parity h.
+    auto wait_mma = [&](int h) {
+        // once a wait has run out this thread stops waiting, so a stuck barrier costs one limit, not one per tile
+        if (!expired && !mbar_wait_bounded(bar, h)) expired = true;
     };
     auto drain = [&](int buffer) {
         tc::fence_after_sync();
+        uint32_t r[4][8];                    // main and corrections of the first round, then of the second
+        tc::ld4_32x32b_x8(tmem_mine + buffer * MT_TMEM_SET, MT_OT, r);
 #pragma unroll
-        for (int part = 0; part < 3; ++part) {
-            uint32_t r[8];
-            tc::ld_32x32b_x8(tmem_mine + buffer * MT_TMEM_SET + part * MT_OT, r);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) yacc[i] += __uint_as_float(r[i]);
+        for (int i = 0; i < 8; ++i) {
+            yacc[i] += __uint_as_float(r[0][i]);
+            yacc[i] += __uint_as_float(r[2][i]);
+            yacc[i] += __uint_as_float(r[1][i]) + __uint_as_float(r[3][i]);
         }
         tc::fence_before_sync();
     };
@@ -377,10 +377,11 @@ matvec_tensor_kernel(const __grid_constant__ MatvecParams p, const __grid_consta
     const int lb = (p.b_sl == 0) ? 0 : l;
     int fail_it = -1;                       // first slab whose wait ran out on this thread
 
-    auto stage = [&](int it) {
-        const int chunk = it / ktiles, kt = it - chunk * ktiles;
-        const int mc0   = m_begin + chunk * MV_TILE;
-        float* st       = stages + (it % MV_STAGES) * STAGE_FLOATS;
+    // slab `it` of the walk, which is slab `kt` of a chunk; kt may run on into the chunks after it
+    auto stage = [&](int it, int chunk, int kt) {
+        for (; kt >= ktiles; kt -= ktiles) ++chunk;
+        const int mc0 = m_begin + chunk * MV_TILE;
+        float* st     = stages + (it % MV_STAGES) * STAGE_FLOATS;
         if constexpr (TMA) {
             const int s        = it % MV_STAGES;
             const uint32_t dst = smem_u32(st);
@@ -395,15 +396,15 @@ matvec_tensor_kernel(const __grid_constant__ MatvecParams p, const __grid_consta
 
     if constexpr (TMA) {
         if (tid == 0)
-            for (int it = 0; it < MV_STAGES && it < total; ++it) stage(it);
+            for (int it = 0; it < MV_STAGES && it < total; ++it) stage(it, 0, it);
     } else {
-        if (total > 0) stage(0);
+        if (total > 0) stage(0, 0, 0);
         cp_async_commit();
     }
 
+    int chunk = 0, kt = 0;                  // (carried along: a division in each slab shows)
     for (int it = 0; it < total; ++it) {
-        const int chunk = it / ktiles, kt = it - chunk * ktiles;
-        const int s     = it % MV_STAGES;
+        const int s = it % MV_STAGES;
         if constexpr (TMA) {
             if (!expired && !mbar_wait_bounded(full_bar(s), (it / MV_STAGES) & 1)) {
                 expired = true;
@@ -412,7 +413,7 @@ matvec_tensor_kernel(const __grid_constant__ MatvecParams p, const __grid_consta
         } else {
             cp_async_wait<0>();
             __syncthreads();
-            if (it + 1 < total) stage(it + 1);
+            if (it + 1 < total) stage(it + 1, chunk, kt + 1);
             cp_async_commit();
         }
 
@@ -425,11 +426,11 @@ matvec_tensor_kernel(const __grid_constant__ MatvecParams p, const __grid_consta
             __syncwarp();
             if (lane == 0 && mbar_arrive_pending(empty_bar(s)) == 1 && it + MV_STAGES < total && !expired) {
                 mbar_try_wait(empty_bar(s), (it / MV_STAGES) & 1);   // the acquire side of the hand-over
-                stage(it + MV_STAGES);
+                stage(it + MV_STAGES, chunk, kt + MV_STAGES);
             }
         }
 
-        if (kt == ktiles - 1) {
+        if (++kt == ktiles) {
             const int mc0 = m_begin + chunk * MV_TILE;
             const uint32_t d_set = tmem + (chunk & 1) * MT_TMEM_SET;
             // diagonal rule; read here, once per tile, so nothing of it stays live through the k loop
@@ -465,7 +466,7 @@ matvec_tensor_kernel(const __grid_constant__ MatvecParams p, const __grid_consta
                     for (int e = 0; e < 4; ++e) cv[e] = (o_ok && mg + e < m_end) ? crow[mg + e] : 0.0f;
                 }
                 // the previous round's MMAs must have finished reading the operand tiles
-                wait_mma();
+                if (h == 1 || chunk > 0) wait_mma(h ^ 1);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     const int r = tn_off + (j >> 2) * 16 + (j & 3);
@@ -485,8 +486,8 @@ matvec_tensor_kernel(const __grid_constant__ MatvecParams p, const __grid_consta
 #pragma unroll
                     for (int e = 0; e < 4; ++e) { hi[e] = tf32_hi(cv[e]); lo[e] = cv[e] - hi[e]; }
                     const int off = (cq >> 3) * MT_SLAB_B + co * 128 + (((cq & 7) ^ (co & 7)) << 4);
-                    *reinterpret_cast<float4*>(tiles + MT_OFF_B_HI + off) = make_float4(hi[0], hi[1], hi[2], hi[3]);
-                    *reinterpret_cast<float4*>(tiles + MT_OFF_B_LO + off) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+                    *reinterpret_cast<float4*>(tiles + MT_OFF_B + off) = make_float4(hi[0], hi[1], hi[2], hi[3]);
+                    *reinterpret_cast<float4*>(tiles + MT_OFF_B + MT_OT * 128 + off) = make_float4(lo[0], lo[1], lo[2], lo[3]);
                 }
                 if (on_diagonal) {
                     // diagonal rule on the parked tile: row n holds 1 + reg at m = n + delta
@@ -505,33 +506,40 @@ matvec_tensor_kernel(const __grid_constant__ MatvecParams p, const __grid_consta
                 tc::fence_smem_to_async();
                 tc::fence_before_sync();
                 __syncthreads();
-                if (tid == 0) {
+                if (warp_u == 5 * h) {       // (another scheduler's warp for the second round)
                     tc::fence_after_sync();
-                    constexpr uint32_t idesc = tc::instr_desc_tf32(MV_TILE, MT_OT);
-#pragma unroll
-                    for (int pass = 0; pass < 3; ++pass) {
-                        const uint32_t a_base = tile_addr + (pass == 1 ? MT_OFF_A_LO : MT_OFF_A_HI);
-                        const uint32_t b_base = tile_addr + (pass == 2 ? MT_OFF_B_LO : MT_OFF_B_HI);
+                    const uint64_t a_hi = tc::smem_desc_k_major_sw128(tile_addr + MT_OFF_A_HI);
+                    const uint64_t a_lo = tc::smem_desc_k_major_sw128(tile_addr + MT_OFF_A_LO);
+                    const uint64_t b_hl = tc::smem_desc_k_major_sw128(tile_addr + MT_OFF_B);
+                    const uint32_t d    = d_set + h * 2 * MT_OT;
+                    if (tc::elect_one()) {
 #pragma unroll
                         for (int kb = 0; kb < 8; ++kb) {
-                            const uint64_t da = tc::smem_desc_k_major_sw128(a_base + (kb >> 2) * MT_SLAB_A + (kb & 3) * 32);
-                            const uint64_t db = tc::smem_desc_k_major_sw128(b_base + (kb >> 2) * MT_SLAB_B + (kb & 3) * 32);
-                            if (pass == 0) tc::mma_tf32(d_set + h * MT_OT, da, db, idesc, kb != 0);
-                            else           tc::mma_tf32(d_set + 2 * MT_OT, da, db, idesc, !(h == 0 && pass == 1 && kb == 0));
+                            const uint32_t da = ((kb >> 2) * MT_SLAB_A + (kb & 3) * 32) >> 4, db = ((kb >> 2) * MT_SLAB_B + (kb & 3) * 32) >> 4;
+                            tc::mma_tf32(d, a_hi + da, b_hl + db, tc::instr_desc_tf32(MV_TILE, 2 * MT_OT), kb != 0);
                         }
+#pragma unroll
+                        for (int kb = 0; kb < 8; ++kb) {
+                            const uint32_t da = ((kb >> 2) * MT_SLAB_A + (kb & 3) * 32) >> 4, db = ((kb >> 2) * MT_SLAB_B + (kb & 3) * 32) >> 4;
+                            tc::mma_tf32(d + MT_OT, a_lo + da, b_hl + db, tc::instr_desc_tf32(MV_TILE, MT_OT), true);
+                        }
+                        tc::commit(bar);
                     }
-                    tc::commit(bar);
+                    __syncwarp();
                 }
-                pending = true;
             }
             // the tile before this one finished before this tile's first round started
             if (chunk > 0) drain((chunk - 1) & 1);
+            kt = 0;
+            ++chunk;
         }
     }
     cp_async_wait<0>();
 
-    wait_mma();
-    if (chunks > 0) drain((chunks - 1) & 1);
+    if (chunks > 0) {
+        wait_mma(1);
+        drain((chunks - 1) & 1);
+    }
     if (expired) {
         atomicExch(&g_matvec_wait_expired, 1);
         if constexpr (TMA) {
