@@ -161,6 +161,7 @@ __global__ void __launch_bounds__(CPA_THREADS, 2) build_cpasync_kernel(const __g
 
     int tm, tn;
     tile_coords(p.tile_first + blockIdx.x, p.tiles_m, p.tiles_n, p.panel, tm, tn);
+    after_previous_grid();
     if (SYM && tn < tm) return;   // the tile's mirror image (tn, tm) writes this part of C
     const int m0 = tm * CPA_TILE;
     const int n0 = tn * CPA_TILE;

@@ -351,8 +351,9 @@ int launch_plan(const BuildPlan& plan, cudaStream_t st) {
         if (q.bandwidth.ptr) q.bandwidth.ptr += (long long)l0 * q.bandwidth.batch_stride;
         if (q.regularization.ptr) q.regularization.ptr += (long long)l0 * q.regularization.batch_stride;
         dim3 grid((unsigned)q.tile_count, (unsigned)q.L, 1);
-        fn<<<grid, BUILD_CPA_THREADS, BUILD_CPA_SMEM_BYTES, st>>>(q);
-        if (int rc = cuda_status(cudaGetLastError(), "launch of build_cpasync_kernel")) return rc;
+        if (int rc = cuda_status(launch_overlapped(fn, grid, BUILD_CPA_THREADS, BUILD_CPA_SMEM_BYTES, st, q),
+                                 "launch of build_cpasync_kernel"))
+            return rc;
     }
     return 0;
 }

@@ -265,10 +265,12 @@ build_small_kernel(const __grid_constant__ SmallParams sp, const __grid_constant
         tn = tn * 2 + ((blockIdx.x >> 1) & 1);
     }
     const int m0 = tm * SB_TILE, n0 = tn * SB_TILE;
-    if (m0 >= p.M || n0 >= p.N) return;
+    if (m0 >= p.M || n0 >= p.N) {
+        after_previous_grid();
+        return;
+    }
     const int K  = p.K;
     const int ktiles = (K + SB_BK - 1) / SB_BK;
-    const float p_inner = (INNER == IN_DIFF_POW || INNER == IN_DIFF_POW_TABLE) ? read_hyper(p.p_inner, l) : 0.0f;
 
     const int tm_off = (warp & 1) * 32 + (lane & 7) * 4;
     const int tn_off = (warp >> 1) * 32 + (lane >> 3) * 4;   // + {0, 16}
@@ -277,6 +279,7 @@ build_small_kernel(const __grid_constant__ SmallParams sp, const __grid_constant
 #pragma unroll
     for (int j = 0; j < 8; ++j) acc[j][0] = acc[j][1] = 0ull;
 
+    float p_inner = 0.0f;
     if constexpr (TMA) {
         const uint32_t smem_base = smem_u32(smem);
         const uint32_t bar_base  = smem_u32(bars);
@@ -301,6 +304,7 @@ build_small_kernel(const __grid_constant__ SmallParams sp, const __grid_constant
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         }
         __syncthreads();
+        after_previous_grid();
         if (tid == 0) {
             for (int s = 0; s < SB_RING && s < ktiles; ++s) issue(s);
         }
@@ -337,18 +341,21 @@ build_small_kernel(const __grid_constant__ SmallParams sp, const __grid_constant
                          p.a_sm, p.a_sk, p.M - m0, K, sp.stage_a, tid, {}};
         SlabLoader lb = {p.B + static_cast<long long>(l) * p.b_sl + static_cast<long long>(n0) * p.b_sn,
                          p.b_sn, p.b_sk, p.N - n0, K, sp.stage_b, tid, {}};
-        la.start(smem, 0);
-        lb.start(smem + SB_BK * PITCH, 0);
-        cp_async_commit();
         PowTable table;
         if constexpr (INNER == IN_DIFF_POW_TABLE) {
             // (the first barrier of the k loop publishes it)
             __shared__ float s_pow[POW_ENTRIES];
+            p_inner = p.p_inner.value;
             fill_pow_table(s_pow, p.pow, p_inner, tid, SB_THREADS);
             table.base = smem_u32(s_pow);
 #pragma unroll
             for (int i = 0; i <= POW_DEGREE; ++i) table.c[i] = pack2(p.pow.c[i], p.pow.c[i]);
         }
+        after_previous_grid();
+        if (INNER == IN_DIFF_POW) p_inner = read_hyper(p.p_inner, l);
+        la.start(smem, 0);
+        lb.start(smem + SB_BK * PITCH, 0);
+        cp_async_commit();
         la.finish(smem);
         lb.finish(smem + SB_BK * PITCH);
         for (int kt = 0; kt < ktiles; ++kt) {
@@ -437,8 +444,8 @@ int launch_build_small(const BuildParams& p, bool tma, cudaStream_t stream) {
     }
     const long long edge = ceil_div_ll(p.N, SB_TILE);
     const long long tiles = p.symmetric ? edge * (edge + 1) / 2 : 4LL * p.tile_count;
-    fn<<<dim3((unsigned)tiles, (unsigned)p.L, 1), SB_THREADS, 0, stream>>>(sp, map_a, map_b);
-    return cuda_status(cudaGetLastError(), "launch of build_small_kernel");
+    return cuda_status(launch_overlapped(fn, dim3((unsigned)tiles, (unsigned)p.L, 1), SB_THREADS, 0, stream, sp, map_a, map_b),
+                       "launch of build_small_kernel");
 }
 
 }  // namespace km

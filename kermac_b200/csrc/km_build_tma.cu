@@ -60,7 +60,10 @@ build_tma_kernel(const __grid_constant__ BuildParams p, const __grid_constant__ 
 
     int tm, tn;
     tile_coords(p.tile_first + blockIdx.x, p.tiles_m, p.tiles_n, p.panel, tm, tn);
-    if (SYM && tn < tm) return;   // the tile's mirror image (tn, tm) writes this part of C
+    if (SYM && tn < tm) {         // the tile's mirror image (tn, tm) writes this part of C
+        after_previous_grid();
+        return;
+    }
     const int m0 = tm * TMA_TILE;
     const int n0 = tn * TMA_TILE;
     const int K  = p.K;
@@ -78,6 +81,7 @@ build_tma_kernel(const __grid_constant__ BuildParams p, const __grid_constant__ 
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncthreads();
+    after_previous_grid();
 
     auto issue = [&](int slab) {
         const int s        = slab % STAGES;
@@ -300,8 +304,9 @@ int launch_build_tma(const BuildParams& p, cudaStream_t stream) {
         if (int rc = encode_operand(&map_a, q.A, q.M, q.K, q.L, q.a_sk, q.a_sl, kBK)) return rc;
         if (int rc = encode_operand(&map_b, q.B, q.N, q.K, q.L, q.b_sk, q.b_sl, kBK)) return rc;
         dim3 grid((unsigned)q.tile_count, (unsigned)q.L, 1);
-        fn<<<grid, TMA_THREADS, kSmemBytes, stream>>>(q, map_a, map_b);
-        if (int rc = cuda_status(cudaGetLastError(), "launch of build_tma_kernel")) return rc;
+        if (int rc = cuda_status(launch_overlapped(fn, grid, TMA_THREADS, kSmemBytes, stream, q, map_a, map_b),
+                                 "launch of build_tma_kernel"))
+            return rc;
     }
     return 0;
 }

@@ -68,6 +68,7 @@ __global__ void __launch_bounds__(G_THREADS, grad_min_blocks(OT, NT)) grad_kerne
 
     const int tid = threadIdx.x;
     const int tmi = tid & 15, tni = tid >> 4;
+    after_previous_grid();
 
     // n-tiles fastest: the blocks that read the same (k range, m-column) tile of a run together
     int bx          = blockIdx.x;
@@ -366,6 +367,7 @@ template <typename Index>
 __global__ void __launch_bounds__(256) grad_reduce_kernel(const float* __restrict__ partial, float* __restrict__ out,
                                                           int M, int N, int O, int L, int splits, long long split_stride,
                                                           long long o_sn, long long o_so, long long o_sl) {
+    after_previous_grid();
     const Index total = (Index)L * O * N * M;
     const Index step  = (Index)gridDim.x * blockDim.x;
     for (Index i = blockIdx.x * (Index)blockDim.x + threadIdx.x; i < total; i += step) {
@@ -670,17 +672,18 @@ int run_plan(const KmGradArgs* args, GradPlan& plan, int splits, void* scratch, 
                              "cudaFuncSetAttribute(grad_kernel)"))
         return rc;
     dim3 grid((unsigned)((long long)p.tiles_m * p.tiles_n * splits), (unsigned)p.o_chunks, (unsigned)p.L);
-    fn<<<grid, G_THREADS, choice.smem_bytes, st>>>(p);
-    if (int rc = cuda_status(cudaGetLastError(), "launch of grad_kernel")) return rc;
+    if (int rc = cuda_status(launch_overlapped(fn, grid, G_THREADS, choice.smem_bytes, st, p), "launch of grad_kernel")) return rc;
     }
     if (splits > 1) {
         const long long total = plan.partial_elems;
         int blocks = (int)(ceil_div_ll(total, 256) < 8LL * sm_count() ? ceil_div_ll(total, 256) : 8LL * sm_count());
         // (below 2^31 the grid stride cannot overflow 32 unsigned bits)
         auto reduce = total < (1LL << 31) ? grad_reduce_kernel<unsigned int> : grad_reduce_kernel<long long>;
-        reduce<<<blocks, 256, 0, st>>>(p.E, args->out, p.M, p.N, p.O, p.L, splits, plan.partial_elems,
-                                                   args->out_stride_n, args->out_stride_o, args->out_stride_l);
-        if (int rc = cuda_status(cudaGetLastError(), "launch of grad_reduce_kernel")) return rc;
+        if (int rc = cuda_status(launch_overlapped(reduce, dim3((unsigned)blocks), 256, 0, st, p.E, args->out, p.M, p.N, p.O, p.L,
+                                                   splits, plan.partial_elems, args->out_stride_n, args->out_stride_o,
+                                                   args->out_stride_l),
+                                 "launch of grad_reduce_kernel"))
+            return rc;
     }
     return 0;
 }

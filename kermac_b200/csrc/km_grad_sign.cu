@@ -169,6 +169,7 @@ grad_sign_kernel(const __grid_constant__ GradTensorParams p, const __grid_consta
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
+    after_previous_grid();
     const uint32_t tmem = s_tmem;
     bool expired = false;
     // (One lane waiting for its warp instead of all 32 was three times slower in all.)
@@ -515,8 +516,7 @@ int grad_sign_launch_as(const GradTensorParams& p, cudaStream_t st) {
                              "cudaFuncSetAttribute(grad_sign_kernel)"))
         return rc;
     dim3 grid((unsigned)((long long)p.tiles_m * p.tiles_n * p.splits), (unsigned)p.o_chunks, (unsigned)p.L);
-    fn<<<grid, S::THREADS, S::SMEM, st>>>(p, map_b);
-    return cuda_status(cudaGetLastError(), "launch of grad_sign_kernel");
+    return cuda_status(launch_overlapped(fn, grid, S::THREADS, S::SMEM, st, p, map_b), "launch of grad_sign_kernel");
 }
 
 template <int OT>

@@ -236,6 +236,7 @@ grad_tensor_kernel(const __grid_constant__ GradTensorParams p, const __grid_cons
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
+    after_previous_grid();
     const uint32_t tmem = s_tmem;
     bool expired = false;
 
@@ -575,8 +576,7 @@ int grad_tensor_launch_shape(const GradTensorParams& p, int norm_kind, cudaStrea
                              "cudaFuncSetAttribute(grad_tensor_kernel)"))
         return rc;
     dim3 grid((unsigned)((long long)p.tiles_m * p.tiles_n * p.splits), (unsigned)p.o_chunks, (unsigned)p.L);
-    fn<<<grid, S::THREADS, S::SMEM_BYTES, st>>>(p, map_a, map_b);
-    return cuda_status(cudaGetLastError(), "launch of grad_tensor_kernel");
+    return cuda_status(launch_overlapped(fn, grid, S::THREADS, S::SMEM_BYTES, st, p, map_a, map_b), "launch of grad_tensor_kernel");
 }
 
 }  // namespace

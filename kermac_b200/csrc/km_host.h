@@ -90,6 +90,24 @@ int cheapest_split(long long units, long long last, Cost cost) {
     return 1;
 }
 
+// fn<<<grid, threads, smem_bytes, stream>>>(args...), with the start of the kernel overlapping the end of the one before
+// it in the stream.  Only for kernels that call after_previous_grid() before they touch global memory.
+template <typename... Params, typename... Args>
+cudaError_t launch_overlapped(void (*fn)(Params...), dim3 grid, int threads, size_t smem_bytes, cudaStream_t stream,
+                              const Args&... args) {
+    cudaLaunchAttribute attribute;
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config = {};
+    config.gridDim          = grid;
+    config.blockDim         = dim3(static_cast<unsigned>(threads), 1, 1);
+    config.dynamicSmemBytes = smem_bytes;
+    config.stream           = stream;
+    config.attrs            = &attribute;
+    config.numAttrs         = 1;
+    return cudaLaunchKernelEx(&config, fn, static_cast<Params>(args)...);
+}
+
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
 // Checks a KmHyper that is in use: a device vector needs a non-negative stride.

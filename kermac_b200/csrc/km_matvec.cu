@@ -74,6 +74,7 @@ __global__ void __launch_bounds__(MV_THREADS, 2) matvec_kernel(const __grid_cons
     const int m_end   = min(p.M, m_begin + p.m_per_split);
     const int chunks  = (m_end > m_begin) ? (m_end - m_begin + MV_TILE - 1) / MV_TILE : 0;
 
+    after_previous_grid();
     const float* A = p.A + (long long)l * p.a_sl;
     const float* B = p.B + (long long)l * p.b_sl + (long long)n0 * p.b_sn;
     const float* C = p.C + (long long)l * p.c_sl;
@@ -304,9 +305,6 @@ matvec_tensor_kernel(const __grid_constant__ MatvecParams p, const __grid_consta
     const int ktiles = K > 0 ? (K + MV_BK - 1) / MV_BK : 1;
     const int total  = chunks * ktiles;
 
-    const float p_inner = (INNER == IN_DIFF_POW || INNER == IN_DOT_POW) ? read_hyper(p.p_inner, l) : 0.0f;
-    const Epilogue epi  = make_epilogue(p.outer_power, p.kernel_type, p.p_outer, p.bandwidth, p.epsilon, l);
-
     const uint32_t ring = smem_u32(s_ring);
     auto full_bar  = [&](int s) { return ring + 8u * s; };
     auto empty_bar = [&](int s) { return ring + 8u * (MV_STAGES + s); };
@@ -326,6 +324,9 @@ matvec_tensor_kernel(const __grid_constant__ MatvecParams p, const __grid_consta
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
+    after_previous_grid();
+    const float p_inner = (INNER == IN_DIFF_POW || INNER == IN_DOT_POW) ? read_hyper(p.p_inner, l) : 0.0f;
+    const Epilogue epi  = make_epilogue(p.outer_power, p.kernel_type, p.p_outer, p.bandwidth, p.epsilon, l);
     const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, s_tmem, 0);
     const int warp_u    = __shfl_sync(0xFFFFFFFFu, warp, 0);     // warp-uniform, and known to be
 
@@ -574,6 +575,7 @@ matvec_tensor_kernel(const __grid_constant__ MatvecParams p, const __grid_consta
 __global__ void __launch_bounds__(256) matvec_reduce_kernel(const float* __restrict__ partial, float* __restrict__ y,
                                                             int N, int O, int L, int splits, long long split_stride,
                                                             long long y_sn, long long y_so, long long y_sl) {
+    after_previous_grid();
     const long long total = (long long)L * N * O;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         float s = 0.0f;
@@ -870,8 +872,9 @@ extern "C" int kermac_b200_kernel_matvec(const KmMatvecArgs* args, void* stream)
             if (int rc = encode_tma_operand(&map_a, p.A, p.M, p.K, p.L, p.a_sk, p.a_sl, MV_BK)) return rc;
             if (int rc = encode_tma_operand(&map_b, p.B, p.N, p.K, p.L, p.b_sk, p.b_sl, MV_BK)) return rc;
         }
-        fn<<<grid, MV_THREADS, MT_SMEM_BYTES, st>>>(p, map_a, map_b);
-        if (int rc = cuda_status(cudaGetLastError(), "launch of matvec_tensor_kernel")) return rc;
+        if (int rc = cuda_status(launch_overlapped(fn, grid, MV_THREADS, MT_SMEM_BYTES, st, p, map_a, map_b),
+                                 "launch of matvec_tensor_kernel"))
+            return rc;
     } else {
         MatvecFn fn = mv_pick(p.inner_id, plan.ot, plan.avec, plan.bvec);
         if (!fn) return fail(KM_ERR_INTERNAL, "no matvec kernel for inner id %d", p.inner_id);
@@ -879,15 +882,16 @@ extern "C" int kermac_b200_kernel_matvec(const KmMatvecArgs* args, void* stream)
         if (int rc = cuda_status(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes),
                                  "cudaFuncSetAttribute(matvec_kernel)"))
             return rc;
-        fn<<<grid, MV_THREADS, smem_bytes, st>>>(p);
-        if (int rc = cuda_status(cudaGetLastError(), "launch of matvec_kernel")) return rc;
+        if (int rc = cuda_status(launch_overlapped(fn, grid, MV_THREADS, smem_bytes, st, p), "launch of matvec_kernel")) return rc;
     }
     if (splits > 1) {
         const long long total = plan.partial_elems;
         int blocks = (int)(ceil_div_ll(total, 256) < 4LL * sm_count() ? ceil_div_ll(total, 256) : 4LL * sm_count());
-        matvec_reduce_kernel<<<blocks, 256, 0, st>>>(p.Y, args->y, p.N, p.O, p.L, splits, plan.partial_elems,
-                                                     args->y_stride_n, args->y_stride_o, args->y_stride_l);
-        if (int rc = cuda_status(cudaGetLastError(), "launch of matvec_reduce_kernel")) return rc;
+        if (int rc = cuda_status(launch_overlapped(matvec_reduce_kernel, dim3((unsigned)blocks), 256, 0, st, p.Y, args->y, p.N,
+                                                   p.O, p.L, splits, plan.partial_elems, args->y_stride_n, args->y_stride_o,
+                                                   args->y_stride_l),
+                                 "launch of matvec_reduce_kernel"))
+            return rc;
     }
     return 0;
 }

@@ -21,6 +21,7 @@ struct PackParams {
 
 __global__ void __launch_bounds__(PK_THREADS) pack_kernel(const __grid_constant__ PackParams p) {
     __shared__ float tile[PK_K][PK_POINTS + 1];
+    after_previous_grid();
     const bool second  = static_cast<int>(blockIdx.x) >= p.first_blocks;
     const PackJob& job = p.job[second ? 1 : 0];
     const int block    = second ? blockIdx.x - p.first_blocks : blockIdx.x;
@@ -82,8 +83,8 @@ int launch_pack(const PackJob* jobs, int n, int K, cudaStream_t stream) {
         if (i == 0) p.first_blocks = (int)blocks;
         if (jobs[i].L > L) L = jobs[i].L;
     }
-    pack_kernel<<<dim3((unsigned)blocks, (unsigned)L, 1), PK_THREADS, 0, stream>>>(p);
-    return cuda_status(cudaGetLastError(), "launch of pack_kernel");
+    return cuda_status(launch_overlapped(pack_kernel, dim3((unsigned)blocks, (unsigned)L, 1), PK_THREADS, 0, stream, p),
+                       "launch of pack_kernel");
 }
 
 }  // namespace km
