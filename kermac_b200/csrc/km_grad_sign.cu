@@ -13,9 +13,9 @@
 // 128 rows n of the block.
 //
 // Work decomposition: a thread block owns 128 rows n, MT columns m and up to OT channels.
-//   16 generating warps (4 groups of 4): a thread owns one row n (a tensor-memory lane); a group takes
-//      16 k of every second slab of 32, reads them once for all m and writes the signs (8 columns of packed
-//      bf16 pairs per m) with tcgen05.st into a ring of A buffers, one slab each;
+//   8 to 16 generating warps (2 to 4 groups of 4): a thread owns one row n (a tensor-memory lane); a group takes
+//      every second to fourth slab of 32 k, or 16 k of every second one, reads them once for all m and writes the signs
+//      (8 columns of packed bf16 pairs per m and 16 k) with tcgen05.st into a ring of A buffers, one slab each;
 //   8 product warps (4 with few channels): P_m for the slab, split and parked in shared memory as the B operand (K-major rows
 //      of 64 bytes, 64-byte swizzle; row = piece * OT + channel);
 //   2 warps (4 with few channels) issue the MMAs, one accumulator of 3 OT columns (rounded up to 16) per m;
@@ -29,16 +29,17 @@
 // The product warps have no global loads of their own: their fence to the asynchronous units waits for
 // every memory operation of the thread, and behind loads in flight it made each slab as long as a load.
 // What bounds it (B200, K = 30000, M = 4096, N = 256; ms, in brackets the kernel that took these calls before):
-// 4 channels 5.25 (6.2), 8: 5.8 (10.6), 16: 8.6 (20.3), 32: 11.3 (22.0), 64: 22.6 (29.5).
+// 4 channels 4.61 (6.2), 8: 4.84 (10.6), 16: 7.64 (20.3), 32: 9.68 (22.0).
 // The MMAs alone would take 2.5 ms at 32 channels (an MMA of 128 rows x N columns holds the tensor pipe N / 2 cycles,
-// also with the stores to tensor memory beside it), the ALU pipe (permutes and logic, half rate) about 3.5.  At 32 channels a slab of
-// 4 m takes some 1600 cycles: the product warps compute for 920 of them (their instructions issue once in four to
-// five cycles beside the generating warps) and a wait for a phase that is long complete costs 100 to 250.  On the way
+// also with the stores to tensor memory beside it), the ALU pipe (permutes and logic, half rate) about 3.5.  Instructions are
+// what the rest goes to: at 4 channels the generating warps rest for 16 % of a slab, at 32 the product warps for 25 %, each
+// warp issuing once in about nine cycles beside the others, and the hand-overs are a third of what is issued.  On the way
 // here (ms at 4 / 32 channels): one thread issuing all MMAs 18.5 / -; every role handing over per 16 k by its own
 // barrier, four issuing warps 6.7 / 14.5; global loads taken from the product warps 7.0 / 14.2; eight product warps
 // and carried copy addresses 7.5 / 12.4; all MMAs of a slab in one elected block 6.2 / 11.9; 16 k of all eight m
 // per group and slab instead of four 5.5 / 11.9; pieces scaled 5.5 / 12.1; infinite and NaN products left to the sums
-// (bf16_joined) instead of being looked for in each product 5.25 / 11.3.
+// (bf16_joined) instead of being looked for in each product 5.25 / 11.3; the constants of sign_pair in registers 4.6 / 10.9;
+// whole slabs for a group 4.6 / 9.7.
 // Hand-over is by mbarriers, one round per slab; every wait is bounded, and a wait that runs out sets a
 // flag (kermac_b200_device_error_flag) and lets the block run to its end without its results.
 #include <cstring>
@@ -54,8 +55,6 @@ namespace {
 
 constexpr int GS_BK       = 32;     // k per slab (two MMAs)
 constexpr int GS_KA       = 16;     // k per MMA
-constexpr int GS_GROUPS   = 4;      // groups of four generating warps
-constexpr int GS_GEN      = 4 * GS_GROUPS;
 constexpr int GS_DRAIN    = 4;
 constexpr int GS_B_BYTES  = GS_TN * GS_BK * 4;   // one staged slab of b
 constexpr int GS_B_STAGES = 4;
@@ -72,11 +71,23 @@ struct GsShape {
     static constexpr int A_OFF     = MT * COLS;                        // tensor-memory columns before the A buffers
     static constexpr int A_COLS    = MT * GS_BK / 2;                   // one A buffer: a slab's signs for all m
     static constexpr int NB        = (512 - A_OFF) / A_COLS >= GS_DONE ? GS_DONE : (512 - A_OFF) / A_COLS;
+    // Groups of four generating warps, and how many of the two halves of a slab's k a group takes.  Whole slabs mean half
+    // as many hand-overs, each some 65 instructions a warp against 96 (4 m) or 192 (8 m) for the signs of a half; they pay
+    // where there are as many A buffers as groups, or with fewer groups.  Measured at K = 30000, M = 4096, N = 256, ms:
+    //   groups x halves   4 x 1    2 x 2    3 x 2    4 x 2
+    //   4 channels        4.61     4.92     5.06     4.73
+    //   8                 5.37     4.84     4.88     4.89
+    //   16                8.10     8.14     8.22     7.64
+    //   32               10.87     9.80     9.68    10.04
+    static constexpr int GROUPS    = OT == 8 ? 2 : OT == 32 ? 3 : 4;
+    static constexpr int HALVES    = OT == 4 ? 1 : 2;
     // product warps, and warps that issue MMAs (two MMAs per accumulator and slab): with few channels there are more
-    // accumulators and fewer products
+    // accumulators and fewer products.  (Half or twice as many product warps: 32 channels 11.6 / 11.7 ms, 8 channels
+    // 6.1 / 5.2; half as many issuing warps: 4 to 16 channels 6.1 / 5.0 / 9.3.)
     static constexpr int PROD      = OT >= 16 ? 8 : 4;
     static constexpr int ISSUERS   = OT >= 16 ? 2 : 4;
-    static constexpr int WARPS     = GS_GEN + PROD + GS_DRAIN + ISSUERS + 2;
+    static constexpr int GEN       = 4 * GROUPS;
+    static constexpr int WARPS     = GEN + PROD + GS_DRAIN + ISSUERS + 2;
     static constexpr int THREADS   = 32 * WARPS;
     static constexpr int AC_FLOATS = MT * GS_BK + OT * GS_C_PITCH;
     static constexpr int OFF_B     = 0;                                // shared memory, from a 1024-byte boundary
@@ -95,8 +106,24 @@ struct GsShape {
 
 __device__ int g_grad_sign_wait_expired = 0;
 
-// Two k of the A operand: +-1 in bf16 with the signs of two differences.
-__device__ __forceinline__ uint32_t sign_pair(u64 diff) { return (upper_halves(diff) & 0x80008000u) | 0x3F803F80u; }
+// Two k of the A operand: +-1 in bf16 with the signs of two differences, (halves & SIGN_BITS) | ONES.  One LOP3 takes at
+// most one constant of its own: written with both as constants it became two, 512 of 2218 ALU instructions a block and
+// slab at 4 channels, so both are kept in registers (signs_in_registers; 4 / 8 / 16 / 32 channels 5.23 / 5.79 / 8.56 /
+// 11.31 -> 4.61 / 5.37 / 8.10 / 10.87 ms).
+struct SignConstants {
+    uint32_t sign_bits, ones;
+};
+__device__ __forceinline__ SignConstants signs_in_registers() {
+    SignConstants k;
+    asm volatile("mov.b32 %0, 0x80008000;" : "=r"(k.sign_bits));
+    asm volatile("mov.b32 %0, 0x3F803F80;" : "=r"(k.ones));
+    return k;
+}
+__device__ __forceinline__ uint32_t sign_pair(u64 diff, SignConstants k) {
+    uint32_t w;
+    asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(w) : "r"(upper_halves(diff)), "r"(k.sign_bits), "r"(k.ones));
+    return w;
+}
 
 template <int OT, int MT, bool TMA>
 __global__ void __launch_bounds__(GsShape<OT, MT, TMA>::THREADS, 1)
@@ -146,14 +173,14 @@ grad_sign_kernel(const __grid_constant__ GradTensorParams p, const __grid_consta
     if (tid == 0) {
         for (int st = 0; st < GS_B_STAGES; ++st) {
             mbar_init(bfull(st), TMA ? 1 : 32);
-            mbar_init(bempty(st), 8);                  // a slab is read by two groups of four warps
+            mbar_init(bempty(st), 8 / S::HALVES);      // a slab is read by one or two groups of four warps
         }
         for (int sl = 0; sl < GS_AC_SLOTS; ++sl) {
             mbar_init(acfull(sl), 32);
             mbar_init(acempty(sl), S::PROD);
         }
         for (int sl = 0; sl < GS_P_SLOTS; ++sl) mbar_init(pfull(sl), S::PROD);
-        for (int b = 0; b < S::NB; ++b) mbar_init(afull(b), 8);
+        for (int b = 0; b < S::NB; ++b) mbar_init(afull(b), 8 / S::HALVES);
         for (int i = 0; i < GS_DONE; ++i) mbar_init(done(i), S::ISSUERS);
         for (int m = 0; m < MT; ++m) {
             mbar_init(dfull(m), 1);
@@ -164,7 +191,7 @@ grad_sign_kernel(const __grid_constant__ GradTensorParams p, const __grid_consta
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         tc::fence_smem_to_async();
     }
-    constexpr int MMA_WARP = GS_GEN + S::PROD + GS_DRAIN;
+    constexpr int MMA_WARP = S::GEN + S::PROD + GS_DRAIN;
     if (warp == MMA_WARP) tc::tmem_alloc(smem_u32(&s_tmem), 512);
     tc::fence_before_sync();
     __syncthreads();
@@ -181,44 +208,48 @@ grad_sign_kernel(const __grid_constant__ GradTensorParams p, const __grid_consta
         }
     };
 
-    if (warp < GS_GEN) {
+    if (warp < S::GEN) {
         // ------------------------------------------------------------------ signs
         const int q = warp & 3, group = warp >> 2;
         const int row = 32 * q + lane;
         const int n   = n0 + row;
         const float* D = p.D + (long long)l * p.d_sl;
-        // this group's part of a slab: 16 k; two groups make up a slab, the other two the next one
-        const int hf = group & 1;
+        // a group takes all 32 k of every GROUPS-th slab, or two groups make up a slab and take 16 k each
+        const int hf0 = S::HALVES == 2 ? 0 : group & 1;
         u64 dd[MT];
 #pragma unroll
         for (int i = 0; i < MT; ++i) {
             const float v = (n < p.N && m0 + i < p.M) ? D[(long long)n * p.ldd + m0 + i] : 0.0f;
             dd[i] = pack2(v, v);
         }
-        const uint32_t t_row = tmem + (static_cast<uint32_t>(32 * q) << 16) + S::A_OFF + hf * MT * (GS_KA / 2);
+        const uint32_t t_row = tmem + (static_cast<uint32_t>(32 * q) << 16) + S::A_OFF;
+        const SignConstants signs = signs_in_registers();
         const unsigned char* brow = tiles + S::OFF_B + row * (GS_BK * 4);
-        for (int s = group >> 1; s < nslabs; s += GS_GROUPS / 2) {
+        for (int s = group * S::HALVES / 2; s < nslabs; s += S::GROUPS * S::HALVES / 2) {
             const int st = s % GS_B_STAGES;
             wait(bfull(st), (s / GS_B_STAGES) & 1);
-            __syncwarp();
-            u64 b2[GS_KA / 2];
-#pragma unroll
-            for (int i = 0; i < GS_KA / 4; ++i) {
-                const int chunk = (hf * (GS_KA / 4) + i) ^ (row & 7);
-                const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(brow + st * GS_B_BYTES + chunk * 16);
-                b2[2 * i]     = v.x;
-                b2[2 * i + 1] = v.y;
-            }
             const int buf = s % S::NB, before = s - S::NB;
             if (before >= 0) wait(done(before % GS_DONE), (before / GS_DONE) & 1);
             __syncwarp();
             tc::fence_after_sync();
 #pragma unroll
-            for (int i = 0; i < MT; i += 2) {
-                uint32_t w[16];
+            for (int h = 0; h < S::HALVES; ++h) {
+                const int hf = hf0 + h;
+                u64 b2[GS_KA / 2];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) w[j] = sign_pair(sub2(dd[i + (j >> 3)], b2[j & 7]));
-                tc::st_32x32b_x16(t_row + buf * S::A_COLS + i * (GS_KA / 2), w);
+                for (int i = 0; i < GS_KA / 4; ++i) {
+                    const int chunk = (hf * (GS_KA / 4) + i) ^ (row & 7);
+                    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(brow + st * GS_B_BYTES + chunk * 16);
+                    b2[2 * i]     = v.x;
+                    b2[2 * i + 1] = v.y;
+                }
+#pragma unroll
+                for (int i = 0; i < MT; i += 2) {
+                    uint32_t w[16];
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) w[j] = sign_pair(sub2(dd[i + (j >> 3)], b2[j & 7]), signs);
+                    tc::st_32x32b_x16(t_row + buf * S::A_COLS + (hf * MT + i) * (GS_KA / 2), w);
+                }
             }
             tc::wait_st();
             tc::fence_before_sync();
@@ -230,9 +261,9 @@ grad_sign_kernel(const __grid_constant__ GradTensorParams p, const __grid_consta
                 mbar_arrive(afull(buf));
             }
         }
-    } else if (warp < GS_GEN + S::PROD) {
+    } else if (warp < S::GEN + S::PROD) {
         // ------------------------------------------------------------------ split products
-        const int pw  = warp - GS_GEN;
+        const int pw  = warp - S::GEN;
         const int o   = OT >= 8 ? (pw % S::OCTS) * 8 + (lane >> 2) : ((lane >> 2) & (OT - 1));
         const int kc  = lane & 3;                                   // eight k of the slab
         const int mi0 = (pw / S::OCTS) * S::MSUB + (OT >= 8 ? 0 : (lane >> 2) / OT);
