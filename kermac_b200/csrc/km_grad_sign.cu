@@ -16,8 +16,8 @@
 //   8 to 16 generating warps (2 to 4 groups of 4): a thread owns one row n (a tensor-memory lane); a group takes
 //      every second to fourth slab of 32 k, or 16 k of every second one, reads them once for all m and writes the signs
 //      (8 columns of packed bf16 pairs per m and 16 k) with tcgen05.st into a ring of A buffers, one slab each;
-//   8 product warps (4 with few channels): P_m for the slab, split and parked in shared memory as the B operand (K-major rows
-//      of 64 bytes, 64-byte swizzle; row = piece * OT + channel);
+//   2 to 8 product warps in two groups that take the slabs in turn: P_m for the slab, split and parked in shared memory as
+//      the B operand (K-major rows of 64 bytes, 64-byte swizzle; row = piece * OT + channel);
 //   2 warps (4 with few channels) issue the MMAs, one accumulator of 3 OT columns (rounded up to 16) per m;
 //   4 draining warps: the tensor core truncates when it accumulates, so a chain is cut every 512 k (32
 //      MMAs), read back and added, rounding to nearest, to running sums in shared memory; the cuts of the
@@ -29,17 +29,17 @@
 // The product warps have no global loads of their own: their fence to the asynchronous units waits for
 // every memory operation of the thread, and behind loads in flight it made each slab as long as a load.
 // What bounds it (B200, K = 30000, M = 4096, N = 256; ms, in brackets the kernel that took these calls before):
-// 4 channels 4.61 (6.2), 8: 4.84 (10.6), 16: 7.64 (20.3), 32: 9.68 (22.0).
+// 4 channels 4.31 (6.2), 8: 4.72 (10.6), 16: 7.14 (20.3), 32: 8.91 (22.0).
 // The MMAs alone would take 2.5 ms at 32 channels (an MMA of 128 rows x N columns holds the tensor pipe N / 2 cycles,
 // also with the stores to tensor memory beside it), the ALU pipe (permutes and logic, half rate) about 3.5.  Instructions are
-// what the rest goes to: at 4 channels the generating warps rest for 16 % of a slab, at 32 the product warps for 25 %, each
-// warp issuing once in about nine cycles beside the others, and the hand-overs are a third of what is issued.  On the way
+// what the rest goes to: at 4 channels the generating warps hardly rest, at 32 the product warps, each warp issuing once in five to
+// nine cycles beside the others, and the hand-overs are a third of what is issued.  On the way
 // here (ms at 4 / 32 channels): one thread issuing all MMAs 18.5 / -; every role handing over per 16 k by its own
 // barrier, four issuing warps 6.7 / 14.5; global loads taken from the product warps 7.0 / 14.2; eight product warps
 // and carried copy addresses 7.5 / 12.4; all MMAs of a slab in one elected block 6.2 / 11.9; 16 k of all eight m
 // per group and slab instead of four 5.5 / 11.9; pieces scaled 5.5 / 12.1; infinite and NaN products left to the sums
 // (bf16_joined) instead of being looked for in each product 5.25 / 11.3; the constants of sign_pair in registers 4.6 / 10.9;
-// whole slabs for a group 4.6 / 9.7.
+// whole slabs for a group of generating warps 4.6 / 9.6; two groups of product warps 4.3 / 9.2; sleeping waits - / 8.9.
 // Hand-over is by mbarriers, one round per slab; every wait is bounded, and a wait that runs out sets a
 // flag (kermac_b200_device_error_flag) and lets the block run to its end without its results.
 #include <cstring>
@@ -74,17 +74,25 @@ struct GsShape {
     // Groups of four generating warps, and how many of the two halves of a slab's k a group takes.  Whole slabs mean half
     // as many hand-overs, each some 65 instructions a warp against 96 (4 m) or 192 (8 m) for the signs of a half; they pay
     // where there are as many A buffers as groups, or with fewer groups.  Measured at K = 30000, M = 4096, N = 256, ms:
-    //   groups x halves   4 x 1    2 x 2    3 x 2    4 x 2
+    //   groups x halves   4 x 1    2 x 2    3 x 2    4 x 2      (one group of product warps)
     //   4 channels        4.61     4.92     5.06     4.73
     //   8                 5.37     4.84     4.88     4.89
     //   16                8.10     8.14     8.22     7.64
-    //   32               10.87     9.80     9.68    10.04
-    static constexpr int GROUPS    = OT == 8 ? 2 : OT == 32 ? 3 : 4;
+    //   32               10.87     9.80     9.68    10.04       (with two groups 2 x 2 9.20, 3 x 2 9.35)
+    static constexpr int GROUPS    = OT == 8 || OT == 32 ? 2 : 4;
     static constexpr int HALVES    = OT == 4 ? 1 : 2;
-    // product warps, and warps that issue MMAs (two MMAs per accumulator and slab): with few channels there are more
-    // accumulators and fewer products.  (Half or twice as many product warps: 32 channels 11.6 / 11.7 ms, 8 channels
-    // 6.1 / 5.2; half as many issuing warps: 4 to 16 channels 6.1 / 5.0 / 9.3.)
-    static constexpr int PROD      = OT >= 16 ? 8 : 4;
+    // Product warps in groups that take every PGROUPS-th slab: a wait for a phase that is long complete costs such a warp
+    // 180 cycles and the fence behind its stores about as much, so it is better off with more products between them.
+    //   warps x groups   one group  2 x 2   4 x 2   8 x 2   3 x 3   6 x 3   12 x 3
+    //   4 channels       4.61 (4)   4.31    4.51            4.38    4.36
+    //   8                4.86 (4)   5.86    4.73    4.98    5.88    4.75
+    //   16               7.62 (8)           7.13    7.15            7.85
+    //   32               9.63 (8)                   9.20                    9.15 (sums of 8192 k and less: 8 x 2)
+    static constexpr int PROD      = OT == 4 ? 2 : OT == 32 ? 8 : 4;
+    static constexpr int PGROUPS   = 2;
+    static constexpr int PWARPS    = PROD / PGROUPS;
+    // warps that issue MMAs (two MMAs per accumulator and slab): with few channels there are more accumulators
+    // (half as many: 4 / 8 / 16 channels 6.1 / 5.0 / 9.3 ms)
     static constexpr int ISSUERS   = OT >= 16 ? 2 : 4;
     static constexpr int GEN       = 4 * GROUPS;
     static constexpr int WARPS     = GEN + PROD + GS_DRAIN + ISSUERS + 2;
@@ -177,9 +185,9 @@ grad_sign_kernel(const __grid_constant__ GradTensorParams p, const __grid_consta
         }
         for (int sl = 0; sl < GS_AC_SLOTS; ++sl) {
             mbar_init(acfull(sl), 32);
-            mbar_init(acempty(sl), S::PROD);
+            mbar_init(acempty(sl), S::PWARPS);
         }
-        for (int sl = 0; sl < GS_P_SLOTS; ++sl) mbar_init(pfull(sl), S::PROD);
+        for (int sl = 0; sl < GS_P_SLOTS; ++sl) mbar_init(pfull(sl), S::PWARPS);
         for (int b = 0; b < S::NB; ++b) mbar_init(afull(b), 8 / S::HALVES);
         for (int i = 0; i < GS_DONE; ++i) mbar_init(done(i), S::ISSUERS);
         for (int m = 0; m < MT; ++m) {
@@ -202,7 +210,9 @@ grad_sign_kernel(const __grid_constant__ GradTensorParams p, const __grid_consta
     // (One lane waiting for its warp instead of all 32 was three times slower in all.)
     auto wait = [&](uint32_t bar, int parity) {
         // once a wait has run out this warp stops waiting: a stuck barrier costs one limit, not one per slab
-        if (!expired && !mbar_wait_bounded(bar, parity)) {
+        // (sleeping: 32 channels 9.19 -> 8.91 ms, where the generating warps rest three quarters of the time; 4 channels
+        // 4.31 -> 4.48, 16 on unaligned rows 2.23 -> 2.26)
+        if (!expired && !(OT == 32 ? mbar_sleep_bounded(bar, parity) : mbar_wait_bounded(bar, parity))) {
             expired = true;
             *reinterpret_cast<volatile int*>(&s_expired) = 1;
         }
@@ -263,13 +273,13 @@ grad_sign_kernel(const __grid_constant__ GradTensorParams p, const __grid_consta
         }
     } else if (warp < S::GEN + S::PROD) {
         // ------------------------------------------------------------------ split products
-        const int pw  = warp - S::GEN;
+        const int pw  = (warp - S::GEN) % S::PWARPS;
         const int o   = OT >= 8 ? (pw % S::OCTS) * 8 + (lane >> 2) : ((lane >> 2) & (OT - 1));
         const int kc  = lane & 3;                                   // eight k of the slab
         const int mi0 = (pw / S::OCTS) * S::MSUB + (OT >= 8 ? 0 : (lane >> 2) / OT);
-        constexpr int MSTEP = (S::PROD / S::OCTS) * S::MSUB;
+        constexpr int MSTEP = (S::PWARPS / S::OCTS) * S::MSUB;
         static_assert(MT % MSTEP == 0, "every product warp takes the same number of m");
-        for (int s = 0; s < nslabs; ++s) {
+        for (int s = (warp - S::GEN) / S::PWARPS; s < nslabs; s += S::PGROUPS) {
             const int ac = s % GS_AC_SLOTS;
             wait(acfull(ac), (s / GS_AC_SLOTS) & 1);
             const int slot = s % GS_P_SLOTS, before = s - GS_P_SLOTS;

@@ -49,6 +49,20 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, int parity, int 
         if (mbar_try_wait(bar, parity)) return true;
     return false;
 }
+// The same as one loop of four instructions whose attempts may each sleep for a microsecond: for warps that wait long
+// beside others that have much to issue.
+__device__ __forceinline__ bool mbar_sleep_bounded(uint32_t bar, int parity, int tries = MBAR_WAIT_TRIES) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\tmov.u32 n, %3;\n"
+        "AGAIN:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, 1000;\n\t"
+        "@p bra DONE;\n\tsub.u32 n, n, 1;\n\tsetp.ne.u32 q, n, 0;\n\t@q bra AGAIN;\n"
+        "DONE:\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity), "r"(tries)
+        : "memory");
+    return done != 0;
+}
 // Tiled TMA copy (no multicast) of one box of a rank-3 tensor into shared memory; the
 // mbarrier receives the byte count.  x is the innermost coordinate: x * 4 bytes must be a
 // multiple of 16.
