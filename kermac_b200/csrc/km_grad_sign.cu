@@ -24,8 +24,8 @@
 //      MT accumulators are staggered, so the MMAs of the others keep the pipe busy meanwhile;
 //   1 warp copies slabs of a (transposed) and c into shared memory;
 //   1 warp brings the 128 x 32 slabs of b into shared memory (128-byte swizzle, so the
-//      16-byte reads of 32 different rows do not collide): a TMA copy when the rows of b are 16-byte
-//      aligned, 4-byte cp.async otherwise, same bits either way.
+//      16-byte reads of 32 different rows do not collide) by TMA when the rows of b are 16-byte
+//      aligned, 4 warps by 4-byte cp.async otherwise, same bits either way.
 // The product warps have no global loads of their own: their fence to the asynchronous units waits for
 // every memory operation of the thread, and behind loads in flight it made each slab as long as a load.
 // What bounds it (B200, K = 30000, M = 4096, N = 256; ms, in brackets the kernel that took these calls before):
@@ -95,7 +95,9 @@ struct GsShape {
     // (half as many: 4 / 8 / 16 channels 6.1 / 5.0 / 9.3 ms)
     static constexpr int ISSUERS   = OT >= 16 ? 2 : 4;
     static constexpr int GEN       = 4 * GROUPS;
-    static constexpr int WARPS     = GEN + PROD + GS_DRAIN + ISSUERS + 2;
+    // warps that bring slabs of b: one with TMA, four that copy a quarter of the rows each without
+    static constexpr int BWARPS    = TMA ? 1 : 4;
+    static constexpr int WARPS     = GEN + PROD + GS_DRAIN + ISSUERS + 1 + BWARPS;
     static constexpr int THREADS   = 32 * WARPS;
     static constexpr int AC_FLOATS = MT * GS_BK + OT * GS_C_PITCH;
     static constexpr int OFF_B     = 0;                                // shared memory, from a 1024-byte boundary
@@ -180,7 +182,7 @@ grad_sign_kernel(const __grid_constant__ GradTensorParams p, const __grid_consta
 
     if (tid == 0) {
         for (int st = 0; st < GS_B_STAGES; ++st) {
-            mbar_init(bfull(st), TMA ? 1 : 32);
+            mbar_init(bfull(st), TMA ? 1 : 32 * S::BWARPS);
             mbar_init(bempty(st), 8 / S::HALVES);      // a slab is read by one or two groups of four warps
         }
         for (int sl = 0; sl < GS_AC_SLOTS; ++sl) {
@@ -514,14 +516,16 @@ grad_sign_kernel(const __grid_constant__ GradTensorParams p, const __grid_consta
             }
             __syncwarp();
         } else {
-            const int rows     = min(GS_TN, p.N - n0);
-            const float* b_src = p.B + (long long)l * p.b_sl + (long long)n0 * p.ldb + k_begin + lane;
+            constexpr int ROWS = GS_TN / S::BWARPS;
+            const int first    = (warp - (MMA_WARP + S::ISSUERS + 1)) * ROWS;
+            const int rows     = max(0, min(ROWS, p.N - n0 - first));
+            const float* b_src = p.B + (long long)l * p.b_sl + (long long)(n0 + first) * p.ldb + k_begin + lane;
             for (int s = 0; s < nslabs; ++s) {
                 const int st = s % GS_B_STAGES;
                 if (s >= GS_B_STAGES) wait(bempty(st), (s / GS_B_STAGES - 1) & 1);
                 __syncwarp();
                 const bool k_ok    = k_begin + s * GS_BK + lane < k_end;
-                const uint32_t dst = base + S::OFF_B + st * GS_B_BYTES + (lane & 3) * 4;
+                const uint32_t dst = base + S::OFF_B + st * GS_B_BYTES + first * 128 + (lane & 3) * 4;
                 const float* src   = k_ok ? b_src : p.B;
                 const int bytes    = k_ok ? 4 : 0;
                 const long long step = k_ok ? p.ldb : 0;
