@@ -77,50 +77,49 @@ def _e2e(host_inputs, run_on_device, out_host, steps, barrier, max_over_ranks):
 
 
 # ------------------------------------------------------------------ fractional p: a two-pipe bound
-# Per (m, n, k) element the |b - a|^p step has two routes (kermac_b200/csrc/km_common.cuh, inner_block):
-#   all-MUFU    sub, lg2 (MUFU), mul by p, ex2 (MUFU), add         3 FP32-pipe lane-ops, 2 MUFU, 5 issue slots
-#   polynomial  sub, lg2 (MUFU), mul by p, 2 clamps (ALU), add/sub/sub to split off the integer part,
-#               5 fma of the polynomial, 1 shift (ALU), 1 fma into the sum
-#                                                                   11 FP32-pipe lane-ops, 1 MUFU, 15 issue slots
-# With a share x of the elements on the polynomial route the kernel cannot be faster than
-#   t(x) = max( (2 - x) / MUFU rate,  (5 + 10 x) / issue rate )      per element
-# (the FP32 pipe itself, (3 + 8 x) / lane rate, is always below the issue term).  The bound is the
-# minimum of t over x; operand loads and the epilogue come on top and are not counted.
-POW_ISSUE_SLOTS = (5.0, 15.0)        # all-MUFU, polynomial
-POW_MUFU_OPS = (2.0, 1.0)
-POW_POLY_SHARE = 6.0 / 8.0           # KM_POW_POLY_EIGHTHS / 8 of the build kernels as compiled
+# Per (m, n, k) element the |b - a|^p step has two routes (kermac_b200/csrc/km_common.cuh, pow_block):
+#   MUFU    sub, lg2 (MUFU), mul by p, ex2 (MUFU), add                        3 FP32-pipe lane-ops, 2 MUFU
+#   table   sub, 3 bit operations (ALU), 1 shared-memory load, 1 fma that scales to [1, 2), 6 fma of the
+#           polynomial, 1 fma into the sum                                    9 FP32-pipe lane-ops, 0 MUFU
+# With a share x of the elements on the table route the kernel cannot be faster than
+#   t(x) = max( 2 (1 - x) / MUFU rate,  (3 + 6 x) / FP32 lane rate )          per element
+# The bound is the minimum of t over x.  Not counted: operand loads, the epilogue, issue slots (3.5 and 8.25 an
+# element), and that most of the packed FMAs have three different sources, which takes them about three cycles
+# of the pipe instead of two.
+POW_LANE_OPS = (3.0, 9.0)            # MUFU route, table route
+POW_MUFU_OPS = (2.0, 0.0)
+POW_TABLE_SHARE = 8.0 / 16.0         # of the 128 x 128 build kernel as compiled (pow_mufu_sixteenths)
 
 
-def pow_two_pipe_seconds(x, issue_rate, mufu_rate):
-    """Model time per element for a polynomial share x (rates in lane-slots and MUFU ops per second)."""
+def pow_two_pipe_seconds(x, lane_rate, mufu_rate):
+    """Model time per element for a table share x (rates in FP32 lane-ops and MUFU ops per second)."""
     mufu = (POW_MUFU_OPS[0] * (1.0 - x) + POW_MUFU_OPS[1] * x) / mufu_rate
-    issue = (POW_ISSUE_SLOTS[0] * (1.0 - x) + POW_ISSUE_SLOTS[1] * x) / issue_rate
-    return max(mufu, issue), mufu, issue
+    lane = (POW_LANE_OPS[0] * (1.0 - x) + POW_LANE_OPS[1] * x) / lane_rate
+    return max(mufu, lane), mufu, lane
 
 
-def fractional_roofline(elements, seconds, pipes, share=POW_POLY_SHARE):
+def fractional_roofline(elements, seconds, pipes, share=POW_TABLE_SHARE):
     """Roofline dict for `elements` (m, n, k) element-steps of |b - a|^p done in `seconds`."""
-    issue_rate = pipes.lane_scalar        # one warp instruction per clock and scheduler = 32 lane-slots
     best_x, best_t = 0.0, float("inf")
     for i in range(0, 1001):
         x = i / 1000.0
-        t = pow_two_pipe_seconds(x, issue_rate, pipes.mufu)[0]
+        t = pow_two_pipe_seconds(x, pipes.lane, pipes.mufu)[0]
         if t < best_t:
             best_x, best_t = x, t
-    t_used, t_mufu, t_issue = pow_two_pipe_seconds(share, issue_rate, pipes.mufu)
+    t_used, t_mufu, t_lane = pow_two_pipe_seconds(share, pipes.lane, pipes.mufu)
     per_element = seconds / elements
     return {
-        "bound": "mufu+issue (two pipes)",
+        "bound": "mufu+fp32 (two pipes)",
         "achieved": 1.0 / per_element / 1e12, "peak": 1.0 / best_t / 1e12, "unit": "T element-steps/s",
         "frac": best_t / per_element,
-        "peak_source": "min over the polynomial share x of max((2-x)/MUFU rate, (5+10x)/issue rate), both rates "
+        "peak_source": "min over the table share x of max(2(1-x)/MUFU rate, (3+6x)/FP32 lane rate), both rates "
                        "measured on this device by kermac_b200_measure_pipe",
         "model_best_share": best_x, "share_in_use": share,
         "frac_of_model_at_share_in_use": t_used / per_element,
-        "limiting_pipe_at_share_in_use": "issue" if t_issue >= t_mufu else "mufu",
+        "limiting_pipe_at_share_in_use": "fp32" if t_lane >= t_mufu else "mufu",
         "all_mufu_bound_ratio": (2.0 / pipes.mufu) / per_element,
-        "mufu_utilisation": (POW_MUFU_OPS[0] * (1 - share) + POW_MUFU_OPS[1] * share) / pipes.mufu / per_element,
-        "issue_utilisation_model": (POW_ISSUE_SLOTS[0] * (1 - share) + POW_ISSUE_SLOTS[1] * share) / issue_rate / per_element,
+        "mufu_utilisation": t_mufu / per_element,
+        "fp32_utilisation_model": t_lane / per_element,
         "traffic": None,
     }
 

@@ -203,8 +203,11 @@ __global__ void __launch_bounds__(G_THREADS, grad_min_blocks(OT, NT)) grad_kerne
         //   p = 1.5: 0: 8.72   1: 8.82   3: 8.66        p = 1.7: 0: 14.84  1: 15.78  3: 15.06
         // With the two multiplicands exchanged (weight first, coefficient second) order 1 falls back to 6.9 ms:
         // what pays is the FIRST source repeating over a long run of instructions (the coefficient pair over
-        // all 8 weights of the row).  Other channel tiles measured no difference and keep order 0.
-        constexpr int ORDER = (OT != 4) ? 0 : (NORM == KM_NORM_L1 ? 1 : ((NORM == KM_NORM_L2 || NORM == G_NORM_SQRT) ? 3 : 0));
+        // all 8 weights of the row).  With 8 and 16 channels a coefficient pair still meets 4 and 2 weights (orders 0 / 1 / 3,
+        // us, K = 4000, M = 2000, N = 256): 16 channels, p = 2 1442 / 1349 / 1444, p = 1.5 1442 / 1437 / 1442; K = 64,
+        // 1000^2, p = 2 56.2 / 52.1 / 56.8, p = 1.7 60.1 / 58.8 / 60.6; 8 channels, p = 1.5 896 / 880 / 890, p = 2 719 / 723 /
+        // 745.  1 and 2 channels measured no difference and keep order 0.
+        constexpr int ORDER = OT >= 8 ? (OT == 8 && NORM == KM_NORM_L2 ? 0 : 1) : (OT != 4) ? 0 : (NORM == KM_NORM_L1 ? 1 : ((NORM == KM_NORM_L2 || NORM == G_NORM_SQRT) ? 3 : 0));
         if constexpr (ORDER == 0) {
 #pragma unroll
         for (int j = 0; j < NT; ++j) {
@@ -450,7 +453,7 @@ int preferred_split(const GradPlan& plan, int norm_type, bool square_root) {
 
 // What the kernels of the p = 1 gradient take, us: a slab of 32 k and the rest of a block (its set-up, first slabs, last
 // sums and stores); what rows of the result that cannot be stored 16 bytes at a time add to the latter, and rows of b or
-// c that cannot be copied 16 bytes at a time to the former (one warp of the sign kernel then copies 128 rows of b word by
+// c that cannot be copied 16 bytes at a time to the former (warps of the sign kernel then copy 128 rows of b word by
 // word).  Fitted on B200 to 10558 calls (K 256 to 30000, M 9 to 4096, N 64 to 1000, O 1 to 64): 95 % of a kernel's calls
 // are within 8 to 20 % of estimated_us().
 struct P1Cost {
