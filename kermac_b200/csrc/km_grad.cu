@@ -455,17 +455,20 @@ int preferred_split(const GradPlan& plan, int norm_type, bool square_root) {
 // sums and stores); what rows of the result that cannot be stored 16 bytes at a time add to the latter, and rows of b or
 // c that cannot be copied 16 bytes at a time to the former (warps of the sign kernel then copy 128 rows of b word by
 // word).  Fitted on B200 to 10558 calls (K 256 to 30000, M 9 to 4096, N 64 to 1000, O 1 to 64): 95 % of a kernel's calls
-// are within 8 to 20 % of estimated_us().
+// are within 8 to 20 % of estimated_us().  The sign kernel's numbers were then lowered with its instructions, by less than its times
+// fell (a slab 0.66, 0.73, 0.55 and 0.69; words 0.16 to 0.45), so that calls that were measured level stay where they
+// are.  Of 6000 calls of the same ranges 580 changed, by 1.18 in the geometric mean; 301 are faster by more than 2 %, 34
+// slower, two of them by more than 5 % (15 us calls).
 struct P1Cost {
     double slab, block, ragged, words;
 };
 P1Cost p1_cost(const GradPlan& plan) {
     if (plan.sign) {
         switch (plan.ot) {
-            case 4: return {0.80, 5.3, 0.5, 0.63};
-            case 8: return {0.89, 6.7, 1.6, 0.53};
-            case 16: return {0.66, 5.1, 1.8, 0.64};
-            default: return {0.87, 7.8, 3.3, 0.66};
+            case 4: return {0.77, 5.3, 0.5, 0.25};
+            case 8: return {0.74, 6.7, 1.6, 0.20};
+            case 16: return {0.56, 5.1, 1.8, 0.56};
+            default: return {0.74, 8.2, 5.0, 0.55};
         }
     }
     if (plan.tensor) return plan.ot == 16 ? P1Cost{1.50, 3.1, 0.3, 0.0} : plan.ot == 32 ? P1Cost{1.67, 5.9, 0.3, 0.0} : P1Cost{1.17, 5.9, 0.3, 0.0};
@@ -504,13 +507,14 @@ double estimated_us(const GradPlan& plan, const KmGradArgs* a, long long sms, lo
 // and is alone on its SM, so short sums lose what many k win.  Measured on B200, us, sign kernel against the other one
 // (FP32 up to 16 channels, weights from 17 on):
 //   K      M     N     O    sign   other         K      M     N     O    sign   other
-//   256    4096  1000  4    353    224           256    1000  1000  16   150    189
-//   320    4096  1000  4    396    277           1024   1000  1000  4    216    253
-//   256    4096  128   4    52     37            1024   1000  64    32   72     62
-//   512    250   500   64   117    108           8192   1000  1000  16   2377   5577
-//   30000  4096  256   2    5250   4460          30000  4096  256   4    5250   6240
-//   30000  4096  256   32   11310  22000         8192   1000  64    4    212    129
-//   8192   1000  1000  4    2506   1727 (b and c in rows that are not 16-byte aligned; 1457 where they are)
+//   256    4096  1000  4    328    222           256    1000  1000  16   139    189
+//   320    4096  1000  4    365    275           1024   1000  1000  4    189    260
+//   256    4096  128   4    48     36            8192   1000  1000  16   1985   5458
+//   512    250   500   64   101    107           8192   1000  1000  4    1202   1724
+//   30000  4096  256   2    4303   4443          30000  4096  256   4    4309   6226
+//   30000  4096  256   32   8902   22000         30000  4096  256   64   18100  29500
+//   8192   1000  1000  4    1497   1723 (b and c in rows that are not 16-byte aligned)
+// (Ties are left to the other kernel.)
 // Its split of k stays within the one that callers were told of (see kermac_b200_cdist_grad_scratch_bytes).
 void consider_sign(const KmGradArgs* a, GradPlan* plan) {
     if (a->norm_type != KM_NORM_L1 || a->contraction == KM_CONTRACT_FP32 || plan->partial_elems == 0) return;
