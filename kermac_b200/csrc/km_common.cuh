@@ -239,7 +239,7 @@ __device__ __forceinline__ void cp_async_wait() {
 // kernel_matvec 10007 x 1009 x 27 rows (three launches) 49.2 -> 43.7, cdist_grad 64 x 1000^2, 16 channels 57.1 -> 54.2.
 // No kernel lets the next one in before its own end (griddepcontrol.launch_dependents): the next grid's blocks then go to
 // whatever SMs have a place free, and a grid of fewer blocks than there are places ends up two on one SM and none on
-// another (a matvec of 112 blocks 58.5 -> 80 us, drawn calls of 6.7 and 28.7 us 9.8 and 37.1).
+// another (a matvec of 112 blocks 58.5 -> 80 us, gradients of 6.7 and 28.7 us 9.8 and 37.1).
 __device__ __forceinline__ void after_previous_grid() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Reads a hyper-parameter for batch entry l.

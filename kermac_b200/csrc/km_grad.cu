@@ -456,9 +456,9 @@ int preferred_split(const GradPlan& plan, int norm_type, bool square_root) {
 // c that cannot be copied 16 bytes at a time to the former (warps of the sign kernel then copy 128 rows of b word by
 // word).  Fitted on B200 to 10558 calls (K 256 to 30000, M 9 to 4096, N 64 to 1000, O 1 to 64): 95 % of a kernel's calls
 // are within 8 to 20 % of estimated_us().  The sign kernel's numbers were then lowered with its instructions, by less than its times
-// fell (a slab 0.66, 0.73, 0.55 and 0.69; words 0.16 to 0.45), so that calls that were measured level stay where they
-// are.  Of 6000 calls of the same ranges 580 changed, by 1.18 in the geometric mean; 301 are faster by more than 2 %, 34
-// slower, two of them by more than 5 % (15 us calls).
+// fell (a slab to 0.66, 0.73, 0.55 and 0.69; words to 0.16 to 0.45), so that calls that were measured level stay where they
+// are.  Of 6000 calls of the same ranges 475 changed, by 1.22 in the geometric mean; 338 are faster by more than 2 %, 12
+// slower, one of them by more than 5 % (15 us).
 struct P1Cost {
     double slab, block, ragged, words;
 };
@@ -468,7 +468,7 @@ P1Cost p1_cost(const GradPlan& plan) {
             case 4: return {0.77, 5.3, 0.5, 0.25};
             case 8: return {0.74, 6.7, 1.6, 0.20};
             case 16: return {0.56, 5.1, 1.8, 0.56};
-            default: return {0.74, 8.2, 5.0, 0.55};
+            default: return {0.84, 7.8, 3.6, 0.50};
         }
     }
     if (plan.tensor) return plan.ot == 16 ? P1Cost{1.50, 3.1, 0.3, 0.0} : plan.ot == 32 ? P1Cost{1.67, 5.9, 0.3, 0.0} : P1Cost{1.17, 5.9, 0.3, 0.0};
