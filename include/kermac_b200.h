@@ -234,11 +234,12 @@ int kermac_b200_cdist_grad_static(const KmGradArgs* args, void* stream);
  * and regularization != 0 the value is 1 + regularization, which gives
  * y = (K + lambda I) c for a square K(X, X) without a second pass.
  *
- * contraction selects where the coefficient product runs: KM_CONTRACT_TENSOR (and
- * KM_CONTRACT_AUTO) on the tcgen05 tensor cores as three tf32 products per term
- * (operands split into a tf32 head and an fp32 remainder, fp32 accumulation: fp32-level
- * accuracy), KM_CONTRACT_FP32 as packed FP32 FMAs.  The kernel-matrix values are
- * computed in FP32 either way.
+ * contraction selects where the coefficient product runs: KM_CONTRACT_TENSOR on the
+ * tcgen05 tensor cores as three tf32 products per term (operands split into a tf32 head
+ * and an fp32 remainder, fp32 accumulation: fp32-level accuracy), KM_CONTRACT_FP32 as
+ * packed FP32 FMAs.  KM_CONTRACT_AUTO takes the tensor cores, except for |b - a| with one
+ * or two channels (up to four from 16 features on), where the FMAs are faster.  The
+ * kernel-matrix values are computed in FP32 either way.
  */
 #define KM_CONTRACT_AUTO   0
 #define KM_CONTRACT_FP32   1

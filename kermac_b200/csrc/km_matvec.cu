@@ -688,6 +688,18 @@ int preferred_split(const MatvecParams& p) {
     return cheapest_split(chunks, last, cost);
 }
 
+// Where KM_CONTRACT_AUTO leaves the coefficient product on the FP32 pipe: |b - a| with up to four channels.  Neither kernel
+// stages that step by TMA, and few channels cost less as packed FMAs than the split, the parking of two operand tiles and
+// the MMAs.  Measured on B200, tensor / FP32, us, O = 2, 4 and 8:
+//   16384^2 x 8: 384 / 366, 384 / 390, 387 / 452      16384^2 x 32: 783 / 723, 783 / 757, 785 / 814
+//   16384^2 x 256: 4958 / 4745, 4956 / 4756, 4953 / 4860      8000^2 x 500: 2297 / 2222, 2297 / 2221, 2297 / 2262
+//   10007 x 1009 x 27 rows: 57.3 / 50.5, 57.4 / 51.6, 57.7 / 56.8      600 x 100 x 12: 10.7 / 9.6, 11.0 / 9.9, 11.0 / 10.9
+// The square step, staged by TMA in the tensor-core kernel, is level or up to 7 % slower with FMAs (16384^2 x 64, O = 2: 1209 /
+// 1243).  By O and K alone, so that shards of the rows and other splits take the same kernel.
+bool fp32_contraction_preferred(const MatvecParams& p) {
+    return p.inner_id == IN_DIFF_ABS && (p.O <= 2 || (p.O <= 4 && p.K >= 16));
+}
+
 // How the operands are staged: 16-byte copies, and TMA where the inner step gains from it.
 void choose_staging(MatvecPlan* plan) {
     const MatvecParams& p = plan->p;
@@ -741,7 +753,8 @@ int make_matvec_plan(const KmMatvecArgs* a, MatvecPlan* plan) {
     p.regularization = a->regularization;
     p.reg_off_m = a->reg_off_x; p.reg_off_n = a->reg_off_y;
     p.epsilon = a->epsilon;
-    plan->tensor = (a->contraction != KM_CONTRACT_FP32);
+    plan->tensor = a->contraction == KM_CONTRACT_TENSOR ||
+                   (a->contraction == KM_CONTRACT_AUTO && !fp32_contraction_preferred(p));
     int ot = 2;
     while (ot < a->o && ot < 16) ot *= 2;
     if (plan->tensor) ot = MT_OT;

@@ -139,7 +139,8 @@ def kernel_matvec(
     added in a fixed order, so the result does not depend on scheduling.  `contraction`
     selects where the coefficient product runs: "tensor" (tcgen05 tensor cores, three tf32
     products per term, fp32-level accuracy), "fp32" (packed FP32 FMAs) or "auto" / None
-    (the environment variable KERMAC_B200_CONTRACTION, else the library default: tensor).
+    (the environment variable KERMAC_B200_CONTRACTION, else the library's choice: tensor, except
+    for |b - a| with one or two channels, or up to four from 16 features on, which are faster as FMAs).
 
     Partial sums (at most 512 MB unless `split_m` asks for more) and copies of points that are held as rows (at most
     1 GiB) take scratch from torch's allocator for the duration of the call.
