@@ -88,7 +88,7 @@ def _e2e(host_inputs, run_on_device, out_host, steps, barrier, max_over_ranks):
 # of the pipe instead of two.
 POW_LANE_OPS = (3.0, 9.0)            # MUFU route, table route
 POW_MUFU_OPS = (2.0, 0.0)
-POW_TABLE_SHARE = 8.0 / 16.0         # of the 128 x 128 build kernel as compiled (pow_mufu_sixteenths)
+POW_TABLE_SHARE = 8.0 / 16.0         # of the build kernels as compiled (POW_MUFU_SIXTEENTHS)
 
 
 def pow_two_pipe_seconds(x, lane_rate, mufu_rate):

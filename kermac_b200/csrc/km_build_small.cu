@@ -43,8 +43,14 @@ constexpr int SB_PITCH   = SB_TILE + 4;     // floats per staged k row without T
 // Resident blocks per SM the inner steps are compiled for.  Measured with 4 / 5 / 6 / 7 blocks (128 / 102 /
 // 85 / 73 registers): |.| 4000 x 4000 x 512 569 / 572 / 623 / 626 us and |.|^1.3 2048 x 2048 x 64 107 / 109 /
 // 115 / 116 us want the registers; the square is level (16384 x 16384 x 512 8247 / 8246 / 8178 / 8227 us).
+// The power by MUFU and table takes more registers still, for a slab loop unrolled by 4 (blocks x unroll x sixteenths of the
+// pairs on MUFU, us, p = 1.3):         4 x 4 x 7   4 x 1 x 8   4 x 2 x 8   3 x 2 x 8   3 x 4 x 8   5 x 4 x 7   4 x 8 x 7
+//   500 x 600 x 300, two of them         115.3       113.9                   112.6       109.4
+//   3000 x 1000 x 800 rows               828         823                     813         806
+//   8000^2 x 96 rows                     1730        1723        1735        1732        1709        1867        2059
+//   6000^2 x 200, with itself            1048        1064        1039        1041        1061        1134        1223
 constexpr int small_min_blocks(int inner) {
-    return (inner == IN_DIFF_ABS || inner == IN_DIFF_POW || inner == IN_DIFF_POW_TABLE) ? 4 : 6;
+    return inner == IN_DIFF_POW_TABLE ? 3 : (inner == IN_DIFF_ABS || inner == IN_DIFF_POW) ? 4 : 6;
 }
 
 __device__ int g_small_wait_expired = 0;

@@ -453,15 +453,14 @@ __device__ __forceinline__ void inner_block(u64 (&acc)[8][MP], const u64 (&ap)[M
 // A pair costs 32 MUFU cycles of a scheduler one way; the other way about 25 cycles of the FP32 pipe (nine packed
 // instructions, most with three different sources), 12 of the ALU and 16 issue slots.  Rows alternate, so both pipes
 // have work at any time.  Measured with 6 / 7 / 8 / 9 of 16 on MUFU: 2 x 16384^2 x 512, p = 1.3, 78.1 / 76.3 / 75.2 /
-// 82 ms (all of them lg2 on MUFU and six of eight ex2_poly2: 98.5); in the 64 x 64 kernel, unrolled by 4, 7 / 8:
-// 8000^2 x 96 rows 1730 / 1885 us (2260), 4000^2 x 512 rows 2301 / 2532 (3040).
-__host__ __device__ constexpr int pow_mufu_sixteenths(int mp_count) { return mp_count == 4 ? 8 : 7; }
+// 82 ms (all of them lg2 on MUFU and six of eight ex2_poly2: 98.5).
+constexpr int POW_MUFU_SIXTEENTHS = 8;
 template <int MP>
 __device__ __forceinline__ constexpr bool pow_pair_uses_mufu(int n, int mp) {
     constexpr int ROWS = 16 / MP;                              // rows of 16 pairs: even ones first
     const int r    = n % ROWS;
     const int rank = (r & 1) ? ROWS / 2 + (r >> 1) : (r >> 1);
-    return rank * MP + mp < pow_mufu_sixteenths(MP);
+    return rank * MP + mp < POW_MUFU_SIXTEENTHS;
 }
 
 // One k step of |b - a|^p, with the arguments of inner_block.
@@ -541,7 +540,7 @@ __device__ __forceinline__ void consume_slab(u64 (&acc)[8][MP], const float* sa,
     // of its rows.  The fractional-power step is ~30 instructions per element; unrolling it
     // that far would not fit the instruction cache, so it is unrolled by 2 only.  The one with the table is some 450
     // instructions a row of 32 pairs and is not unrolled at all there (2 x 16384^2 x 512, p = 1.3: 76.3 ms, by 2 85.6,
-    // by 4 84.4); in the 64 x 64 kernel, with half the pairs, by 4 (8000^2 x 96 rows: 1853, by 2 1816, by 4 1730 us).
+    // by 4 84.4); in the 64 x 64 kernel, with half the pairs, by 4 (table at small_min_blocks()).
     constexpr int UNROLL = INNER == IN_DIFF_POW_TABLE ? (MP == 4 ? 1 : 4) : (INNER == IN_DIFF_POW || INNER == IN_DOT_POW) ? 2 : BK;
     if (kvalid >= BK) {
 #pragma unroll UNROLL
