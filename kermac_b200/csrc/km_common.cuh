@@ -230,11 +230,14 @@ __device__ __forceinline__ void cp_async_wait() {
 }
 
 // ---------------------------------------------------------------- overlapped launches
-// Kernels are launched with programmatic stream serialization (launch_overlapped): a grid's blocks start when the last
-// block of the kernel before it in the stream has ended, without waiting for the end of that kernel to be reported and
-// its writes to be flushed.  Their set-up (barriers, tensor memory, tables) runs meanwhile, and everything that touches
-// global memory stands behind after_previous_grid(), which returns when the grids before have completed and their
-// writes are visible.  Every block of every kernel passes it, also one that has nothing to do, so a grid completes only
+// Kernels are launched with programmatic stream serialization (launch_overlapped): a grid's blocks start when every block
+// of the kernel before it in the stream has ended or let its dependents in, without waiting for the end of that kernel to
+// be reported and its writes to be flushed.  Behind a kernel of this library that means its last block has ended (none
+// lets the next one in, see below); a library kernel may let these blocks in while its own are still at work.  The set-up
+// (barriers, tables) runs meanwhile, and everything that touches global memory stands behind after_previous_grid(), which
+// returns when the grids before have completed and their writes are visible.  So does the allocation of tensor memory: a
+// block of the kernel before that has still to allocate its own would wait for this one's, and this one for that block.
+// Every block of every kernel passes it, also one that has nothing to do, so a grid completes only
 // after the ones before it.  Back-to-back calls, us: cdist 128 x 96 x 10 6.1 -> 4.5, 2048^2 x 64 22.5 -> 20.2,
 // kernel_matvec 10007 x 1009 x 27 rows (three launches) 49.2 -> 43.7, cdist_grad 64 x 1000^2, 16 channels 57.1 -> 54.2.
 // No kernel lets the next one in before its own end (griddepcontrol.launch_dependents): the next grid's blocks then go to

@@ -202,11 +202,11 @@ grad_sign_kernel(const __grid_constant__ GradTensorParams p, const __grid_consta
         tc::fence_smem_to_async();
     }
     constexpr int MMA_WARP = S::GEN + S::PROD + GS_DRAIN;
+    after_previous_grid();
     if (warp == MMA_WARP) tc::tmem_alloc(smem_u32(&s_tmem), 512);
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    after_previous_grid();
     const uint32_t tmem = s_tmem;
     bool expired = false;
     // (One lane waiting for its warp instead of all 32 was three times slower in all.)

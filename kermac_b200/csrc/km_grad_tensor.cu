@@ -232,11 +232,11 @@ grad_tensor_kernel(const __grid_constant__ GradTensorParams p, const __grid_cons
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         tc::fence_smem_to_async();
     }
+    after_previous_grid();
     if (warp == S::GEN_WARPS) tc::tmem_alloc(smem_u32(&s_tmem), S::TMEM_COLS);
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    after_previous_grid();
     const uint32_t tmem = s_tmem;
     bool expired = false;
 

@@ -320,11 +320,11 @@ matvec_tensor_kernel(const __grid_constant__ MatvecParams p, const __grid_consta
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         tc::fence_smem_to_async();
     }
+    after_previous_grid();
     if (warp == 0) tc::tmem_alloc(smem_u32(&s_tmem), MT_TMEM_COLS);
     tc::fence_before_sync();
     __syncthreads();
     tc::fence_after_sync();
-    after_previous_grid();
     const float p_inner = (INNER == IN_DIFF_POW || INNER == IN_DOT_POW) ? read_hyper(p.p_inner, l) : 0.0f;
     const Epilogue epi  = make_epilogue(p.outer_power, p.kernel_type, p.p_outer, p.bandwidth, p.epsilon, l);
     const uint32_t tmem = __shfl_sync(0xFFFFFFFFu, s_tmem, 0);
