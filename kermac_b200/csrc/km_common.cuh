@@ -238,7 +238,8 @@ __device__ __forceinline__ void cp_async_wait() {
 // returns when the grids before have completed and their writes are visible.  So does the allocation of tensor memory: a
 // block of the kernel before that has still to allocate its own would wait for this one's, and this one for that block.
 // Every block of every kernel passes it, also one that has nothing to do, so a grid completes only
-// after the ones before it.  Back-to-back calls, us: cdist 128 x 96 x 10 6.1 -> 4.5, 2048^2 x 64 22.5 -> 20.2,
+// after the ones before it.  No pointer of such a kernel is __restrict__: what it points to may still be written when the
+// kernel starts, and a load from memory that is promised not to change may be moved in front of the wait.  Back-to-back calls, us: cdist 128 x 96 x 10 6.1 -> 4.5, 2048^2 x 64 22.5 -> 20.2,
 // kernel_matvec 10007 x 1009 x 27 rows (three launches) 49.2 -> 43.7, cdist_grad 64 x 1000^2, 16 channels 57.1 -> 54.2.
 // No kernel lets the next one in before its own end (griddepcontrol.launch_dependents): the next grid's blocks then go to
 // whatever SMs have a place free, and a grid of fewer blocks than there are places ends up two on one SM and none on

@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(G_THREADS, grad_min_blocks(OT, NT)) grad_kerne
 // reading the partials: indices are 32-bit wherever they fit, because the 64-bit divisions take longer than the
 // loads, and four splits are loaded ahead of the adds.
 template <typename Index>
-__global__ void __launch_bounds__(256) grad_reduce_kernel(const float* __restrict__ partial, float* __restrict__ out,
+__global__ void __launch_bounds__(256) grad_reduce_kernel(const float* partial, float* out,
                                                           int M, int N, int O, int L, int splits, long long split_stride,
                                                           long long o_sn, long long o_so, long long o_sl) {
     after_previous_grid();

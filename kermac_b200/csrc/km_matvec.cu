@@ -572,7 +572,7 @@ matvec_tensor_kernel(const __grid_constant__ MatvecParams p, const __grid_consta
     if (warp == 0) tc::tmem_dealloc(tmem, MT_TMEM_COLS);
 }
 
-__global__ void __launch_bounds__(256) matvec_reduce_kernel(const float* __restrict__ partial, float* __restrict__ y,
+__global__ void __launch_bounds__(256) matvec_reduce_kernel(const float* partial, float* y,
                                                             int N, int O, int L, int splits, long long split_stride,
                                                             long long y_sn, long long y_so, long long y_sl) {
     after_previous_grid();

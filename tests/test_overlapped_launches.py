@@ -38,3 +38,9 @@ def test_order_against_the_previous_grid(name, parameters, body):
     assert wait and "return;" not in before           # every block passes the wait
     # tensor memory is taken when the kernel before has given its own back
     assert "tmem_alloc" not in before
+
+
+@pytest.mark.parametrize("name, parameters, body", KERNELS, ids=[k[0] for k in KERNELS])
+def test_nothing_is_promised_to_stay_unwritten(name, parameters, body):
+    # the kernel before may still be writing what this one reads: loads must not move in front of the wait
+    assert "__restrict__" not in parameters + body and "__ldg" not in body
