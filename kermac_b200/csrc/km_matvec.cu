@@ -6,8 +6,8 @@
 // builds the 128 x 128 kernel-matrix tile exactly as the build kernel does (same
 // staging, same packed 8 x 8 register blocks, same outer chain and epsilon mask),
 // parks the tile in shared memory, and contracts it with the chunk's coefficients
-// c[o, m] into per-thread accumulators y[n, o..] that live in registers for the
-// whole walk.  The sum over m is therefore taken in a fixed order inside one block.
+// c[o, m]; the tile's sums are added to per-thread accumulators y[n, o..] that live in
+// registers for the whole walk.  The sum over m is therefore taken in a fixed order inside one block.
 // With split_m > 1 the m range is divided over several blocks whose partial sums go
 // to caller-provided scratch and are added in a fixed order by a second kernel.
 //
@@ -168,7 +168,12 @@ __global__ void __launch_bounds__(MV_THREADS, 2) matvec_kernel(const __grid_cons
                 }
             }
             __syncthreads();
+            // A tile's products are summed by themselves and added to the running sums once, so these are rounded M / 128
+            // times and not M times (131072 columns in one block, |b - a|, c = 1: largest error of a result 1.5e-5 -> 1.3e-6).
             if constexpr (OT >= 4) {
+                u64 ysum[OH / 2];
+#pragma unroll
+                for (int i = 0; i < OH / 2; ++i) ysum[i] = 0ull;
 #pragma unroll 2
                 for (int mm = 0; mm < MV_TILE; mm += 4) {
                     const float4 k4  = *reinterpret_cast<const float4*>(s_kt + cn * MV_KT_PITCH + mm);
@@ -178,16 +183,17 @@ __global__ void __launch_bounds__(MV_THREADS, 2) matvec_kernel(const __grid_cons
                         const u64 kd  = pack2(kv[e], kv[e]);
                         const u64* cp = reinterpret_cast<const u64*>(s_c + (mm + e) * OT + ch * OH);
 #pragma unroll
-                        for (int i = 0; i < OH / 2; ++i) yacc[i] = fma2(kd, cp[i], yacc[i]);
+                        for (int i = 0; i < OH / 2; ++i) ysum[i] = fma2(kd, cp[i], ysum[i]);
                     }
                 }
+#pragma unroll
+                for (int i = 0; i < OH / 2; ++i) yacc[i] = add2(yacc[i], ysum[i]);
             } else {
                 // OT == 2: one channel per thread half
-                float y0, y1;
-                unpack2(yacc[0], y0, y1);
+                float y0 = 0.0f;
 #pragma unroll 8
                 for (int mm = 0; mm < MV_TILE; ++mm) y0 = fmaf(s_kt[cn * MV_KT_PITCH + mm], s_c[mm * OT + ch], y0);
-                yacc[0] = pack2(y0, y1);
+                yacc[0] = add2(yacc[0], pack2(y0, 0.0f));
             }
             // the next chunk's epilogue overwrites s_kt / s_c only after the barrier at
             // the top of a later iteration, which every thread passes after this point
@@ -691,9 +697,11 @@ int preferred_split(const MatvecParams& p) {
 // Where KM_CONTRACT_AUTO leaves the coefficient product on the FP32 pipe: |b - a| with up to four channels.  Neither kernel
 // stages that step by TMA, and few channels cost less as packed FMAs than the split, the parking of two operand tiles and
 // the MMAs.  Measured on B200, tensor / FP32, us, O = 2, 4 and 8:
-//   16384^2 x 8: 384 / 366, 384 / 390, 387 / 452      16384^2 x 32: 783 / 723, 783 / 757, 785 / 814
-//   16384^2 x 256: 4958 / 4745, 4956 / 4756, 4953 / 4860      8000^2 x 500: 2297 / 2222, 2297 / 2221, 2297 / 2262
-//   10007 x 1009 x 27 rows: 57.3 / 50.5, 57.4 / 51.6, 57.7 / 56.8      600 x 100 x 12: 10.7 / 9.6, 11.0 / 9.9, 11.0 / 10.9
+//   16384^2 x 8: 381 / 366, 382 / 377, 385 / 447      16384^2 x 32: 782 / 721, 782 / 743, 784 / 805
+//   16384^2 x 256: 4950 / 4734, 4949 / 4765, 4950 / 4793      8000^2 x 500: 2293 / 2215, 2294 / 2225, 2294 / 2227
+//   10007 x 1009 x 27 rows: 55.4 / 48.3, 55.5 / 49.9, 55.8 / 55.4      600 x 100 x 12: 10.4 / 8.7, 10.2 / 9.0, 10.4 / 9.9
+// Its results are no further from 64 bits (131072 columns x 64, random coefficients, largest error over the largest entry, O = 2
+// and 4: automatic split 1.6e-6 / 7.9e-7 and 9.8e-7 / 4.8e-7, one block 3.2e-6 / 1.9e-6 and 2.2e-6 / 9.8e-7).
 // The square step, staged by TMA in the tensor-core kernel, is level or up to 7 % slower with FMAs (16384^2 x 64, O = 2: 1209 /
 // 1243).  By O and K alone, so that shards of the rows and other splits take the same kernel.
 bool fp32_contraction_preferred(const MatvecParams& p) {

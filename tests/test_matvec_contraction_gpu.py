@@ -26,3 +26,22 @@ def test_automatic_contraction(kernel, K, O, expect, layout):
     dist = diff.abs().sum(-1) if kernel == "l1" else diff.square().sum(-1).sqrt()
     want = torch.exp(-dist / K) @ c.double().t()
     assert (got["auto"].reshape(want.shape).double() - want).abs().max() <= 5e-5 * want.abs().max()
+
+
+@pytest.mark.parametrize("K, O", [(3, 1), (16, 2), (16, 4)])
+def test_a_long_sum_in_one_block_is_not_one_chain_of_roundings(K, O):
+    """131072 positive terms in one block, taken to the FP32 kernel by the rule above.  Summed tile by tile a running sum is
+    rounded 1024 times; as random walks those come to sqrt(1024 / 3) * 0.4 * 2^-24 = 4e-7 of it, and 4e-6 is ten times
+    that.  One chain over all terms is rounded 131072 times: 5e-6 in the mean and 1.5e-5 in the worst of these entries."""
+    M, N = 131072, 300
+    gen = torch.Generator().manual_seed(K + O)
+    a, b = torch.randn(M, K, generator=gen).cuda(), torch.randn(N, K, generator=gen).cuda()
+    c = (torch.rand(O, M, generator=gen) + 0.5).cuda()
+    want = torch.zeros(N, O, dtype=torch.float64, device="cuda")
+    for i in range(0, M, 8192):
+        dist = (b.double()[:, None] - a[i:i + 8192].double()[None]).abs().sum(-1)
+        want += torch.exp(-dist / (1.13 * K)) @ c[:, i:i + 8192].double().t()
+    got = {name: kermac.kernel_matvec(kermac.kernel_descriptor_laplace_l1, a, b, c, bandwidth=1.13 * K, split_m=1, contraction=name)
+           for name in ("auto", "fp32")}
+    assert torch.equal(got["auto"], got["fp32"])
+    assert (got["auto"].reshape(want.shape).double() - want).abs().max() <= 4e-6 * want.abs().max()
