@@ -18,6 +18,7 @@ int fail(int code, const char* fmt, ...) {
 
 int cuda_status(cudaError_t e, const char* what) {
     if (e == cudaSuccess) return 0;
+    cudaGetLastError();   // reported here, so no longer the runtime's last error, which a later launch would be checked against
     snprintf(g_last_error, sizeof(g_last_error), "%s: %s (%s)", what, cudaGetErrorString(e), cudaGetErrorName(e));
     return static_cast<int>(e);
 }

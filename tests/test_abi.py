@@ -116,6 +116,37 @@ def test_integration_sample_binding_matches_the_compiled_header(tmp_path):
     _assert_matches(layout, {"KmHyper": scope["KmHyper"], "KmBuildArgs": scope["KmBuildArgs"]}, "INTEGRATION.md")
 
 
+REFUSED_LAUNCH = r"""
+#include "km_abi.cu"
+// a runtime that refuses every launch and, as the real one, keeps the error until cudaGetLastError() takes it
+static cudaError_t last = cudaSuccess;
+extern "C" {
+cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t*, const void*, void**) { return last = cudaErrorInvalidConfiguration; }
+cudaError_t cudaGetLastError(void) { const cudaError_t e = last; last = cudaSuccess; return e; }
+const char* cudaGetErrorString(cudaError_t) { return "refused"; }
+const char* cudaGetErrorName(cudaError_t) { return "name"; }
+cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr, int) { *v = 10; return cudaSuccess; }
+cudaError_t cudaMemcpy2DAsync(void*, size_t, const void*, size_t, size_t, size_t, cudaMemcpyKind, cudaStream_t) { return cudaSuccess; }
+}
+static void kernel(int) {}
+int main() {
+    const int rc = km::cuda_status(km::launch_overlapped(kernel, dim3(1), 32, 0, nullptr, 1), "launch of kernel");
+    printf("%d %d %s\n", rc, (int)cudaGetLastError(), kermac_b200_last_error());
+}
+"""
+
+
+def test_a_refused_launch_is_reported_once(tmp_path):
+    """The error of a launch is the caller's return code; the next launch's check must not find it again."""
+    csrc = os.path.join(ROOT, "kermac_b200", "csrc")
+    (tmp_path / "refused.cpp").write_text(REFUSED_LAUNCH)
+    subprocess.run(["g++", "-std=c++17", "-I", csrc, "-I", os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include"),
+                    str(tmp_path / "refused.cpp"), "-o", str(tmp_path / "refused")], check=True)
+    out = subprocess.run([str(tmp_path / "refused")], check=True, capture_output=True, text=True).stdout
+    assert out.strip() == "9 0 launch of kernel: refused (name)"
+
+
 def _build_args(**kw):
     a = _native.KmBuildArgs()
     a.m, a.n, a.k, a.l = 4, 4, 4, 1
