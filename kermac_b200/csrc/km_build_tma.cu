@@ -328,7 +328,8 @@ __global__ void wait_expiry_selftest_kernel(int tries, int* gave_up) {
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    if (threadIdx.x == 0 && !mbar_wait_bounded(bar_addr, 0, tries)) {
+    // both forms of the wait have to give up
+    if (threadIdx.x == 0 && !mbar_wait_bounded(bar_addr, 0, tries) && !mbar_sleep_bounded(bar_addr, 0, tries)) {
         atomicExch(&g_tma_wait_expired, 1);
         if (gave_up) *gave_up = 1;
     }

@@ -49,8 +49,8 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t bar, int parity, int 
         if (mbar_try_wait(bar, parity)) return true;
     return false;
 }
-// The same as one loop of four instructions whose attempts may each sleep for a microsecond: for warps that wait long
-// beside others that have much to issue.
+// The same as one loop of four instructions whose attempts may each sleep for a microsecond (some four seconds in all): for
+// warps that wait long beside others that have much to issue.  `tries` is at least 1.
 __device__ __forceinline__ bool mbar_sleep_bounded(uint32_t bar, int parity, int tries = MBAR_WAIT_TRIES) {
     uint32_t done;
     asm volatile(

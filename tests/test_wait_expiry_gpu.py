@@ -1,6 +1,7 @@
 """The report path of a bounded device-side wait, made to run out on purpose and safely: a one-block
-kernel waits a thousand attempts on an mbarrier that nothing arrives at, gives up, raises the device
-error flag and ends (kermac_b200_selftest_wait_expiry).  No fault, no trap, no hang: the loop is
+kernel waits a thousand attempts on an mbarrier that nothing arrives at, in both forms of the wait (polling, and
+sleeping up to a microsecond an attempt), gives up, raises the device error flag and ends
+(kermac_b200_selftest_wait_expiry).  A wait that reports success raises no flag.  No fault, no trap, no hang: the loop is
 bounded by construction."""
 import pytest
 import torch
