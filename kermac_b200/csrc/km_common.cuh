@@ -155,7 +155,9 @@ __device__ __forceinline__ void ex2_poly2(float x0, float x1, u64& r, u64& scale
 //             infinity of the sign that the polynomial has there
 //   e = 255   an infinity times an infinity of its own sign, negated: f = -inf, T has the sign of the polynomial; a NaN
 //             stays one
-// The polynomial is within 3e-7 of m^p for exponents in [POW_MIN, POW_MAX], and within 1.5e-7 up to 3.5.
+// Evaluated in float the polynomial is within 3.5e-7 of m^p for exponents up to 2, 5e-7 up to 3 and 9e-7 up to POW_MAX (next to
+// m = 1, where its terms cancel; the interpolation alone is within 1e-7, the rest is the rounding of its coefficients and
+// of each step).  lg2 and ex2 on MUFU give 4e-7, 5e-7 and 6e-7 for such x, and 1e-6 to 2.4e-6 a few octaves away.
 constexpr int   POW_DEGREE = 6;
 constexpr int   POW_ENTRIES = 512;
 constexpr float POW_MIN = 1.01f, POW_MAX = 4.0f;

@@ -3,8 +3,10 @@ float64 and against the lg2 / ex2 route, which a p given as a tensor takes.
 
 Bounds.  On MUFU a term is 2^x, x = p lg2|d|: lg2.approx is within 2^-22 of lg2|d| between 1/2 and 2 and within 2^-22 of
 its size elsewhere, the product rounds by 2^-24 of x, ex2.approx by 2^-22 of the result, so a term is within
-2^-22 (ln 2 (1.25 |x| + p) + 1) of the power.  The table and its polynomial are within 4e-7, less than that.  Adding K positive
+2^-22 (ln 2 (1.25 |x| + p) + 1) of the power.  The table and its polynomial are within 3.5e-7 up to p = 2, 5e-7 up to 3 and 9e-7 up to 4
+(_polynomial_error), about as much as that leaves for |d| = 1 and less elsewhere.  Adding K positive
 terms rounds by at most K units of 2^-25 in the mean.  Raw sums are compared, so no outer power adds to it."""
+import numpy as np
 import pytest
 import torch
 
@@ -115,3 +117,45 @@ def test_infinite_and_undefined_differences():
     want = _exact(a, a, 1.3)                                 # inf - inf is NaN, 6e38 overflows
     assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), mufu.isinf())
     assert torch.equal(got.isnan(), mufu.isnan())
+
+
+def _polynomial_error(p, m):
+    """Largest relative error of the degree-6 polynomial through m^p at the Chebyshev nodes of [1, 2), its coefficients and
+    each step rounded to float32 (a product of two floats is exact in float64)."""
+    nodes = 1.5 + 0.5 * np.cos(np.pi * (np.arange(7) + 0.5) / 7)
+    c = np.polyfit(nodes - 1.5, nodes ** p, 6).astype(np.float32).astype(np.float64)
+    f = m - 1.5
+    q = np.full_like(f, c[0])
+    for coefficient in c[1:]:
+        q = (q * f + coefficient).astype(np.float32).astype(np.float64)
+    return np.abs(q / m ** p - 1.0).max()
+
+
+@pytest.mark.parametrize("low, high, bound", [(1.01, 2.0, 3.5e-7), (2.0, 3.0, 5e-7), (3.0, 4.0, 9e-7)])
+def test_the_polynomial_stays_within_the_stated_error(low, high, bound):
+    m = np.concatenate([np.arange(1.0, 2.0, 2.0 ** -12), 1.0 + np.arange(512) * 2.0 ** -23])
+    worst = max(_polynomial_error(float(np.float32(p)), m) for p in np.arange(low, high, 0.003))
+    assert 0.5 * bound < worst <= bound
+
+
+@gpu
+@pytest.mark.parametrize("p", [1.01, 1.3, 1.72, 1.99, 2.88, 3.46, 3.7, 3.999])
+@pytest.mark.parametrize("variant", ["auto", "cpasync"])
+def test_pairs_that_take_the_table(p, variant, monkeypatch):
+    """One feature, the b side zero, a contiguous along the points: column n of the result is the power of a alone, by lg2 and
+    ex2 for even n and by the table for odd n, where 2^0 m^p is the polynomial as it is."""
+    if variant != "auto":
+        monkeypatch.setenv("KERMAC_B200_VARIANT", variant)
+    m = torch.cat([torch.arange(0, 4096) * 2.0 ** -12, torch.arange(0, 512) * 2.0 ** -23]) + 1.0
+    for octave in (0, -7, 5):
+        x = torch.ldexp(m, torch.tensor(octave)).cuda()
+        b = torch.zeros(1, 70, device="cuda").t()
+        out = torch.empty(1, 70, len(x), device="cuda").transpose(1, 2)
+        kermac.cdist(x[None].t(), b, out=out, p=p, skip_epilogue=True)
+        even, odd = out[0][:, ::2], out[0][:, 1::2]
+        assert torch.equal(even, even[:, :1].expand_as(even)) and torch.equal(odd, odd[:, :1].expand_as(odd))
+        assert not torch.equal(even, odd)
+        exact = x.double() ** float(torch.tensor(p, dtype=torch.float32))
+        # elsewhere the table entry, within a unit of its last place, and the product's rounding come to it
+        bound = (3.5e-7 if p < 2 else 9e-7) + (0.0 if octave == 0 else 2.0 ** -23 + 2.0 ** -24)
+        assert ((odd[:, 0].double() - exact) / exact).abs().max() <= bound
