@@ -90,7 +90,7 @@ struct BuildPlan {
 //   torch rows, 16-byte aligned: always, because the 64 x 64 kernel loads those 16 bytes at a time too
 //       square  2 x 1000^2 x 64: 22.9 / 18.8   8000^2 x 96: 580 / 431   16384^2 x 256: 5330 / 4695
 //       |.|     2 x 1000^2 x 64: 28.9 / 17.6   8000^2 x 96: 637 / 429   16384^2 x 256: 5947 / 4671
-//       |.|^1.3 2 x 1000^2 x 64: 74.0 / 65.9   8000^2 x 96: 2413 / 2230 16384^2 x 256: 26139 / 24770
+//       |.|^1.3 2 x 1000^2 x 64: 57.1 / 49.5   8000^2 x 96: 1875 / 1708 16384^2 x 256: 20322 / 18460
 // Otherwise the gain is in how evenly tiles fall on the 148 SMs: an SM's share is ceil(4 T / 148) quarter tiles, or
 // ceil(T / 148) whole ones.  The 64 x 64 kernel is the faster one where quarters make the largest share smaller by
 // more than its longer k step costs, and where the k loop is short in any case (T: 128 x 128 tiles).
@@ -117,12 +117,18 @@ struct BuildPlan {
 //               share 1    1536^2 x 256: 51.6 / 50.2   x 512: 92.5 / 94.8   2112^2 (T 289) x 372: 129 / 133   x 1024: 332 / 352
 //               with itself 1536^2 x 700: 131 / 103   4000^2 (T 528) x 372: 266 / 229
 //               4000^2 x 256: 303 / 293   x 512: 580 / 576   16384^2 x 96: 1858 / 1825   x 128: 2374 / 2397
-//   |.|^1.3, operands not held as aligned rows: a short k loop, or up to 2048 tiles:
-//       contiguous points 2048^2 x 512: 923 / 814   4000^2 x 1024: 6276 / 6079   4736 x 4096 x 600: 4217 / 4229
-//               4400^2 x 600: 4732 / 4359   5760^2 x 600: 7340 / 7240   16384^2 x 128: 12559 / 12527   x 256: 24802 / 24864
-//       word by word 1000^2 x 27: 44.8 / 21.7   4001 x 4000 x 600: 3909 / 3835   5501 x 5500 x 600: 7209 / 7069
-//               8001 x 8003 x 300: 7543 / 7636
-//       with itself 4400^2 x 600: 2765 / 2264   5700^2 x 600: 3858 / 3704
+//   |.|^1.3, operands not held as aligned rows: a short k loop, or up to 2048 tiles (table of powers; in brackets the step
+//   by lg2 and ex2 alone, which a p in device memory takes):
+//       contiguous points 2048^2 x 512: 702 / 603 (919 / 804)   4000^2 x 1024: 4778 / 4490 (6279 / 6026)
+//               4736 x 4096 x 600: 3207 / 3135 (4220 / 4197)   4400^2 x 600: 3596 / 3221 (4725 / 4319)
+//               5760^2 x 600: 5579 / 5359 (7338 / 7178)   16384^2 x 64: 4866 / 4880 (6370 / 6302)
+//               x 128: 9573 / 9445 (12559 / 12416)   x 256: 18899 / 18480 (24800 / 24638)
+//       word by word 1000^2 x 27: 28.6 / 15.0 (34.6 / 18.6)   4001 x 4000 x 600: 3056 / 2932 (3911 / 3810)
+//               5501 x 5500 x 600: 5627 / 5400 (7214 / 7028)   8001 x 8003 x 300: 5873 / 5849 (7524 / 7594)
+//       with itself 4400^2 x 600: 2171 / 1720 (2760 / 2255)   5700^2 x 600: 3022 / 2816 (3860 / 3693)
+//               8000^2 x 200: 2033 / 1839 (2586 / 2392)
+//   (The line was drawn for the step without the table, when the two kernels were level beyond it; above 2048 tiles and 128
+//   features the 128 x 128 kernel is now 2 to 5 % the slower one, 10 % with itself.)
 // The line is drawn by the whole problem, not by the launch's tile range, so that ranges add up to the full
 // launch's bits.  For |.|^p, whose two forms of the exponential the two kernels spread differently over a tile, it
 // must not depend either on whether operands have been packed (the caller's scratch) or on symmetry (which a range
@@ -275,10 +281,10 @@ struct PackPlan {
 // Measured on B200, the 64 x 64 kernel on torch rows against the kernel that packed operands take, us:
 //   square  4000^2 x 64: 82 / 70   8000^2 x 96: 431 / 382   4000^2 x 512: 568 / 509   16384^2 x 512: 9050 / 8030
 //   |.|     8000^2 x 96: 429 / 427   4000^2 x 512: 568 / 569   16384^2 x 512: 9090 / 8800
-//   |.|^1.3 level everywhere
+//   |.|^1.3 8000^2 x 96: 1708 / 1722   4000^2 x 512: 2255 / 2260   16384^2 x 512: 36650 / 36660
 // so a pair and feature costs 7.4e-15 s less for the square and product steps, and 2e-15 s for |.| where packed
 // operands go to the 128 x 128 kernel.  An operand that could only be copied word by word costs 1e-14 s more
-// (square 8001 x 8003 x 300: 1561 us, packed 1150; |.| 1727 / 1250; |.|^1.3 7543 / 6940).  Packing must save half as much again as it costs.
+// (square 8001 x 8003 x 300: 1561 us, packed 1150; |.| 1727 / 1250; |.|^1.3 5873 / 5429).  Packing must save half as much again as it costs.
 void plan_pack_operands(const BuildPlan& plan, PackPlan* pack) {
     std::memset(pack, 0, sizeof(*pack));
     const BuildParams& p = plan.p;

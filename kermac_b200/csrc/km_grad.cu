@@ -454,11 +454,12 @@ int preferred_split(const GradPlan& plan, int norm_type, bool square_root) {
 // What the kernels of the p = 1 gradient take, us: a slab of 32 k and the rest of a block (its set-up, first slabs, last
 // sums and stores); what rows of the result that cannot be stored 16 bytes at a time add to the latter, and rows of b or
 // c that cannot be copied 16 bytes at a time to the former (warps of the sign kernel then copy 128 rows of b word by
-// word).  Fitted on B200 to 10558 calls (K 256 to 30000, M 9 to 4096, N 64 to 1000, O 1 to 64): 95 % of a kernel's calls
-// are within 8 to 20 % of estimated_us().  The sign kernel's numbers were then lowered with its instructions, by less than its times
-// fell (a slab to 0.66, 0.73, 0.55 and 0.69; words to 0.16 to 0.45), so that calls that were measured level stay where they
-// are.  Of 6000 calls of the same ranges 475 changed, by 1.22 in the geometric mean; 338 are faster by more than 2 %, 12
-// slower, one of them by more than 5 % (15 us).
+// word).  The numbers of the FP32 and the weights kernel were fitted on B200 to 10558 calls (K 256 to 30000, M 9 to 4096, N 64
+// to 1000, O 1 to 64), of which 95 % are within 8 to 20 % of estimated_us().  The sign kernel's were fitted so too and then
+// lowered when it became faster, but by less than its times fell: for 4 / 8 / 16 / 32 channels a slab takes 0.66 / 0.73 / 0.55
+// / 0.69 us and words 0.16 to 0.45.  Its times are therefore overestimated, and calls near the line keep the other kernel
+// although the sign kernel is up to 1.2 times as fast there (the lines marked * at consider_sign()).  Of 6000 calls of
+// the same ranges 475 had changed their kernel with the lowered numbers, and none of them became slower by it.
 struct P1Cost {
     double slab, block, ragged, words;
 };
@@ -507,14 +508,16 @@ double estimated_us(const GradPlan& plan, const KmGradArgs* a, long long sms, lo
 // and is alone on its SM, so short sums lose what many k win.  Measured on B200, us, sign kernel against the other one
 // (FP32 up to 16 channels, weights from 17 on):
 //   K      M     N     O    sign   other         K      M     N     O    sign   other
-//   256    4096  1000  4    328    222           256    1000  1000  16   139    189
-//   320    4096  1000  4    365    275           1024   1000  1000  4    189    260
-//   256    4096  128   4    48     36            8192   1000  1000  16   1985   5458
-//   512    250   500   64   101    107           8192   1000  1000  4    1202   1724
-//   30000  4096  256   2    4303   4443          30000  4096  256   4    4309   6226
-//   30000  4096  256   32   8902   22000         30000  4096  256   64   18100  29500
-//   8192   1000  1000  4    1497   1723 (b and c in rows that are not 16-byte aligned)
-// (Ties are left to the other kernel.)
+//   256    4096  1000  4    328    221           256    1000  1000  16   133    182
+//   320    4096  1000  3    358    273           1024   1000  1000  4    181    251
+//   256    4096  128   4    47     35            8192   1000  1000  16   1976   5456
+// * 512    250   500   64   100    105           8192   1000  1000  4    1201   1723
+// * 30000  4096  256   2    4311   4443          30000  4096  256   4    4314   6225
+//   30000  4096  256   32   8993   22054         30000  4096  256   64   18030  29480
+// b and c in rows that are not 16-byte aligned:
+// * 8192   1000  1000  4    1497   1723          30000  4096  256   16   9760   19950
+// * 30000  4096  256   4    5397   6226          30000  4096  256   32   15410  22840
+// * 30000  4096  256   64   30760  36350       * 1001   1000  300   4    92     97
 // Its split of k stays within the one that callers were told of (see kermac_b200_cdist_grad_scratch_bytes).
 void consider_sign(const KmGradArgs* a, GradPlan* plan) {
     if (a->norm_type != KM_NORM_L1 || a->contraction == KM_CONTRACT_FP32 || plan->partial_elems == 0) return;

@@ -672,9 +672,13 @@ struct MatvecPlan {
 // Preferred m split: the smallest within 0.5 % of the least estimated time.  An SM works through its share of the
 // blocks two at a time, or one by one about 13 % slower per chunk, so what counts is the largest share,
 // ceil(blocks / SMs), times the chunks of a block; a block costs about 1.5 us besides and the reduction 3 us and
-// a little per partial result.  A chunk of 128 x 128 pairs takes about 4.5 + 0.155 K us.  Measured with the
+// a little per partial result.  A chunk of 128 x 128 pairs takes about 4.5 + 0.155 K us.  (These were fitted when each MMA of
+// a tile was issued by itself and launches did not overlap.  Now a chunk of the square step takes 2.9 + 0.153 K us where an SM
+// has one block, 10 % less with two (K = 8, 27, 64, 200, 500: 4.2, 7.3, 12.7, 32.4, 79.7, of two blocks together 6.5, 12.2,
+// 22.8, 62.3, 150), a block 3 us besides and the reduction about 1.5; the splits chosen are within 4 % of the best of those
+// tried: 10007 x 1009 x 27 44.0 with 16, 42.4 with 79; 50000 x 500 x 16 65.8 with 37, 63.2 with 128.)  Measured with the
 // operands contiguous along the points, us, against the rule before (whole waves of two blocks per SM, at least
-// 8 chunks a block, at most 32 splits):
+// 8 chunks a block, at most 32 splits), with the kernel of that time:
 //   M 10007  N 1009  K 27:  72 (10 splits) -> 49 (16)       M 1000   N 300  K 27: 66 (1) -> 17 (8)
 //   M 10007  N 1009  K 200: 287 (10) -> 169 (79)            M 100000 N 100  K 64: 332 (32) -> 94 (261)
 //   M 20000  N 20000 K 64:  1962 (1) -> 1873 (16)           M 131072 N 65536 K 64: 4 splits either way
