@@ -155,6 +155,26 @@ bool small_preferred(const BuildParams& p, bool avec, bool bvec, bool awide, boo
     return tiles <= 512 || (tiles <= 1024 && p.K <= 512);
 }
 
+// Where |.|^p with few features is faster through the table of powers, although every block fills the table first and the 64 x 64
+// kernel then has three blocks on an SM instead of four.  Measured on B200, p = 1.3, time with the table over time
+// without (contiguous points, rows and words alike), features:
+//                      1      2      3      4      5      6      7      8      10     12     16     17     18     20     24
+//   64^2               1.06   1.12   1.12   1.10   1.06   1.03   1.01   0.99   0.94   0.91   1.01
+//   1000^2             1.21   1.13   1.02   0.98   0.94   0.91   0.89   0.87   0.86   0.84   0.87
+//   4 x 1000^2         1.47   1.26   1.18   1.10   1.05   1.00   0.97   0.94   0.90   0.86   0.91
+//   20000^2            1.47   1.33   1.18   1.08   1.01   0.98   0.95   0.93   0.87   0.84   0.90
+// and of a matrix with itself, where blocks store their tile twice and lean more on one another; slabs are 16 features, and one
+// that is whole runs other code than the one that is not, so that 17 features fetch both:
+//   1000^2             1.15   1.11   1.08   1.06   1.04   1.02   1.01   1.00   0.97   0.95   0.98   0.98   0.97   0.95   0.93
+//   4 x 1000^2         1.56   1.54   1.50   1.39   1.27   1.19   1.16   1.13   1.08   0.98   0.97   0.98   0.97   0.95   0.90
+//   20000^2            1.40   1.37   1.31   1.23   1.15   1.09   1.05   1.04   0.99   0.95   1.03   1.09   1.07   1.01   0.91
+// (Without a line at all 12000^2 x 1 took 291 us instead of 200.)  By what the operands are and not by p.symmetric, which tile
+// ranges and KM_SYMMETRY_OFF switch off: the bits stay the same.
+bool pow_table_preferred(const BuildParams& p) {
+    const bool same = p.A == p.B && p.M == p.N && p.a_sm == p.b_sn && p.a_sk == p.b_sk && p.a_sl == p.b_sl;
+    return same ? p.K > 20 || (p.K >= 11 && p.K <= 15) : p.K >= 6;
+}
+
 int make_plan(const KmBuildArgs* a, BuildPlan* plan) {
     if (!a) return fail(KM_ERR_NULL_POINTER, "args is NULL");
     if (a->m < 0 || a->n < 0 || a->k < 0 || a->l < 1)
@@ -218,7 +238,7 @@ int make_plan(const KmBuildArgs* a, BuildPlan* plan) {
     p.outer_power    = a->outer_power;
     p.kernel_type    = a->kernel_type;
     p.p_inner        = a->p_inner;
-    if (p.inner_id == IN_DIFF_POW && !p.p_inner.ptr) p.pow = pow_coefs(p.p_inner.value);
+    if (p.inner_id == IN_DIFF_POW && !p.p_inner.ptr && pow_table_preferred(p)) p.pow = pow_coefs(p.p_inner.value);
     p.p_outer        = a->p_outer;
     p.bandwidth      = a->bandwidth;
     p.regularization = a->regularization;

@@ -57,6 +57,26 @@ def test_which_exponents_take_the_table(p, table):
     assert ("pow=table" in _native.describe_build(_build_args(p))) is table
 
 
+@pytest.mark.parametrize("n", [40, 1000, 8000])
+@pytest.mark.parametrize("rows", [False, True])
+def test_few_features_keep_the_mufu_route(rows, n):
+    """The line lies at 6 features, for a matrix with itself at 11 to 15 and from 21 on, and follows neither the tile range nor
+    whether the mirror image is computed."""
+    for k in range(1, 40):
+        for same in (False, True):
+            args = _build_args(1.3, n, k)
+            if rows:
+                args.a_stride_m, args.a_stride_k, args.b_stride_n, args.b_stride_k = k, 1, k, 1
+            if not same:
+                args.b = 0x2000
+            table = "pow=table" in _native.describe_build(args)
+            assert table is (k in range(11, 16) or k > 20 if same else k >= 6)
+            args.symmetry = 1
+            assert ("pow=table" in _native.describe_build(args)) is table
+            args.symmetry, args.tile_count = 0, 1
+            assert ("pow=table" in _native.describe_build(args)) is table
+
+
 def test_a_tensor_exponent_and_the_tma_variant_keep_the_mufu_route():
     args = _build_args(1.3)
     args.variant = _native.VARIANT_TMA
@@ -87,7 +107,8 @@ def test_against_float64(shape, p, variant, monkeypatch):
 @gpu
 @pytest.mark.parametrize("variant", ["auto", "cpasync"])
 @pytest.mark.parametrize("p", [1.01, 1.3, 2.3, 3.7])
-def test_values_at_the_ends_of_the_range(p, variant, monkeypatch):
+@pytest.mark.parametrize("features", [3, 8])
+def test_values_at_the_ends_of_the_range(features, p, variant, monkeypatch):
     # one value against zeros in every place of a register block, so that every pair's route sees it
     if variant != "auto":
         monkeypatch.setenv("KERMAC_B200_VARIANT", variant)
@@ -95,9 +116,9 @@ def test_values_at_the_ends_of_the_range(p, variant, monkeypatch):
     values = torch.tensor([0.0, -0.0, 1e-45, 1e-39, 1.2e-38, 2e-30, 1.0, 1.9999999, 1e9, 1e19, 8e37, 1.6e38, 1.8e38, 3.4e38,
                            inf, nan])
     values = torch.cat([values, -values])
-    a = torch.zeros(40 * len(values), 3, device="cuda")
+    a = torch.zeros(40 * len(values), features, device="cuda")
     a[:, 0] = values.repeat_interleave(40)
-    b = torch.zeros(130, 3, device="cuda")
+    b = torch.zeros(130, features, device="cuda")
     want = values.repeat_interleave(40)[:, None].expand(-1, 130).cuda().double().abs() ** p
     for got in _both_routes(a, b, p):
         assert torch.equal(got.isnan(), want.isnan())
@@ -110,9 +131,11 @@ def test_values_at_the_ends_of_the_range(p, variant, monkeypatch):
 
 
 @gpu
-def test_infinite_and_undefined_differences():
+@pytest.mark.parametrize("features", [2, 24])
+def test_infinite_and_undefined_differences(features):
     inf = float("inf")
-    a = torch.tensor([[inf, 1.0], [-inf, 1.0], [3e38, 0.0], [0.0, 0.0]], device="cuda")
+    a = torch.zeros(4, features, device="cuda")
+    a[:, :2] = torch.tensor([[inf, 1.0], [-inf, 1.0], [3e38, 0.0], [0.0, 0.0]])
     got, mufu = _both_routes(a, a, 1.3)
     want = _exact(a, a, 1.3)                                 # inf - inf is NaN, 6e38 overflows
     assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), mufu.isinf())
@@ -142,16 +165,17 @@ def test_the_polynomial_stays_within_the_stated_error(low, high, bound):
 @pytest.mark.parametrize("p", [1.01, 1.3, 1.72, 1.99, 2.88, 3.46, 3.7, 3.999])
 @pytest.mark.parametrize("variant", ["auto", "cpasync"])
 def test_pairs_that_take_the_table(p, variant, monkeypatch):
-    """One feature, the b side zero, a contiguous along the points: column n of the result is the power of a alone, by lg2 and
-    ex2 for even n and by the table for odd n, where 2^0 m^p is the polynomial as it is."""
+    """One feature that is not zero, the b side zero, a contiguous along the points: column n of the result is the power of a
+    alone, by lg2 and ex2 for even n and by the table for odd n, where 2^0 m^p is the polynomial as it is."""
     if variant != "auto":
         monkeypatch.setenv("KERMAC_B200_VARIANT", variant)
     m = torch.cat([torch.arange(0, 4096) * 2.0 ** -12, torch.arange(0, 512) * 2.0 ** -23]) + 1.0
     for octave in (0, -7, 5):
         x = torch.ldexp(m, torch.tensor(octave)).cuda()
-        b = torch.zeros(1, 70, device="cuda").t()
+        a, b = torch.zeros(6, len(x), device="cuda"), torch.zeros(6, 70, device="cuda")
+        a[2] = x
         out = torch.empty(1, 70, len(x), device="cuda").transpose(1, 2)
-        kermac.cdist(x[None].t(), b, out=out, p=p, skip_epilogue=True)
+        kermac.cdist(a.t(), b.t(), out=out, p=p, skip_epilogue=True)
         even, odd = out[0][:, ::2], out[0][:, 1::2]
         assert torch.equal(even, even[:, :1].expand_as(even)) and torch.equal(odd, odd[:, :1].expand_as(odd))
         assert not torch.equal(even, odd)
