@@ -30,7 +30,7 @@
 // every memory operation of the thread, and behind loads in flight it made each slab as long as a load.
 // What bounds it (B200, K = 30000, M = 4096, N = 256; ms, in brackets the kernel that took these calls before):
 // 4 channels 4.31 (6.2), 8: 4.72 (10.6), 16: 7.13 (20.3), 32: 9.0 with the
-// same inputs again, 9.3 with new ones (22.0), 64: 18.0 to 18.4.
+// same inputs again, 9.3 to 9.4 with new ones (22.0), 64: 18.0 to 18.4.
 // The MMAs alone would take 2.5 ms at 32 channels (an MMA of 128 rows x N columns holds the tensor pipe N / 2 cycles,
 // also with the stores to tensor memory beside it), the ALU pipe (permutes and logic, half rate) about 3.5.  Instructions are
 // what the rest goes to: at 4 channels the generating warps hardly rest, at 32 the product warps, each warp issuing once in five to
